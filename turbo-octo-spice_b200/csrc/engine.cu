@@ -59,7 +59,7 @@ __global__ void k_fill(float* p, size_t n, float v) {
 // sums of (w*delta, w, loglam); coordinate ranges; sortedness.
 __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t* npix,
                        size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pack, double* wd, float* w,
-                       double4* prefix, float4* range, unsigned int* flags,
+                       double4* prefix, double2* pre2, double2* row2, float4* range, unsigned int* flags,
                        unsigned long long* maxbits) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -69,12 +69,16 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
     const uint32_t n = npix[s];
     const uint64_t po = o + (uint64_t)kPad * (s + 1);
     double4* pre = prefix + o + s;
+    double2* p2 = pre2 + o + s;
     double c0 = 0, c1 = 0, c2 = 0;
     float dmin = INFINITY, dmax = -INFINITY, lmin = INFINITY, lmax = -INFINITY;
     double mwd = 0, mw = 0, ml = 0, md = 0;
     float gap = INFINITY;  // smallest positive step between consecutive distances
     bool unsorted = false;
-    if (lane == 0) pre[0] = make_double4(0, 0, 0, 0);
+    if (lane == 0) {
+      pre[0] = make_double4(0, 0, 0, 0);
+      p2[0] = make_double2(0, 0);
+    }
     for (uint32_t b = 0; b < n; b += 32) {
       const uint32_t k = b + lane;
       double v0 = 0, v1 = 0, v2 = 0;
@@ -87,6 +91,7 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
         v2 = (double)px.loglam;
         wd[o + k] = v0;
         w[o + k] = px.weight;
+        row2[o + k] = make_double2(v0, v1);
         PixPack q;
         q.d = px.distance;
         q.w = px.weight;
@@ -120,7 +125,10 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
           v2 += u2;
         }
       }
-      if (k < n) pre[k + 1] = make_double4(c0 + v0, c1 + v1, c2 + v2, 0);
+      if (k < n) {
+        pre[k + 1] = make_double4(c0 + v0, c1 + v1, c2 + v2, 0);
+        p2[k + 1] = make_double2(c0 + v0, c1 + v1);
+      }
       c0 += __shfl_sync(kFull, v0, 31);
       c1 += __shfl_sync(kFull, v1, 31);
       c2 += __shfl_sync(kFull, v2, 31);
@@ -615,36 +623,109 @@ __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint3
   }
 }
 
-// Boundary table B[g][t], t = 0 .. 2 nk - 1 (nk = n0 + 1 thresholds): the
-// first grid index g2 whose value x2 = U[g2] passes the boundary predicate of
-// threshold T[k] against x1 = U[g],
+// Loglam of every grid value, and whether it is a function of the value:
+// pass 0 writes the loglam of each on-grid pixel (equal values write the same
+// one, or some one of them), pass 1 counts the pixels that differ from it.
+__global__ void k_grid_loglam(int pass, const float* lpad, const uint64_t* off, const uint32_t* npix, size_t n_los,
+                              const uint32_t* gfirst, float* gl, unsigned long long* n_bad) {
+  const int lane = threadIdx.x & 31;
+  const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
+  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  for (size_t s = warp; s < n_los; s += nwarps) {
+    const uint32_t f = gfirst[s], n = npix[s];
+    if (f == kNoGrid) continue;
+    const float* l = lpad + off[s] + (uint64_t)kPad * (s + 1);
+    unsigned bad = 0;
+    for (uint32_t p = lane; p < n; p += 32) {
+      if (pass == 0) gl[f + p] = l[p];
+      else if (gl[f + p] != l[p]) bad = 1;
+    }
+    if (bad) atomicAdd(n_bad, 1ull);
+  }
+}
+
+constexpr int kTableThreads = 256;
+
+// glp[g] = sum over g' < g of gl[g'] - lmid, g = 0 .. ng (one block).
+__global__ void __launch_bounds__(kTableThreads) k_grid_lprefix(const float* gl, int ng, double lmid, double* glp) {
+  using Scan = cub::BlockScan<double, kTableThreads>;
+  __shared__ typename Scan::TempStorage tmp;
+  double base = 0.0;
+  for (int b = 0; b <= ng; b += kTableThreads) {
+    const int g = b + threadIdx.x;
+    double ex, sum;
+    Scan(tmp).ExclusiveSum(g < ng ? (double)gl[g] - lmid : 0.0, ex, sum);
+    if (g <= ng) glp[g] = base + ex;
+    base += sum;
+    __syncthreads();
+  }
+}
+
+// Boundary tables of the grid sweep; one block per boundary t = 0 .. 2 nk - 1
+// (nk = n0 + 1 thresholds).  B_t[g] is the first grid index g2 whose value
+// x2 = U[g2] passes the boundary predicate of threshold T[k] against x1 = U[g],
 //   side 1, t <= n0 (k = n0 - t):      x2 >= x1 or  fl(x1 - x2) <  T[k];
 //   side 0, t = n0 + 1 + k:            x2 >= x1 and fl(x2 - x1) >= T[k].
 // Along t the entries are non-decreasing, so the row's columns split into the
-// consecutive runs [B[t], B[t+1]): first-axis bin n0 - 1 - t below x1
-// (t < n0), the |x1 - x2| < T[0] gap (t = n0), bin t - n0 - 1 above x1.
-__global__ void k_grid_table(const float* U, int ng, const float* thr, int nk, uint16_t* Q) {
-  const int nb = 2 * nk;
-  const size_t total = (size_t)ng * nb;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int tb = (int)(e % nb);
-    const int g = (int)(e / nb);
-    const int side = tb < nk ? 1 : 0;
-    const int k = side ? nk - 1 - tb : tb - nk;
-    const float x1 = U[g], t = thr[k];
+// consecutive runs [B_t, B_{t+1}): first-axis bin n0 - 1 - t below x1
+// (t < n0), the |x1 - x2| < T[0] gap (t = n0), bin t - n0 - 1 above x1; along
+// g they are non-decreasing too, so `inv` holds the first row that reaches
+// each column.  tb and tz are prefix sums over the rows.
+__global__ void __launch_bounds__(kTableThreads)
+    k_grid_tables(const float* U, const float* gl, const double* glp, double lmid, int ng, int ngp, const float* thr,
+                  int nk, uint16_t* tab, uint16_t* inv, uint32_t* tb, double* tz) {
+  using ScanD = cub::BlockScan<double, kTableThreads>;
+  using ScanU = cub::BlockScan<uint32_t, kTableThreads>;
+  __shared__ union {
+    typename ScanD::TempStorage d;
+    typename ScanU::TempStorage u;
+  } tmp;
+  const int t = blockIdx.x;
+  const int side = t < nk ? 1 : 0;
+  const float T = thr[side ? nk - 1 - t : t - nk];
+  tab += (size_t)t * ngp;
+  inv += (size_t)t * (ng + 1);
+  tb += (size_t)t * (ng + 1);
+  tz += (size_t)t * (ng + 1);
+  uint32_t base_u = 0;
+  double base_d = 0.0;
+  for (int b = 0; b <= ng; b += kTableThreads) {
+    const int g = b + threadIdx.x;
+    int lo = 0;
+    if (g < ng) {
+      const float x1 = U[g];
+      int hi = ng;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const float x2 = U[mid];
+        const bool ge = x2 >= x1;
+        const bool pass = side ? (ge || !(__fsub_rn(x1, x2) >= T)) : (ge && __fsub_rn(x2, x1) >= T);
+        if (pass) hi = mid; else lo = mid + 1;
+      }
+      tab[g] = (uint16_t)lo;
+    }
+    uint32_t eu, su;
+    ScanU(tmp.u).ExclusiveSum((uint32_t)lo, eu, su);
+    __syncthreads();
+    double ed, sd;
+    ScanD(tmp.d).ExclusiveSum(g < ng ? 0.5 * (((double)gl[g] - lmid) * (double)lo + glp[lo]) : 0.0, ed, sd);
+    __syncthreads();
+    if (g <= ng) {
+      tb[g] = base_u + eu;
+      tz[g] = base_d + ed;
+    }
+    base_u += su;
+    base_d += sd;
+  }
+  for (int g = ng + threadIdx.x; g < ngp; g += kTableThreads) tab[g] = (uint16_t)ng;
+  __syncthreads();
+  for (int x = threadIdx.x; x <= ng; x += kTableThreads) {
     int lo = 0, hi = ng;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      const float x2 = U[mid];
-      const bool ge = x2 >= x1;
-      const bool pass = side ? (ge || !(__fsub_rn(x1, x2) >= t)) : (ge && __fsub_rn(x2, x1) >= t);
-      if (pass)
-        hi = mid;
-      else
-        lo = mid + 1;
+      if ((int)tab[mid] >= x) hi = mid; else lo = mid + 1;
     }
-    Q[e] = (uint16_t)lo;
+    inv[x] = (uint16_t)lo;
   }
 }
 
@@ -697,6 +778,28 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   TOS_CUDA_TRY(cudaGetLastError());
   unsigned long long h = 0;
   TOS_CUDA_TRY(cudaMemcpyAsync(&h, nok.p, 8, cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h == 0) return TOS_OK;
+  // the grid sweep takes a pixel's loglam from its grid value: not usable
+  // when two pixels of one value differ in it
+  TOS_TRY(cat->d_gl[w].alloc(ng));
+  TOS_TRY(cat->d_glp[w].alloc(ng + 1));
+  TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gl[w].p, 0, ng * sizeof(float), st));
+  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 8, st));
+  for (int pass = 0; pass < 2; ++pass)
+    k_grid_loglam<<<grid_for(e, cat->n_los * 32, 256), 256, 0, st>>>(pass, cat->d_loglam_pad.p, cat->d_off.p,
+                                                                    cat->d_npix.p, cat->n_los, cat->d_gfirst[w].p,
+                                                                    cat->d_gl[w].p, nok.p);
+  TOS_CUDA_TRY(cudaGetLastError());
+  unsigned long long bad = 0;
+  float lmid = 0.f;
+  TOS_CUDA_TRY(cudaMemcpyAsync(&bad, nok.p, 8, cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaMemcpyAsync(&lmid, cat->d_gl[w].p + ng / 2, sizeof(float), cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  if (bad) return TOS_OK;
+  cat->grid_lmid[w] = (double)lmid;
+  k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, ng, (double)lmid, cat->d_glp[w].p);
+  TOS_CUDA_TRY(cudaGetLastError());
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   cat->grid_n[w] = ng;
   cat->grid_los[w] = h;
@@ -1008,6 +1111,8 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   TOS_TRY(cat->d_wd.alloc(total));
   TOS_TRY(cat->d_w.alloc(total));
   TOS_TRY(cat->d_prefix.alloc(total + n_los));
+  TOS_TRY(cat->d_pre2.alloc(total + n_los));
+  TOS_TRY(cat->d_row2.alloc(total));
   TOS_TRY(cat->d_range.alloc(n_los));
   TOS_TRY(cat->d_flags.alloc(3));
   TOS_TRY(cat->d_maxes.alloc(4));
@@ -1061,7 +1166,7 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   k_fill_pack<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_pack.p, padded);
   k_prep<<<grid_for(e, n_los * 32, 256), 256, 0, st>>>(
       cat->d_raw.p, cat->d_off.p, cat->d_npix.p, n_los, cat->d_dist_pad.p, cat->d_loglam_pad.p, cat->d_pack.p,
-      cat->d_wd.p, cat->d_w.p, cat->d_prefix.p, cat->d_range.p, cat->d_flags.p,
+      cat->d_wd.p, cat->d_w.p, cat->d_prefix.p, cat->d_pre2.p, cat->d_row2.p, cat->d_range.p, cat->d_flags.p,
       (unsigned long long*)cat->d_maxes.p);
   TOS_CUDA_TRY(cudaGetLastError());
   unsigned int fl[3] = {0u, 0u, 0u};
@@ -1210,8 +1315,9 @@ uint64_t catalog_data_bytes(const tos_catalog* c) {
                c->d_members.bytes() + c->d_npix.bytes() + c->d_off.bytes() + c->d_raw.bytes() +
                c->d_dist_pad.bytes() + c->d_loglam_pad.bytes() + c->d_pack.bytes() + c->d_wd.bytes() +
                c->d_w.bytes() +
-               c->d_prefix.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
-  for (int w = 0; w < 2; ++w) b += c->d_grid[w].bytes() + c->d_gfirst[w].bytes();
+               c->d_prefix.bytes() + c->d_pre2.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
+  for (int w = 0; w < 2; ++w)
+    b += c->d_grid[w].bytes() + c->d_gl[w].bytes() + c->d_glp[w].bytes() + c->d_gfirst[w].bytes();
   return b;
 }
 
@@ -1220,7 +1326,8 @@ size_t Workspace::bytes() const {
          d_cand.bytes() +
          d_item_off.bytes() + d_item_i.bytes() + d_item_j.bytes() + d_item_sep.bytes() +
          d_item_c.bytes() + d_cell_pairs.bytes() + d_acc.bytes() + d_out.bytes() +
-         d_counters.bytes() + d_thr.bytes() + d_gq.bytes() + d_cub_tmp.bytes();
+         d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_ginv.bytes() + d_gtb.bytes() +
+         d_gtz.bytes() + d_cub_tmp.bytes();
 }
 
 // Counter words of a run: kernel counters [0, 16), the theta-edge flags of
@@ -1637,15 +1744,35 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     const int w = (G.type == TOS_OBSERVING) ? 1 : 0;
     TOS_TRY(ensure_grid(e, cat, w, st));
     const int ng = cat->grid_n[w];
-    if (ng > 0 && cat->grid_los[w] > 0) {
-      const size_t nq = (size_t)2 * ng * (n0 + 1);
-      TOS_TRY(ws->d_gq.alloc(nq));
-      k_grid_table<<<grid_for(e, nq, 256), 256, 0, st>>>(cat->d_grid[w].p, ng, ws->d_thr.p,
-                                                         (int)n0 + 1, ws->d_gq.p);
+    // the boundary tables take 16 bytes per boundary and grid value; beyond
+    // 2 GiB of them the pointer sweep takes the items
+    const bool tables_fit = (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 16.0 < 2147483648.0;
+    if (ng > 0 && cat->grid_los[w] > 0 && tables_fit) {
+      const size_t nbd = 2 * ((size_t)n0 + 1);
+      const int ngp = (ng + 7) / 4 * 4;
+      TOS_TRY(ws->d_gtab.alloc(nbd * ngp));
+      TOS_TRY(ws->d_ginv.alloc(nbd * (ng + 1)));
+      TOS_TRY(ws->d_gtb.alloc(nbd * (ng + 1)));
+      TOS_TRY(ws->d_gtz.alloc(nbd * (ng + 1)));
+      k_grid_tables<<<(unsigned)nbd, kTableThreads, 0, st>>>(
+          cat->d_grid[w].p, cat->d_gl[w].p, cat->d_glp[w].p, cat->grid_lmid[w], ng, ngp, ws->d_thr.p, (int)n0 + 1,
+          ws->d_gtab.p, ws->d_ginv.p, ws->d_gtb.p, ws->d_gtz.p);
       TOS_CUDA_TRY(cudaGetLastError());
-      A.gq = ws->d_gq.p;
+      A.gtab = ws->d_gtab.p;
+      A.ginv = ws->d_ginv.p;
+      A.gtb = ws->d_gtb.p;
+      A.gtz = ws->d_gtz.p;
+      A.gU = cat->d_grid[w].p;
+      A.gl = cat->d_gl[w].p;
+      A.glp = cat->d_glp[w].p;
+      A.lmid = cat->grid_lmid[w];
+      A.jit_u = std::ldexp(cat->max_d * cat->max_d, -24) * rg.inv1 * rg.inv1 * 1.01;
+      A.pre2 = cat->d_pre2.p;
+      A.row2 = cat->d_row2.p;
       A.gfirst = cat->d_gfirst[w].p;
       A.ng = ng;
+      A.ngp = ngp;
+      A.max_np = (int)cat->max_np;
       A.grid_split = 1;
       use_grid = true;
     }

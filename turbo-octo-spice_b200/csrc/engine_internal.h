@@ -82,7 +82,9 @@ struct Workspace {
   DevBuf<tos_xibin> d_out;                        // combined / per row output
   DevBuf<unsigned long long> d_counters;          // misc counters
   DevBuf<float> d_thr;                            // first-axis thresholds of the run sweep
-  DevBuf<uint16_t> d_gq;                          // boundary table of the current call
+  DevBuf<uint16_t> d_gtab, d_ginv;                // boundary tables of the current call (grid sweep)
+  DevBuf<uint32_t> d_gtb;
+  DevBuf<double> d_gtz;
   DevBuf<unsigned char> d_cub_tmp;
   // the last completed per-cell run in d_acc
   bool last_valid = false;
@@ -149,6 +151,8 @@ struct tos_catalog {
   tos::DevBuf<double> d_wd;         // w*delta per pixel, exact in double
   tos::DevBuf<float> d_w;           // weight per pixel
   tos::DevBuf<double4> d_prefix;    // per sightline N+1 exclusive prefix sums of (w*delta, w, loglam)
+  tos::DevBuf<double2> d_pre2;      // its (w*delta, w) alone
+  tos::DevBuf<double2> d_row2;      // (w*delta, w) per pixel
   tos::DevBuf<float4> d_range;      // per sightline (dmin, dmax, lmin, lmax)
   tos::DevBuf<unsigned int> d_flags;// [0]: bit 0 some sightline is not sorted by distance and
                                     // loglam, bit 1 a non-finite value; [1] order key of the
@@ -166,6 +170,9 @@ struct tos_catalog {
   int grid_n[2] = {0, 0};                              // distinct values (0: no usable grid)
   uint64_t grid_los[2] = {0, 0};                       // sightlines contiguous on the grid
   tos::DevBuf<float> d_grid[2];                        // sorted distinct values
+  tos::DevBuf<float> d_gl[2];                          // loglam of each value
+  tos::DevBuf<double> d_glp[2];                        // exclusive prefix sums of loglam - lmid
+  double grid_lmid[2] = {0, 0};                        // loglam of the middle value
   tos::DevBuf<uint32_t> d_gfirst[2];                   // per sightline grid index of pixel 0 or kNoGrid
   // the workspace of tos_xi_run on this catalogue; its per-cell sums stay
   // there after the run for the covariance calls

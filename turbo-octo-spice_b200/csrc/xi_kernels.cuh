@@ -103,11 +103,22 @@ struct PairArgs {
                              // pixel-pair kernel skips those and evaluates the rest exactly
   double run_amin;           // Cartesian: smallest 2(1 - cos theta) the run sweep accepts
   const float* thr;          // run sweep: first-axis thresholds T[0..n0]
-  // boundary table of the catalogue's common first-axis grid (grid sweep)
-  const uint16_t* gq;        // [ng][2 n0 + 2]: a grid row's run boundaries in column order
-                             // (k_grid_table, engine.cu)
+  // the catalogue's common first-axis grid and its boundary tables (grid
+  // sweep; boundary t = 0 .. 2 n0 + 1 of grid row g, k_grid_tables, engine.cu)
+  const uint16_t* gtab;      // [2 n0 + 2][ngp]: B_t[g], first column of boundary t in row g
+  const uint16_t* ginv;      // [2 n0 + 2][ng + 1]: first row g with B_t[g] >= x
+  const uint32_t* gtb;       // [2 n0 + 2][ng + 1]: sum of B_t over the rows below g (mod 2^32)
+  const double* gtz;         // [2 n0 + 2][ng + 1]: sum of (l'[g'] B_t[g'] + glp[B_t[g']]) / 2 over them
+  const float* gU;           // [ng]: the grid's values
+  const float* gl;           // [ng]: loglam of each grid value
+  const double* glp;         // [ng + 1]: exclusive prefix sums of l' = loglam - lmid
   const uint32_t* gfirst;    // per sightline: grid index of pixel 0, or kNoGrid
-  int ng;                    // grid values
+  const double2* pre2;       // prefix sums (wd, w) alone, laid out as `prefix`
+  const double2* row2;       // (w*delta, w) per pixel
+  double lmid;               // loglam near the middle of the grid
+  double jit_u;              // bound of the float rounding of d1*d1, times inv1^2
+  int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
+  int max_np;                // longest sightline
   int grid_split;            // the grid kernel takes the run items whose sightlines are on the grid
   int diag_split;            // Polar: the diagonal-sweep kernel takes the items whose z index is
                              // constant; the pixel-pair kernel evaluates the rest exactly
