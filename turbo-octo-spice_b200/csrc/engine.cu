@@ -545,6 +545,26 @@ int bitlen(uint32_t v) {
   return b;
 }
 
+// Bounds of the r_perp code edges m = 0 .. n1 (PairArgs::edges).  Column code
+// >= m means t = sqrt(u) - min1 inv1 >= m (m = 0: t > -1); the margins cover
+// four times the FP64 re-evaluation window of 2^-k1 bins, the FP32 rounding
+// of u (4e-6 relative), and in x and y the float rounding `jit` of d1*d1.
+std::vector<float4> code_edges(const RefGrid& g, int k1, double jit) {
+  std::vector<float4> e(g.n1 + 1);
+  const double off = -g.min1 * g.inv1;
+  for (uint32_t m = 0; m <= g.n1; ++m) {
+    const double s = (m == 0 ? -1.0 : (double)m) - off;
+    if (!(s > 0)) {  // below every column
+      e[m] = make_float4(-1.f, -1.f, -1.f, -1.f);
+      continue;
+    }
+    const double dt = std::ldexp(4.0, -k1) + 1e-6 * std::fabs(off);
+    const double w = 2 * s * dt + dt * dt + 4e-6 * s * s;
+    e[m] = make_float4((float)(s * s - w - jit), (float)(s * s + w + jit), (float)(s * s - w), (float)(s * s + w));
+  }
+  return e;
+}
+
 bool is_pow2(double v) {
   if (!(v > 0) || !std::isfinite(v)) return false;
   int e;
@@ -645,6 +665,7 @@ __global__ void k_grid_loglam(int pass, const float* lpad, const uint64_t* off, 
 }
 
 constexpr int kTableThreads = 256;
+constexpr int kSkewPad = 3;  // blocks before a skewed boundary's first and after its last
 
 // glp[g] = sum over g' < g of gl[g'] - lmid, g = 0 .. ng (one block).
 __global__ void __launch_bounds__(kTableThreads) k_grid_lprefix(const float* gl, int ng, double lmid, double* glp) {
@@ -673,7 +694,8 @@ __global__ void __launch_bounds__(kTableThreads) k_grid_lprefix(const float* gl,
 // each column.  tb and tz are prefix sums over the rows.
 __global__ void __launch_bounds__(kTableThreads)
     k_grid_tables(const float* U, const float* gl, const double* glp, double lmid, int ng, int ngp, const float* thr,
-                  int nk, uint16_t* tab, uint16_t* inv, uint32_t* tb, double* tz) {
+                  int nk, int full_skew, int nblk, uint16_t* tab, uint16_t* inv, uint32_t* tb, double* tz,
+                  uint32_t* skew, uint2* tabs, uint16_t* glev, int nlev, double lev0, double dlev) {
   using ScanD = cub::BlockScan<double, kTableThreads>;
   using ScanU = cub::BlockScan<uint32_t, kTableThreads>;
   __shared__ union {
@@ -726,6 +748,35 @@ __global__ void __launch_bounds__(kTableThreads)
       if ((int)tab[mid] >= x) hi = mid; else lo = mid + 1;
     }
     inv[x] = (uint16_t)lo;
+  }
+  // the skewed copy (see PairArgs::gtabs): the row at which the boundary
+  // meets the anti-diagonal through the middle of the grid (or its middle
+  // column), from the end of the grid
+  __shared__ int s_skew;
+  if (threadIdx.x == 0) {
+    int lo = 0, hi = ng;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if ((full_skew ? 2 * (int)tab[mid] : mid + (int)tab[mid]) >= ng) hi = mid; else lo = mid + 1;
+    }
+    s_skew = kSkewPad + ((ng - lo) >> 2);
+    skew[t] = (uint32_t)s_skew;
+  }
+  __syncthreads();
+  const int ns = s_skew;
+  uint2* dst = tabs + ((size_t)(t >> 5) * nblk + ns) * 32 + (t & 31);
+  for (int b = threadIdx.x; b < ngp / 4; b += kTableThreads)
+    dst[(size_t)b * 32] = reinterpret_cast<const uint2*>(tab)[b];
+  // first row whose product of values reaches each level
+  for (int l = threadIdx.x; glev && l <= nlev; l += kTableThreads) {
+    const double q = lev0 + (double)l * dlev;
+    int lo = 0, hi = ng;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      const int c = tab[mid];
+      if (c >= ng || (double)U[mid] * (double)U[c] >= q) hi = mid; else lo = mid + 1;
+    }
+    glev[(size_t)t * (nlev + 1) + l] = (uint16_t)lo;
   }
 }
 
@@ -800,6 +851,9 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   cat->grid_lmid[w] = (double)lmid;
   k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, ng, (double)lmid, cat->d_glp[w].p);
   TOS_CUDA_TRY(cudaGetLastError());
+  TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  TOS_CUDA_TRY(cudaMemcpyAsync(&cat->grid_lo[w], cat->d_grid[w].p, sizeof(float), cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaMemcpyAsync(&cat->grid_hi[w], cat->d_grid[w].p + ng - 1, sizeof(float), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   cat->grid_n[w] = ng;
   cat->grid_los[w] = h;
@@ -1327,7 +1381,7 @@ size_t Workspace::bytes() const {
          d_item_off.bytes() + d_item_i.bytes() + d_item_j.bytes() + d_item_sep.bytes() +
          d_item_c.bytes() + d_cell_pairs.bytes() + d_acc.bytes() + d_out.bytes() +
          d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_ginv.bytes() + d_gtb.bytes() +
-         d_gtz.bytes() + d_cub_tmp.bytes();
+         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
 }
 
 // Counter words of a run: kernel counters [0, 16), the theta-edge flags of
@@ -1486,7 +1540,8 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   TOS_CUDA_TRY(cudaMemsetAsync(ws->d_counters.p, 0, kCounterWords * 8, st));
   // [0..3] kernel counters, [4] pair-kernel item counter, [5] candidates,
   // [6] window flushes, [7] run-kernel item counter, [8] run items, [9] grid
-  // items, [10] grid-kernel item counter,
+  // items, [10] grid-kernel item counter, [11] diagonal-kernel item counter,
+  // [12] diagonal items, [13] a grid-kernel wait ran out,
   // [16] theta indices on an edge, [17..] their item numbers (4096 at most)
   unsigned long long* ctr = ws->d_counters.p;
   const double theta_min = G.axis[1].min, theta_inv = 1.0 / axis_width(G.axis[1]);
@@ -1740,13 +1795,14 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   }
   // --- grid sweep: catalogues whose first-axis values lie on a small common grid
   bool use_grid = false;
+  std::vector<float4> edges;  // kept until the stream sync
   if (use_runs) {
     const int w = (G.type == TOS_OBSERVING) ? 1 : 0;
     TOS_TRY(ensure_grid(e, cat, w, st));
     const int ng = cat->grid_n[w];
-    // the boundary tables take 16 bytes per boundary and grid value; beyond
+    // the boundary tables take 20 bytes per boundary and grid value; beyond
     // 2 GiB of them the pointer sweep takes the items
-    const bool tables_fit = (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 16.0 < 2147483648.0;
+    const bool tables_fit = (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 20.0 < 2147483648.0;
     if (ng > 0 && cat->grid_los[w] > 0 && tables_fit) {
       const size_t nbd = 2 * ((size_t)n0 + 1);
       const int ngp = (ng + 7) / 4 * 4;
@@ -1754,19 +1810,43 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       TOS_TRY(ws->d_ginv.alloc(nbd * (ng + 1)));
       TOS_TRY(ws->d_gtb.alloc(nbd * (ng + 1)));
       TOS_TRY(ws->d_gtz.alloc(nbd * (ng + 1)));
+      const bool cart = G.type == TOS_CARTESIAN;
+      // levels of d1 d2: finer than a row (at most 2048)
+      const int nlev = cart ? std::min(2048, std::max(64, 2 * ng)) : 0;
+      const double lev0 = (double)cat->grid_lo[w] * cat->grid_lo[w];
+      const double dlev = cart ? std::max((double)cat->grid_hi[w] * cat->grid_hi[w] - lev0, 1e-6 * lev0) / nlev : 1.0;
+      if (cart) {
+        edges = code_edges(rg, A.k1, std::ldexp(cat->max_d * cat->max_d, -24) * rg.inv1 * rg.inv1 * 1.01);
+        TOS_TRY(ws->d_edges.alloc(edges.size()));
+        TOS_CUDA_TRY(cudaMemcpyAsync(ws->d_edges.p, edges.data(), edges.size() * sizeof(float4),
+                                     cudaMemcpyHostToDevice, st));
+        TOS_TRY(ws->d_glev.alloc(nbd * (nlev + 1)));
+      }
+      const int nblk = ngp / 4 + ng / 4 + 2 * kSkewPad;  // 4-row blocks of a skewed boundary
+      TOS_TRY(ws->d_gskew.alloc(nbd));
+      TOS_TRY(ws->d_gtabs.alloc((nbd + 31) / 32 * 32 * nblk));
       k_grid_tables<<<(unsigned)nbd, kTableThreads, 0, st>>>(
           cat->d_grid[w].p, cat->d_gl[w].p, cat->d_glp[w].p, cat->grid_lmid[w], ng, ngp, ws->d_thr.p, (int)n0 + 1,
-          ws->d_gtab.p, ws->d_ginv.p, ws->d_gtb.p, ws->d_gtz.p);
+          G.type == TOS_OBSERVING ? 1 : 0, nblk, ws->d_gtab.p, ws->d_ginv.p, ws->d_gtb.p, ws->d_gtz.p, ws->d_gskew.p,
+          ws->d_gtabs.p, cart ? ws->d_glev.p : nullptr, nlev, lev0, dlev);
       TOS_CUDA_TRY(cudaGetLastError());
       A.gtab = ws->d_gtab.p;
       A.ginv = ws->d_ginv.p;
       A.gtb = ws->d_gtb.p;
       A.gtz = ws->d_gtz.p;
+      A.gtabs = ws->d_gtabs.p;
+      A.gskew = ws->d_gskew.p;
+      A.nblk = nblk;
       A.gU = cat->d_grid[w].p;
       A.gl = cat->d_gl[w].p;
       A.glp = cat->d_glp[w].p;
       A.lmid = cat->grid_lmid[w];
-      A.jit_u = std::ldexp(cat->max_d * cat->max_d, -24) * rg.inv1 * rg.inv1 * 1.01;
+      A.edges = ws->d_edges.p;
+      A.glev = ws->d_glev.p;
+      A.nlev = nlev;
+      A.lev_scale = (float)(1.0 / dlev);
+      // a hundredth of a level and 4e-6 of it cover the FP32 rounding of an edge's level
+      A.lev_off = (float)(-lev0 / dlev - 0.01 - 4e-6 * (lev0 / dlev + nlev));
       A.pre2 = cat->d_pre2.p;
       A.row2 = cat->d_row2.p;
       A.gfirst = cat->d_gfirst[w].p;
@@ -1940,10 +2020,11 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   if (n_rows)
     TOS_CUDA_TRY(cudaMemcpyAsync(out_cells, ws->d_out.p + nb, n_rows * nb * sizeof(tos_xibin),
                                  cudaMemcpyDeviceToHost, st));
-  unsigned long long hc[13];
+  unsigned long long hc[14];
   TOS_CUDA_TRY(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaEventRecord(e->ev[4], st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  if (hc[13]) return fail(TOS_ERR_TIMEOUT, "a wait of the grid sweep ran out");
   ws->last_valid = (plan == nullptr);  // slot rows are not per-cell sums
   ws->last_nb = nb;
   for (int k = 0; k < 7; ++k) ws->last_inv_scale[k] = 1.0 / A.scale[k];

@@ -82,8 +82,10 @@ struct Workspace {
   DevBuf<tos_xibin> d_out;                        // combined / per row output
   DevBuf<unsigned long long> d_counters;          // misc counters
   DevBuf<float> d_thr;                            // first-axis thresholds of the run sweep
-  DevBuf<uint16_t> d_gtab, d_ginv;                // boundary tables of the current call (grid sweep)
-  DevBuf<uint32_t> d_gtb;
+  DevBuf<uint16_t> d_gtab, d_ginv, d_glev;        // boundary tables of the current call (grid sweep)
+  DevBuf<uint32_t> d_gtb, d_gskew;
+  DevBuf<uint2> d_gtabs;
+  DevBuf<float4> d_edges;
   DevBuf<double> d_gtz;
   DevBuf<unsigned char> d_cub_tmp;
   // the last completed per-cell run in d_acc
@@ -173,6 +175,7 @@ struct tos_catalog {
   tos::DevBuf<float> d_gl[2];                          // loglam of each value
   tos::DevBuf<double> d_glp[2];                        // exclusive prefix sums of loglam - lmid
   double grid_lmid[2] = {0, 0};                        // loglam of the middle value
+  float grid_lo[2] = {0, 0}, grid_hi[2] = {0, 0};      // smallest and largest value
   tos::DevBuf<uint32_t> d_gfirst[2];                   // per sightline grid index of pixel 0 or kNoGrid
   // the workspace of tos_xi_run on this catalogue; its per-cell sums stay
   // there after the run for the covariance calls

@@ -32,8 +32,9 @@ __device__ __forceinline__ long long to_fixed(double c, double scale) {
 // rounded first and the exact remainder carries the low 44 bits.
 __device__ __forceinline__ long long to_fixed_wide(double c, double sh) {
   const double v = c * sh;
-  const long long qh = __double_as_longlong(__dadd_rn(v, kMagic52)) - kMagic52Bits;
-  const double rem = v - (double)qh;  // exact, |rem| <= 0.5
+  const double r = __dadd_rn(v, kMagic52);
+  const long long qh = __double_as_longlong(r) - kMagic52Bits;
+  const double rem = v - __dsub_rn(r, kMagic52);  // r - magic is qh exactly; |rem| <= 0.5
   return (qh << 44) + to_fixed(rem, 17592186044416.0 /* 2^44 */);
 }
 

@@ -34,17 +34,24 @@
 // one column.  The z sums and pair counts of a stretch of rows depend on the
 // grid alone and come from prefix tables over the rows.
 //
-// What bounds it: shared-memory reads.  A step (one row of 32 boundaries)
-// takes two 16-byte reads per lane; lanes of neighbouring boundaries sit
-// about three rows and three columns apart, so their reads fall in different
-// banks, and the seven FP64 instructions of a step issue beside them.
+// What bounds it: shared-memory reads and the latency of the table reads
+// around the inner loop (LSU data pipe 63 %, issue 41 %, most stalled cycles on
+// L2 reads; ncu, 1,000 sightlines).  A step (one row of 32 boundaries) takes
+// two 16-byte reads per lane at the least eight wavefronts; starting the lanes
+// at row residues that keep both reads of eight lanes in different banks took
+// the bank conflicts from 1.3e9 to 0.3e9 wavefronts of 2.5e9.
 //
 // Measured on a B200 against the version that evaluated the r_perp code at
 // every boundary of every row and bisected each split run (one warp per item):
-// 16,000 sightlines at 16 per square degree, 50 x 50 bins: 970 -> 306 ms;
-// 2,000 sightlines on 100 square degrees: 125 -> 39.9 ms; 48 sightlines (one
-// wave, where the four warps of a CTA also shorten an item): 1.58 -> 0.17 ms;
-// observing coordinates, 500 sightlines: 11.3 -> 7.3 ms.
+//                                            that  bands  + tables, pipeline
+//   16,000 sightlines at 16/deg^2, 50 x 50   970   306    237 ms
+//   2,000 sightlines on 100 deg^2            125   39.9   30.9
+//   48 sightlines (one wave)                 1.58  0.17   0.18
+//   observing, 500 sightlines                11.3  7.3    6.4
+// "Tables, pipeline": rows of code edges from a level table instead of a
+// bisection (the bisection and its dependent reads took a fifth of the time),
+// boundaries read from a skewed table (one sector for four lanes), two item
+// buffers filled by bulk copies, the grid's values in shared memory.
 #include <algorithm>
 
 #include "xi_sweep.cuh"
@@ -65,21 +72,62 @@ struct BandSums {
 };
 
 // One item as its warps see it.
-template <bool SMEM>
 struct BandItem {
   int fi, fj, ni, nj;  // first grid index and pixels of the two sightlines
+  int tf, bands, per;  // first band with a pair, their number, bands per group (0 bands: the end)
+  float ap;            // Cartesian: 2 (1 - c) inv1^2
+  double c;
   const double2* P;    // prefix sums (w*delta, w) of sightline j, by column
   const double2* R;    // (w*delta, w) of sightline i, by row
   const double4* Ri;   // prefix sums of sightline i
-  double c;
-  float ap;            // Cartesian: 2 (1 - c) inv1^2
   Dest d;
 };
 
-// Row constants of the r_perp code of grid row g.
-__device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, int g) {
+// ---- the item pipeline ----------------------------------------------------
+// Two item buffers per CTA.  Warp 0 prepares item k + 1 (claims it, finds its
+// bands, starts the bulk copies of its prefix sums and row values) before its
+// share of item k; each warp goes from item to item on its own, so a warp
+// with fewer rows does not wait for the others unless it gets two items ahead.
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void bar_init(unsigned long long* b, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned long long* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void bar_arrive_tx(unsigned long long* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+// Wait for the phase of the given parity; false when kWaitLimit tries ran
+// out, each of which the hardware may suspend for about a microsecond.
+constexpr int kWaitLimit = 1 << 22;
+__device__ __forceinline__ bool bar_wait(unsigned long long* b, uint32_t parity) {
+  for (int k = 0; k < kWaitLimit; ++k) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_addr(b)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
+// into shared memory, counted on barrier b.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* b) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(b))
+               : "memory");
+}
+
+// Row constants of the r_perp code of a row of distance d1.
+__device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, float d1) {
   RowV R;
-  R.d1 = A.gU[g];
+  R.d1 = d1;
   const float p = __fmul_rn(R.d1, R.d1);
   const float err = __fmaf_rn(R.d1, R.d1, -p);  // d1*d1 = p + err exactly
   R.A1 = __fmul_rn(R.d1, ap);
@@ -87,28 +135,22 @@ __device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, int g) {
   return R;
 }
 
-// The bounds (lo, hi) of code edge m on u = 2 (1 - c) d1 d2 inv1^2 as computed
-// in FP32 without the row's rounding term: a column with u < lo has a code
-// below m and one with u >= hi has a code of at least m, for sure.  The margin
-// covers the float rounding of d1*d1 (jit_u), four times the width of the
-// FP64 re-evaluation window, and the FP32 rounding of u.
-__device__ __forceinline__ float2 edge_bounds(const PairArgs& A, int m) {
-  const float te = (m == 0) ? -1.0f : (float)m;
-  const float se = te - A.off1f;
-  if (!(se > 0.f)) return make_float2(-1.f, -1.f);  // below every column
-  const float dt = ldexpf(4.f, -A.k1) + 1e-6f * fabsf(A.off1f);
-  const float w = A.jit_u + 2.f * se * dt + dt * dt + 4e-6f * se * se;
-  return make_float2(se * se - w, se * se + w);
-}
-
-// First column in [lo, hi) of row R with code >= m (hi when there is none).
+// First column in [lo, hi) of row R with code >= m (hi when there is none),
+// eb = the edge's bounds without the margin
+// for the row's rounding term, which is part of u here: columns are compared
+// in FP32 with the edge, and the few within its margin are binned as the
+// pixel-pair kernel does.
 template <bool MINPOS>
 __device__ __forceinline__ int edge_column(const PairArgs& A, const RowV& R, const float* colx, double c,
-                                           int lo, int hi, int m, unsigned& rech) {
+                                           int lo, int hi, int m, float2 eb, unsigned& rech) {
+  const int end = hi;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (perp_code<MINPOS>(A, R, colx[mid], c, rech) >= m) hi = mid; else lo = mid + 1;
+    if (fabsf(__fmaf_rn(R.A1, colx[mid], R.dl1)) >= eb.x) hi = mid; else lo = mid + 1;
   }
+  while (lo < end && fabsf(__fmaf_rn(R.A1, colx[lo], R.dl1)) < eb.y &&
+         perp_code<MINPOS>(A, R, colx[lo], c, rech) < m)
+    ++lo;
   return lo;
 }
 
@@ -116,7 +158,7 @@ __device__ __forceinline__ int edge_column(const PairArgs& A, const RowV& R, con
 // prefix sums, for a bin whose telescoped sums cancel to rounding level: a
 // bin all of whose weights are zero sums to exactly zero this way.
 template <int COORD, bool MINPOS>
-__device__ __noinline__ void band_by_rows(const PairArgs& A, const double2* P, const double2* R, int fi, int fj,
+__device__ __noinline__ void band_by_rows(const PairArgs& A, const double2* P, const double2* R, const float* U, int fi, int fj,
                                           int nj, double c, float ap, const uint16_t* tt, int g0, int g1, int code,
                                           double* out) {
   double s[6] = {0, 0, 0, 0, 0, 0};
@@ -124,9 +166,10 @@ __device__ __noinline__ void band_by_rows(const PairArgs& A, const double2* P, c
   for (int g = g0; g < g1; ++g) {
     int lo = min(max((int)tt[g] - fj, 0), nj), hi = min(max((int)tt[A.ngp + g] - fj, 0), nj);
     if (COORD == kCart) {
-      const RowV V = code_row(A, ap, g);
-      const int e = edge_column<MINPOS>(A, V, A.gU + fj, c, lo, hi, code + 1, rech);
-      lo = edge_column<MINPOS>(A, V, A.gU + fj, c, lo, e, code, rech);
+      const RowV V = code_row(A, ap, U[g]);
+      const float4 e1 = A.edges[code + 1], e0 = A.edges[code];
+      const int e = edge_column<MINPOS>(A, V, U + fj, c, lo, hi, code + 1, make_float2(e1.z, e1.w), rech);
+      lo = edge_column<MINPOS>(A, V, U + fj, c, lo, e, code, make_float2(e0.z, e0.w), rech);
       hi = e;
     }
     if (hi <= lo) continue;
@@ -143,47 +186,75 @@ __device__ __noinline__ void band_by_rows(const PairArgs& A, const double2* P, c
   for (int f = 0; f < 6; ++f) out[f] = s[f];
 }
 
+// Add grid row g's part of X_t (edge column q; from the row `rho` on less the
+// columns below b0, which V_t no longer holds).
+__device__ __forceinline__ void add_edge_row(const PairArgs& A, const BandItem& it, int g, int q, int b0, bool past,
+                                             double lpj, BandSums& x) {
+  double2 p = it.P[q];
+  const double2 r = it.R[g - it.fi];
+  double bd = (double)q, l = A.glp[it.fj + q] - lpj;
+  int bn = q;
+  if (past) {
+    const double2 p0 = it.P[b0];
+    p.x -= p0.x;
+    p.y -= p0.y;
+    bn -= b0;
+    bd = (double)bn;
+    l -= A.glp[it.fj + b0] - lpj;
+  }
+  x.s[0] = __fma_rn(r.x, p.x, x.s[0]);
+  x.s[1] = __fma_rn(r.x, bd, x.s[1]);
+  x.s[2] += p.x;
+  x.s[3] = __fma_rn(r.y, p.y, x.s[3]);
+  x.s[4] = __fma_rn(r.y, bd, x.s[4]);
+  x.s[5] += p.y;
+  x.z = __fma_rn(0.5, __fma_rn((double)A.gl[g] - A.lmid, bd, l), x.z);
+  x.n += (uint32_t)bn;
+}
+
 // Bands t0 .. t0 + m - 1 of an item; lane = boundary t0 + lane (lane <= m).
-template <int COORD, bool MINPOS, bool SMEM>
-__device__ __forceinline__ void band_group(const PairArgs& A, const BandItem<SMEM>& it, int t0, int m, int lane,
-                                           unsigned long long* stats) {
+// U: the grid's values (in shared memory where the kernel stages them).
+template <int COORD, bool MINPOS>
+__device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it, const float* U, int t0, int m,
+                                           int lane, unsigned long long* stats) {
   const int n0 = (int)A.g.n0, n1 = (int)A.g.n1;
   const int t = t0 + min(lane, m);
   const bool bound = lane <= m;           // this lane owns a boundary
   const bool owner = lane < m && t != n0; // and a band that is binned
-  const int k = (t < n0) ? n0 - 1 - t : t - n0 - 1;
   const int fi = it.fi, fj = it.fj, nj = it.nj, ge = it.fi + it.ni;
   const float ap = it.ap;
   const uint16_t* tt = A.gtab + (size_t)t * A.ngp;         // B_t by grid row
-  const uint16_t* inv = A.ginv + (size_t)t * (A.ng + 1);   // first row with B_t >= column
-  const double* tz = A.gtz + (size_t)t * (A.ng + 1);       // prefix sums over the rows
-  const uint32_t* tb = A.gtb + (size_t)t * (A.ng + 1);
+  const uint2* ts = A.gtabs + ((size_t)(t >> 5) * A.nblk + A.gskew[t]) * 32 + (t & 31);  // the same, skewed
+  const size_t tr = (size_t)t * (A.ng + 1);
+  const uint16_t* inv = A.ginv + tr;   // first row with B_t >= column
+  const double* tz = A.gtz + tr;       // prefix sums over the rows
+  const uint32_t* tb = A.gtb + tr;
   const double lpj = A.glp[fj], dfj = (double)fj;
   // rows with 0 < b_t < nj: [z, y)
   const int z = bound ? min(max((int)inv[fj + 1], fi), ge) : fi;
   const int y = bound ? min(max((int)inv[fj + nj], fi), ge) : fi;
   const int z1 = __shfl_down_sync(kFull, z, 1), y1 = __shfl_down_sync(kFull, y, 1);
-  // codes the bands of the group can hold
-  int m0 = 1, mtop = 1;  // edges m0 .. mtop; the last is above every code unless it is n1
+  // codes the bands of the group can hold: edges m0 .. mtop, the last of them
+  // (top) above every code unless it is n1
+  int m0 = 1, mtop = 1;
   bool top = true;
   if (COORD == kCart) {
     float ulo = 1e30f, uhi = 0.f;
     if (owner && z1 < y) {  // rows of band t: from the first with b_{t+1} > 0 to the last with b_t < nj
       const int c0 = min(max((int)tt[z1] - fj, 0), nj - 1);
       const int c1 = min((int)tt[A.ngp + y - 1] - fj, nj) - 1;
-      ulo = __fmul_rn(__fmul_rn(A.gU[z1], ap), A.gU[fj + c0]);
-      uhi = __fmul_rn(__fmul_rn(A.gU[y - 1], ap), A.gU[fj + max(c1, 0)]);
+      ulo = __fmul_rn(__fmul_rn(U[z1], ap), U[fj + c0]);
+      uhi = __fmul_rn(__fmul_rn(U[y - 1], ap), U[fj + max(c1, 0)]);
     }
     ulo = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(ulo)));
     uhi = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(uhi)));
     if (ulo > uhi) return;  // no band of the group has a row
-    const float tlo = sqrtf(ulo) + A.off1f, thi = sqrtf(uhi) + A.off1f;
-    m0 = max((int)floorf(fminf(tlo, 1e9f)), 0);
-    while (m0 <= n1 && !(ulo < edge_bounds(A, m0).y)) ++m0;      // edges below every pair of the group
-    while (m0 > 0 && ulo < edge_bounds(A, m0 - 1).y) --m0;
-    if (m0 > n1) m0 = n1 + 1;  // every pair is above the axis
+    const float tlo = sqrt_approx(ulo) + A.off1f, thi = sqrt_approx(uhi) + A.off1f;
+    m0 = min(max((int)floorf(fminf(tlo, 1e9f)), 0), n1);
+    while (m0 <= n1 && !(ulo < A.edges[m0].y)) ++m0;  // edges below every pair of the group
+    while (m0 > 0 && ulo < A.edges[m0 - 1].y) --m0;
     mtop = min(max((int)floorf(fminf(thi, 1e9f)), m0), n1);
-    while (mtop < n1 && !(uhi < edge_bounds(A, mtop + 1).x)) ++mtop;  // edges above every pair
+    while (mtop < n1 && !(uhi < A.edges[mtop + 1].x)) ++mtop;  // edges above every pair
     top = mtop < n1;           // the highest codes end with the band, not with an edge
     if (top) ++mtop;
     if (m0 > mtop) m0 = mtop;  // no edge crosses the group
@@ -194,8 +265,19 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem<SME
     const uint32_t nt1 = (tb1[y1] - tb1[z1]) - (uint32_t)fj * (uint32_t)(y1 - z1) + (uint32_t)nj * (uint32_t)(y - y1);
     stats[0] += nt1 - nt;
   }
+  // rho(e): a row of [z, y] below which u < edges[e].x at column b_t, from
+  // the level table: u >= edges[e].x needs d1 d2 >= edges[e].x / ap
+  const uint16_t* lev = A.glev + (size_t)t * (A.nlev + 1);
+  const float rap = COORD == kCart ? __fdividef(A.lev_scale, ap) : 0.f;
+  auto row_bound = [&](int e) {
+    if (COORD == kObs || (top && e == mtop)) return y;
+    const float l = __fmaf_rn(A.edges[e].x, rap, A.lev_off);
+    return l >= 0.f ? min(max((int)lev[(int)fminf(l, (float)A.nlev)], z), y) : z;
+  };
   unsigned rech = 0;
-  int cur = z;
+  int cur = z, rho = row_bound(m0);
+  double tzc = tz[z], lpc = A.glp[z];
+  uint32_t tbc = tb[z];
   BandSums xp;  // X_t of the edge before
 #pragma unroll
   for (int f = 0; f < 6; ++f) xp.s[f] = 0.0;
@@ -204,31 +286,50 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem<SME
   const double bias = 4503599627370496.0 + dfj;  // 2^52 + f_j
 #pragma unroll 1
   for (int e = m0; e <= mtop; ++e) {
-    const bool last = top && e == mtop;
-    float2 eb = make_float2(0.f, 0.f);
-    int rho = y;
-    if (COORD == kCart && !last) {
-      eb = edge_bounds(A, e);
-      // rho: first row in [cur, y) with u >= eb.x at column b_t
-      int lo = cur, hi = y;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const float u = __fmul_rn(__fmul_rn(A.gU[mid], ap), A.gU[tt[mid]]);
-        if (u >= eb.x) hi = mid; else lo = mid + 1;
-      }
-      rho = lo;
-    }
-    // V: rows [cur, rho), four at a time
+    const bool last = COORD == kObs || (top && e == mtop);
+    // loads of this edge's row and the next edge's bound, used after the loop
+    const double tzr = tz[rho], lpr = A.glp[rho];
+    const uint32_t tbr = tb[rho];
+    const int rho_next = e < mtop ? row_bound(e + 1) : y;
+    // V: rows [cur, rho), four at a time.  A lane's row and column advance
+    // together, so the banks that eight lanes read side by side (one 128-byte
+    // wavefront when all differ) are set by where each starts: with lane l
+    // starting in a row of residue m l mod 8 (m odd) its columns have the
+    // residues m l + (column - row), and m = 1, 3, 5 or 7 is taken for the most
+    // different ones.  A lane idles through the rows before cur.
     double a[6] = {0, 0, 0, 0, 0, 0};
     {
-      int g = cur & ~3;
-      const uint2* tp = reinterpret_cast<const uint2*>(tt + g);
+      const int l8 = lane & 7;
+      const int lag = rho > cur ? (int)tt[cur] - cur : l8;
+      unsigned used = (1u << ((l8 + lag) & 7)) | (0x100u << ((3 * l8 + lag) & 7)) | (0x10000u << ((5 * l8 + lag) & 7)) |
+                      (0x1000000u << ((7 * l8 + lag) & 7));
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) used |= __shfl_xor_sync(kFull, used, o);
+      int mul = 1, best = __popc(used & 0xFFu);
+#pragma unroll
+      for (int q = 1; q < 4; ++q) {
+        const int n = __popc(used & (0xFFu << (8 * q)));
+        if (n > best) {
+          best = n;
+          mul = 2 * q + 1;
+        }
+      }
+      int g = cur - ((cur - mul * l8) & 7);
+      const uint2* tp = ts + (g >> 2) * 32;
+      const bool odd = g & 1, high = g & 2;  // the group's first row in its table entry
       const double2* rp = it.R + (g - fi);
       const double2* pj = it.P - fj;
+      uint2 w = __ldg(tp), wn = __ldg(tp + 32);
+      tp += 64;
 #pragma unroll 1
       for (; g < rho; g += 4, rp += 4) {
-        const uint2 w = __ldg(tp++);
-        const uint32_t x[4] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16};
+        const uint2 wp = __ldg(tp);  // two groups ahead
+        tp += 32;
+        const uint32_t u0 = high ? w.y : w.x, u1 = high ? wn.x : w.y, u2 = high ? wn.y : wn.x;
+        const uint32_t v0 = odd ? __funnelshift_r(u0, u1, 16) : u0, v1 = odd ? __funnelshift_r(u1, u2, 16) : u1;
+        const uint32_t x[4] = {v0 & 0xFFFFu, v0 >> 16, v1 & 0xFFFFu, v1 >> 16};
+        w = wn;
+        wn = wp;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           if (g + q >= cur && g + q < rho) {
@@ -244,30 +345,15 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem<SME
         }
       }
     }
-    // z sum and pair count of the same rows
-    double vz = 0.0;
-    uint32_t vn = 0;
-    if (rho > cur) {
-      vz = (tz[rho] - tz[cur]) - 0.5 * (dfj * (A.glp[rho] - A.glp[cur]) + lpj * (double)(rho - cur));
-      vn = (tb[rho] - tb[cur]) - (uint32_t)fj * (uint32_t)(rho - cur);
-    }
-    // band: boundary t + 1 less boundary t
-    const int rho1 = __shfl_down_sync(kFull, rho, 1);
-    BandSums v;
-    {
-#pragma unroll
-      for (int f = 0; f < 6; ++f) v.s[f] = __shfl_down_sync(kFull, a[f], 1) - a[f];
-      v.z = __shfl_down_sync(kFull, vz, 1) - vz;
-      v.n = __shfl_down_sync(kFull, vn, 1) - vn;
-    }
     // X: rows from rho1 in which the edge crosses the band
+    const int rho1 = __shfl_down_sync(kFull, rho, 1);
     BandSums x;
 #pragma unroll
     for (int f = 0; f < 6; ++f) x.s[f] = 0.0;
     x.z = 0.0;
     x.n = 0;
     if (owner) {
-      if (COORD == kObs || last) {
+      if (last) {
         // the band's end: rows [y1, y) with every column from b_t on
         if (y > y1) {
           const double2 p = it.P[nj];
@@ -282,134 +368,184 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem<SME
           x.z = 0.5 * ((A.glp[y] - A.glp[y1]) * dn + (A.glp[fj + nj] - lpj) * dr);
           x.n = (uint32_t)nj * (uint32_t)(y - y1);
         }
-      } else {
-        const float* colx = A.gU + fj;
+      } else if (rho1 < y) {
+        const float4 eb = A.edges[e];
+        const float* colx = U + fj;
+        const uint16_t* t1 = tt + A.ngp;
+        int b0n = tt[rho1], b1n = t1[rho1];
         for (int g = rho1; g < y; ++g) {
-          const int b0 = min(max((int)tt[g] - fj, 0), nj), b1 = min((int)tt[A.ngp + g] - fj, nj);
-          const RowV V = code_row(A, ap, g);
+          const int b0 = max(b0n - fj, 0), b1 = min(b1n - fj, nj);
+          b0n = tt[g + 1];  // (a boundary's row of the table is longer than the grid)
+          b1n = t1[g + 1];
+          const RowV V = code_row(A, ap, U[g]);
           if (__fmul_rn(V.A1, colx[b0]) >= eb.y) break;  // this row and all after it lie above the edge
-          const int q = edge_column<MINPOS>(A, V, colx, it.c, b0, b1, e, rech);
-          double2 p = it.P[q];
-          const double2 r = it.R[g - fi];
-          double bd = (double)q, lz = A.glp[fj + q];
-          int bn = q;
-          double l0 = lpj;
-          if (g >= rho) {  // V_t stopped before this row
-            const double2 p0 = it.P[b0];
-            p.x -= p0.x;
-            p.y -= p0.y;
-            bd -= (double)b0;
-            bn -= b0;
-            l0 = A.glp[fj + b0];
-          }
-          x.s[0] = __fma_rn(r.x, p.x, x.s[0]);
-          x.s[1] = __fma_rn(r.x, bd, x.s[1]);
-          x.s[2] += p.x;
-          x.s[3] = __fma_rn(r.y, p.y, x.s[3]);
-          x.s[4] = __fma_rn(r.y, bd, x.s[4]);
-          x.s[5] += p.y;
-          x.z = __fma_rn(0.5, __fma_rn((double)A.gl[g] - A.lmid, bd, lz - l0), x.z);
-          x.n += (uint32_t)bn;
+          const int q = edge_column<MINPOS>(A, V, colx, it.c, b0, b1, e, make_float2(eb.z, eb.w), rech);
+          add_edge_row(A, it, g, q, b0, g >= rho, lpj, x);
         }
       }
-      // the bin of the codes between this edge and the one before
-      const int code = (COORD == kObs) ? 0 : e - 1;
-      FAcc F;
-      F.n = v.n + x.n - xp.n;
-      if (F.n != 0u && code >= 0) {
-        const double zc = v.z + x.z - xp.z;
-        bool tiny = false;
+    }
+    // z sum and pair count of the rows [cur, rho)
+    const double vz = (tzr - tzc) - 0.5 * (dfj * (lpr - lpc) + lpj * (double)(rho - cur));
+    const uint32_t vn = (tbr - tbc) - (uint32_t)fj * (uint32_t)(rho - cur);
+    // the bin of the codes between this edge and the one before: boundary
+    // t + 1 less boundary t, and the edges' rows
+    const int code = (COORD == kObs) ? 0 : e - 1;
+    FAcc F;
+    F.n = __shfl_down_sync(kFull, vn, 1) - vn + x.n - xp.n;
+    const double zc = __shfl_down_sync(kFull, vz, 1) - vz + x.z - xp.z;
+    bool tiny = false;
 #pragma unroll
-        for (int f = 0; f < 6; ++f) {
-          F.s[f] = v.s[f] + x.s[f] - xp.s[f];
-          const double mag = fabs(a[f]) + fabs(v.s[f]) + fabs(x.s[f]) + fabs(xp.s[f]);
-          tiny = tiny || (F.s[f] != 0.0 && fabs(F.s[f]) < 0x1p-36 * mag);
-        }
-        if (tiny) {
-          double s[6];
-          band_by_rows<COORD, MINPOS>(A, it.P, it.R, fi, fj, nj, it.c, ap, tt, z1, y, code, s);
+    for (int f = 0; f < 6; ++f) {
+      const double v = __shfl_down_sync(kFull, a[f], 1) - a[f];
+      F.s[f] = v + x.s[f] - xp.s[f];
+      // a sum that cancels to rounding level may be one whose every term is zero
+      const double mag = fabs(a[f]) + fabs(v) + fabs(x.s[f]) + fabs(xp.s[f]);
+      tiny = tiny || (F.s[f] != 0.0 && fabs(F.s[f]) < 0x1p-36 * mag);
+    }
+    if (owner && F.n != 0u && code >= 0) {
+      if (tiny) {
+        double s[6];
+        band_by_rows<COORD, MINPOS>(A, it.P, it.R, U, fi, fj, nj, it.c, ap, tt, min(z1, y), y, code, s);
 #pragma unroll
-          for (int f = 0; f < 6; ++f) F.s[f] = s[f];
-        }
-        F.s[6] = __fma_rn(A.lmid, (double)F.n, zc);
-        F.code = code;
-        add_bin<COORD>(A, it.d, k, code, F);
+        for (int f = 0; f < 6; ++f) F.s[f] = s[f];
       }
+      F.s[6] = __fma_rn(A.lmid, (double)F.n, zc);
+      F.code = code;
+      add_bin<COORD>(A, it.d, (t < n0) ? n0 - 1 - t : t - n0 - 1, code, F);
     }
     xp = x;
     cur = rho;
+    rho = rho_next;
+    tzc = tzr;
+    lpc = lpr;
+    tbc = tbr;
   }
   stats[1] += rech;
 }
 
-// The arguments stay in the kernel's parameter space (__grid_constant__):
-// the inlined sweep reads them as constant-bank operands.
-template <int COORD, bool MINPOS, bool SMEM>
-__global__ void __launch_bounds__(kGridThreads, 5) grid_kernel(const __grid_constant__ PairArgs A) {
-  extern __shared__ double2 band_smem[];
-  __shared__ unsigned long long s_idx;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned long long stats[2] = {0ull, 0ull};  // pairs in bands, FP64 re-evaluations
-  unsigned long long n_taken = 0;
-  const int n0 = (int)A.g.n0, nb = 2 * n0 + 1;
+// Prepare the next owned item into `h` (all lanes of one warp; SMEM: its data
+// into buf, arriving on `full`).
+template <int COORD, bool SMEM>
+__device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double2* buf, unsigned long long* full,
+                                             int lane, unsigned long long& n_taken) {
+  const int nb = 2 * (int)A.g.n0 + 1;
+  BandItem it;
+  it.bands = 0;
   for (;;) {
-    __syncthreads();  // the last item's shared data is free
-    if (tid == 0) s_idx = atomicAdd(A.next_item, 1ull);
-    __syncthreads();
-    const unsigned long long idx = s_idx;
+    unsigned long long idx = 0;
+    if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
+    idx = __shfl_sync(kFull, idx, 0);
     if (idx >= A.n_items) break;
     if (item_owner(A, idx) != kOwnerGrid) continue;  // another kernel's item
-    if (warp == 0) ++n_taken;
+    ++n_taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
-    BandItem<SMEM> it;
     it.ni = (int)A.npix[i];
     it.nj = (int)A.npix[j];
     it.fi = (int)A.gfirst[i];
     it.fj = (int)A.gfirst[j];
+    // bands that hold a pair: b_{t+1} > 0 in the last row, b_t < nj in the first
+    int tf = nb, tl = -1;
+    const int gl = it.fi + it.ni - 1;
+    for (int b = 0; b < nb; b += 32) {
+      const int t = b + lane;
+      const bool in = t < nb && (int)A.gtab[(size_t)(t + 1) * A.ngp + gl] > it.fj &&
+                      (int)A.gtab[(size_t)t * A.ngp + it.fi] < it.fj + it.nj;
+      const unsigned q = __ballot_sync(kFull, in);
+      if (q) {
+        tf = min(tf, b + __ffs(q) - 1);
+        tl = b + 31 - __clz(q);
+      }
+    }
+    if (tl < tf) continue;
     it.c = A.item_c[idx];
     const double a = 2.0 * dsub(1.0, it.c);
     it.ap = (float)(a * A.g.inv1 * A.g.inv1);
     it.Ri = A.prefix + A.off[i] + i;
     const double2* gP = A.pre2 + A.off[j] + j;
     const double2* gR = A.row2 + A.off[i];
-    // bands that hold a pair: b_{t+1} > 0 in the last row, b_t < nj in the first
-    int tf = nb, tl = -1;
-    {
-      const int gl = it.fi + it.ni - 1;
-      for (int b = 0; b < nb; b += 32) {
-        const int t = b + lane;
-        const bool in = t < nb && (int)A.gtab[(size_t)(t + 1) * A.ngp + gl] > it.fj &&
-                        (int)A.gtab[(size_t)t * A.ngp + it.fi] < it.fj + it.nj;
-        const unsigned q = __ballot_sync(kFull, in);
-        if (q) {
-          tf = min(tf, b + __ffs(q) - 1);
-          tl = b + 31 - __clz(q);
-        }
-      }
-    }
-    if (tl < tf) continue;  // the same in every warp
-    if (SMEM) {
-      double2* sP = band_smem;
-      double2* sR = band_smem + A.max_np + 1;
-      for (int q = tid; q <= it.nj; q += kGridThreads) sP[q] = gP[q];
-      for (int q = tid; q < it.ni; q += kGridThreads) sR[q] = gR[q];
-      it.P = sP;
-      it.R = sR;
-    } else {
-      it.P = gP;
-      it.R = gR;
-    }
+    it.P = SMEM ? buf : gP;
+    it.R = SMEM ? buf + A.max_np + 1 : gR;
     const float4 ri = A.range[i], rj = A.range[j];
     it.d.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
     it.d.cell = dest_row(A, i, j);
     it.d.sep = (COORD == kObs) ? A.item_sep[idx] : 0u;
-    __syncthreads();
-    const int bands = tl - tf + 1;
-    const int groups = (bands + kBandsPerWarp - 1) / kBandsPerWarp;
-    const int per = (bands + groups - 1) / groups;
-    for (int q = warp; q * per < bands; q += kGridWarps)
-      band_group<COORD, MINPOS, SMEM>(A, it, tf + q * per, min(per, bands - q * per), lane, stats);
+    it.tf = tf;
+    it.bands = tl - tf + 1;
+    const int groups = (it.bands + kBandsPerWarp - 1) / kBandsPerWarp;
+    it.per = (it.bands + groups - 1) / groups;
+    if (lane == 0) {
+      *h = it;
+      if (SMEM) {
+        const uint32_t bp = (uint32_t)(it.nj + 1) * 16u, br = (uint32_t)it.ni * 16u;
+        bar_arrive_tx(full, bp + br);
+        bulk_load(buf, gP, bp, full);
+        bulk_load(buf + A.max_np + 1, gR, br, full);
+      } else {
+        bar_arrive(full);
+      }
+    }
+    __syncwarp();
+    return;
   }
+  if (lane == 0) {  // no item left
+    *h = it;
+    bar_arrive(full);
+  }
+  __syncwarp();
+}
+
+// The arguments stay in the kernel's parameter space (__grid_constant__):
+// the inlined sweep reads them as constant-bank operands.
+template <int COORD, bool MINPOS, bool SMEM>
+__global__ void __launch_bounds__(kGridThreads, 4) grid_kernel(const __grid_constant__ PairArgs A) {
+  extern __shared__ double2 band_smem[];
+  __shared__ BandItem s_item[2];
+  __shared__ unsigned long long s_full[2], s_empty[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int buf_len = 2 * A.max_np + 1;
+  const float* U = A.gU;
+  if (SMEM) {
+    float* u = reinterpret_cast<float*>(band_smem + 2 * (size_t)buf_len);
+    for (int g = tid; g < A.ng; g += kGridThreads) u[g] = A.gU[g];
+    U = u;
+  }
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b) {
+      bar_init(&s_full[b], 1);
+      bar_init(&s_empty[b], kGridWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  unsigned long long stats[2] = {0ull, 0ull};  // pairs in bands, FP64 re-evaluations
+  unsigned long long n_taken = 0;
+  bool ok = true, ended = false;
+  if (warp == 0) prepare_item<COORD, SMEM>(A, &s_item[0], band_smem, &s_full[0], lane, n_taken);
+  for (uint32_t k = 0;; ++k) {
+    const uint32_t b = k & 1u, parity = (k >> 1) & 1u;
+    ok = bar_wait(&s_full[b], parity);
+    if (!ok) break;
+    BandItem it = s_item[b];
+    if (it.bands == 0) break;
+    if (SMEM) {  // the same pointers, known to be in shared memory
+      it.P = band_smem + (size_t)b * buf_len;
+      it.R = it.P + A.max_np + 1;
+    }
+    if (warp == 0 && !ended) {
+      const uint32_t nb = b ^ 1u;
+      // item k - 1 (the other buffer's) is done by every warp
+      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
+      if (!ok) break;
+      prepare_item<COORD, SMEM>(A, &s_item[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0), &s_full[nb], lane,
+                                n_taken);
+      ended = s_item[nb].bands == 0;
+    }
+    for (int q = warp; q * it.per < it.bands; q += kGridWarps)
+      band_group<COORD, MINPOS>(A, it, U, it.tf + q * it.per, min(it.per, it.bands - q * it.per), lane, stats);
+    __syncwarp();
+    if (lane == 0) bar_arrive(&s_empty[b]);
+  }
+  if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
   add_counters(A, lane, stats[0], stats[1], n_taken, 9);
 }
 
@@ -417,7 +553,8 @@ __global__ void __launch_bounds__(kGridThreads, 5) grid_kernel(const __grid_cons
 // limit: as many as fit), or with `max_out` set only that limit.
 template <int COORD, bool MINPOS, bool SMEM>
 cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  const size_t smem = SMEM ? (size_t)(2 * a.max_np + 1) * sizeof(double2) : 0;
+  // two items and the grid's values
+  const size_t smem = SMEM ? 2 * (size_t)(2 * a.max_np + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float) : 0;
   auto kern = grid_kernel<COORD, MINPOS, SMEM>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -434,14 +571,16 @@ cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
   return cudaGetLastError();
 }
 
-// Longest sightline whose prefix sums and row values are staged in shared
-// memory: both fit a CTA with at least two CTAs on an SM.
-constexpr int kBandSmemPixels = 3400;
+// Items and the grid's values are staged in shared memory when two items'
+// prefix sums and row values and the values fit a CTA (227 KB), the usual
+// case: 622-pixel forests on 1,800 values take 47 KB.
+constexpr size_t kBandSmem = 224 * 1024;
 
 template <int COORD, bool MINPOS>
 cudaError_t launch_grid2(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  return a.max_np <= kBandSmemPixels ? launch_grid<COORD, MINPOS, true>(a, num_sms, ctas_per_sm, stream, max_out)
-                                     : launch_grid<COORD, MINPOS, false>(a, num_sms, ctas_per_sm, stream, max_out);
+  const bool fits = 2 * (size_t)(2 * a.max_np + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float) <= kBandSmem;
+  return fits ? launch_grid<COORD, MINPOS, true>(a, num_sms, ctas_per_sm, stream, max_out)
+              : launch_grid<COORD, MINPOS, false>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
 }  // namespace

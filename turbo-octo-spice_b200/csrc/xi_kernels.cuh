@@ -106,6 +106,15 @@ struct PairArgs {
   // the catalogue's common first-axis grid and its boundary tables (grid
   // sweep; boundary t = 0 .. 2 n0 + 1 of grid row g, k_grid_tables, engine.cu)
   const uint16_t* gtab;      // [2 n0 + 2][ngp]: B_t[g], first column of boundary t in row g
+  // gtab once more, four rows to an entry, in the order the sweep reads it:
+  // entry (t, q) is the rows 4 (q - gskew[t]) .. + 3 of boundary t, and 32
+  // boundaries lie side by side.  The lanes of a warp own neighbouring
+  // boundaries and reach a code edge near one anti-diagonal of the (row,
+  // column) plane (observing: start at one column), so with the skew their
+  // reads fall into a few consecutive sectors.
+  const uint2* gtabs;        // [(2 n0 + 2) / 32 rounded up][nblk][32]
+  const uint32_t* gskew;     // [2 n0 + 2]
+  int nblk;
   const uint16_t* ginv;      // [2 n0 + 2][ng + 1]: first row g with B_t[g] >= x
   const uint32_t* gtb;       // [2 n0 + 2][ng + 1]: sum of B_t over the rows below g (mod 2^32)
   const double* gtz;         // [2 n0 + 2][ng + 1]: sum of (l'[g'] B_t[g'] + glp[B_t[g']]) / 2 over them
@@ -116,7 +125,16 @@ struct PairArgs {
   const double2* pre2;       // prefix sums (wd, w) alone, laid out as `prefix`
   const double2* row2;       // (w*delta, w) per pixel
   double lmid;               // loglam near the middle of the grid
-  double jit_u;              // bound of the float rounding of d1*d1, times inv1^2
+  // bounds (x, y) of code edge m = 0 .. n1 on u = 2 (1 - c) d1 d2 inv1^2 as
+  // computed in FP32 without the row's rounding term: a column with u < x has
+  // a code below m and one with u >= y a code of at least m, for sure; (z, w):
+  // the same for u with the rounding term
+  const float4* edges;
+  // glev[t][l]: first row with d1 d2 >= level l at boundary t, levels uniform
+  // from the square of the smallest value: l = (d1 d2) * lev_scale + lev_off
+  const uint16_t* glev;
+  int nlev;
+  float lev_scale, lev_off;
   int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
   int max_np;                // longest sightline
   int grid_split;            // the grid kernel takes the run items whose sightlines are on the grid
