@@ -38,16 +38,6 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 
 // ---- catalogue preparation -------------------------------------------------
 
-__global__ void k_fill_pack(PixPack* p, size_t n) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-    PixPack q;
-    q.d = kSentinel;
-    q.w = 0.f;
-    q.wd = 0.0;
-    p[k] = q;
-  }
-}
-
 __global__ void k_fill(float* p, size_t n, float v) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
        k += (size_t)gridDim.x * blockDim.x)
@@ -58,7 +48,7 @@ __global__ void k_fill(float* p, size_t n, float v) {
 // w*delta (exact product of two floats in double), weights; exclusive prefix
 // sums of (w*delta, w, loglam); coordinate ranges; sortedness.
 __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t* npix,
-                       size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pack, double* wd, float* w,
+                       size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pix2, double* wd, float* w,
                        double4* prefix, double2* pre2, double2* row2, float4* range, unsigned int* flags,
                        unsigned long long* maxbits) {
   const int lane = threadIdx.x & 31;
@@ -70,6 +60,7 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
     const uint64_t po = o + (uint64_t)kPad * (s + 1);
     double4* pre = prefix + o + s;
     double2* p2 = pre2 + o + s;
+    const uint64_t o2 = o + (uint64_t)(3 * kParityPad) * s + kParityPad;  // the first even pixel
     double c0 = 0, c1 = 0, c2 = 0;
     float dmin = INFINITY, dmax = -INFINITY, lmin = INFINITY, lmax = -INFINITY;
     double mwd = 0, mw = 0, ml = 0, md = 0;
@@ -96,7 +87,7 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
         q.d = px.distance;
         q.w = px.weight;
         q.wd = v0;
-        pack[po + k] = q;
+        pix2[o2 + (k & 1u) * (((n + 1) >> 1) + kParityPad) + (k >> 1)] = q;
         dmin = fminf(dmin, px.distance);
         dmax = fmaxf(dmax, px.distance);
         lmin = fminf(lmin, px.loglam);
@@ -563,6 +554,66 @@ std::vector<float4> code_edges(const RefGrid& g, int k1, double jit) {
     e[m] = make_float4((float)(s * s - w - jit), (float)(s * s + w + jit), (float)(s * s - w), (float)(s * s + w));
   }
   return e;
+}
+
+// Smallest double x >= 0 with reached(x) (monotone), near the guess g: 0 when
+// reached(0).
+template <class Pred>
+double first_double(double g, Pred reached) {
+  if (reached(0.0)) return 0.0;
+  double x = std::max(g, 1e-300), lo = 0.0;
+  for (int k = 0; k < 64 && !reached(x); ++k) {  // up in growing steps of the last place
+    lo = x;
+    x += std::ldexp(x, k / 2 - 52);
+  }
+  while (!reached(x)) {
+    lo = x;
+    x = x * 2 + 1;
+    if (!std::isfinite(x)) return INFINITY;
+  }
+  if (lo == 0.0)
+    for (int k = 0; k < 64; ++k) {
+      const double y = x - std::ldexp(x, k / 2 - 52);
+      if (!(y > 0) || !reached(y)) {
+        lo = std::max(y, 0.0);
+        break;
+      }
+      x = y;
+    }
+  uint64_t a, b;
+  std::memcpy(&a, &lo, 8);
+  std::memcpy(&b, &x, 8);
+  while (b - a > 1) {  // over the ordered bit patterns
+    const uint64_t m = a + (b - a) / 2;
+    double y;
+    std::memcpy(&y, &m, 8);
+    if (reached(y)) b = m; else a = m;
+  }
+  std::memcpy(&x, &b, 8);
+  return x;
+}
+
+// Thresholds of the Polar codes (PairArgs::thr_r2, thr_mu2): code >= k means
+// ref_u32((x - min) * inv) >= k with t > -1 (k = 0: t > -1).
+std::vector<double> polar_thresholds(const RefGrid& g) {
+  std::vector<double> th;
+  auto code = [](double x, double min, double inv, int n) {
+    const double t = dmul(dsub(x, min), inv);
+    if (!(t > -1.0)) return -1;
+    return t >= (double)n ? n : (int)ref_u32(t);
+  };
+  for (int k = 0; k <= (int)g.n0; ++k) {
+    const double r = g.min0 + (k == 0 ? -1.0 : (double)k) / g.inv0;
+    th.push_back(first_double(r * r, [&](double r2) { return code(std::sqrt(r2), g.min0, g.inv0, (int)g.n0) >= k; }));
+  }
+  th.push_back(INFINITY);
+  for (int m = 0; m <= (int)g.n1; ++m) {
+    const double x = first_double(g.min1 + (m == 0 ? -1.0 : (double)m) / g.inv1,
+                                  [&](double mu) { return code(mu, g.min1, g.inv1, (int)g.n1) >= m; });
+    th.push_back(x * x);
+  }
+  th.push_back(INFINITY);
+  return th;
 }
 
 bool is_pow2(double v) {
@@ -1161,7 +1212,7 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   const size_t padded = total + (size_t)kPad * (n_los + 1);
   TOS_TRY(cat->d_dist_pad.alloc(padded));
   TOS_TRY(cat->d_loglam_pad.alloc(padded));
-  TOS_TRY(cat->d_pack.alloc(padded));
+  TOS_TRY(cat->d_pix2.alloc(total + (size_t)(3 * kParityPad) * n_los));
   TOS_TRY(cat->d_wd.alloc(total));
   TOS_TRY(cat->d_w.alloc(total));
   TOS_TRY(cat->d_prefix.alloc(total + n_los));
@@ -1217,9 +1268,9 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   if (omega_matter > 0) TOS_TRY(fill_distances_device(e, cat->d_raw.p, total, omega_matter, st));
   k_fill<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_dist_pad.p, padded, kSentinel);
   k_fill<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_loglam_pad.p, padded, kSentinel);
-  k_fill_pack<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_pack.p, padded);
+  TOS_CUDA_TRY(cudaMemsetAsync(cat->d_pix2.p, 0, (total + (size_t)(3 * kParityPad) * n_los) * sizeof(PixPack), st));
   k_prep<<<grid_for(e, n_los * 32, 256), 256, 0, st>>>(
-      cat->d_raw.p, cat->d_off.p, cat->d_npix.p, n_los, cat->d_dist_pad.p, cat->d_loglam_pad.p, cat->d_pack.p,
+      cat->d_raw.p, cat->d_off.p, cat->d_npix.p, n_los, cat->d_dist_pad.p, cat->d_loglam_pad.p, cat->d_pix2.p,
       cat->d_wd.p, cat->d_w.p, cat->d_prefix.p, cat->d_pre2.p, cat->d_row2.p, cat->d_range.p, cat->d_flags.p,
       (unsigned long long*)cat->d_maxes.p);
   TOS_CUDA_TRY(cudaGetLastError());
@@ -1367,7 +1418,7 @@ uint64_t catalog_data_bytes(const tos_catalog* c) {
                c->d_plate_trig.bytes() + c->d_cell_grange.bytes() +
                c->d_group_cell_start.bytes() + c->d_cell_idx.bytes() + c->d_cell_start.bytes() +
                c->d_members.bytes() + c->d_npix.bytes() + c->d_off.bytes() + c->d_raw.bytes() +
-               c->d_dist_pad.bytes() + c->d_loglam_pad.bytes() + c->d_pack.bytes() + c->d_wd.bytes() +
+               c->d_dist_pad.bytes() + c->d_loglam_pad.bytes() + c->d_pix2.bytes() + c->d_wd.bytes() +
                c->d_w.bytes() +
                c->d_prefix.bytes() + c->d_pre2.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
   for (int w = 0; w < 2; ++w)
@@ -1381,7 +1432,7 @@ size_t Workspace::bytes() const {
          d_item_off.bytes() + d_item_i.bytes() + d_item_j.bytes() + d_item_sep.bytes() +
          d_item_c.bytes() + d_cell_pairs.bytes() + d_acc.bytes() + d_out.bytes() +
          d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_ginv.bytes() + d_gtb.bytes() +
-         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
+         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_pthr.bytes() + d_pthr.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
 }
 
 // Counter words of a run: kernel counters [0, 16), the theta-edge flags of
@@ -1398,13 +1449,14 @@ static void CUDART_CB sweep_chunk_done(void* share) { static_cast<SweepShare*>(s
 // Fixed-point scales for kernels whose FP64 register sums can hold a whole
 // item's pairs of a bin (at most max_np^2 pairs): every field takes the wide
 // 62-bit conversion (the run, grid and diagonal sweeps).
-static void set_wide_scales(PairArgs& A, const tos_catalog* cat) {
+// spare: bits left free for the number of sightline pairs a row can receive.
+static void set_wide_scales(PairArgs& A, const tos_catalog* cat, int spare) {
   const double m = std::max<double>(1.0, cat->max_np);
   const double wdm = std::max(cat->max_abs_wd, 1e-300), wm = std::max(cat->max_w, 1e-300),
                lm = std::max(cat->max_l, 1e-300);
   const double bound[7] = {wdm * m * wdm, wdm * m, m * wdm, wm * m * wm, wm * m, m * wm, lm * m};
   for (int k = 0; k < 7; ++k) {
-    int f = (int)std::floor(62.0 - std::log2(bound[k] * m));
+    int f = (int)std::floor(62.0 - spare - std::log2(bound[k] * m));
     f = std::max(-60, std::min(f, 200));
     A.scale[k] = std::ldexp(1.0, f);
     A.scale_hi[k] = std::ldexp(1.0, f - 44);
@@ -1585,8 +1637,13 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     n_pixel_pairs += v;
     max_cell_pairs = std::max(max_cell_pairs, v);
   }
+  // Bits kept free below 2^62 in the values added, so that the high words
+  // (the values shifted right by 26) of a row cannot overflow: a row takes at
+  // most max_row_items sightline pairs, each below 2^62 in all (wide scales)
+  // or in each of at most max_np runs' worth (the pixel-pair kernel).
+  int spare_items = 0, spare_runs = 0;
   {
-    // the carry-free accumulators take fewer than 2^32 adds per (row, bin):
+    // at most 2^32 adds per (row, bin) (the carry-free accumulators take 2^38):
     // a sightline pair makes at most kMaxAddsPerItemBin * max_np of them
     std::vector<uint64_t> cell_items(nc, 0);
     for (uint32_t s = 0; s < nm; ++s) cell_items[cat->cell_idx[s]] += prim_items[s];
@@ -1595,6 +1652,9 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       max_row_items = plan->max_row_items(cell_items);
     else
       for (uint64_t v : cell_items) max_row_items = std::max(max_row_items, v);
+    const double rows = (double)std::max<uint64_t>(1, max_row_items);
+    spare_items = std::max(0, (int)std::ceil(std::log2(rows)) - 26);
+    spare_runs = std::max(0, (int)std::ceil(std::log2(rows * std::max<double>(1, cat->max_np))) - 26);
     const double adds = (double)max_row_items * kMaxAddsPerItemBin * std::max<double>(1, cat->max_np);
     if (!(adds < 4294967296.0))
       return fail(TOS_ERR_UNSUPPORTED,
@@ -1643,7 +1703,8 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   A.npix = cat->d_npix.p;
   A.dist_pad = cat->d_dist_pad.p;
   A.loglam_pad = cat->d_loglam_pad.p;
-  A.pack = cat->d_pack.p;
+  A.pix2 = cat->d_pix2.p;
+  A.max_np = (int)cat->max_np;
   A.wd = cat->d_wd.p;
   A.w = cat->d_w.p;
   A.prefix = cat->d_prefix.p;
@@ -1676,7 +1737,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
                  lm = std::max(cat->max_l, 1e-300);
     const double bound[7] = {wdm * m * wdm, wdm * m, m * wdm, wm * m * wm, wm * m, m * wm, lm * m};
     for (int k = 0; k < 7; ++k) {
-      const double top = (k < kSigned) ? 62.0 : 42.0;
+      const double top = (k < kSigned) ? 62.0 - spare_runs : 42.0;
       int f = (int)std::floor(top - std::log2(bound[k]));
       f = std::max(-60, std::min(f, 200));
       A.scale[k] = std::ldexp(1.0, f);
@@ -1789,7 +1850,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       TOS_CUDA_TRY(cudaMemcpyAsync(ws->d_thr.p, thr.data(), (n0 + 1) * sizeof(float),
                                    cudaMemcpyHostToDevice, st));
       A.thr = ws->d_thr.p;
-      set_wide_scales(A, cat);
+      set_wide_scales(A, cat, spare_items);
       A.run_split = 1;
     }
   }
@@ -1852,7 +1913,6 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       A.gfirst = cat->d_gfirst[w].p;
       A.ng = ng;
       A.ngp = ngp;
-      A.max_np = (int)cat->max_np;
       A.grid_split = 1;
       use_grid = true;
     }
@@ -1860,14 +1920,23 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // --- diagonal sweep (Polar, sorted sightlines): every item whose z index is
   // constant.  Its lanes add one run of pairs at a time, so the adds to one
   // (row, bin) are at most the row's pixel pairs, which must stay below the
-  // 2^32 adds the carry-free sums take.
+  // 2^38 adds the carry-free sums take.
   bool use_diag = false;
+  std::vector<double> pthr;  // kept until the stream sync
   if (G.type == TOS_POLAR && cat->sorted && !A.force_exact && n_items > 0) {
     const uint64_t max_row_pairs =
         plan ? plan->max_row_items(std::vector<uint64_t>(cell_pairs.begin(), cell_pairs.end())) : max_cell_pairs;
-    if (max_row_pairs < (1ull << 32)) {
-      set_wide_scales(A, cat);
+    if (max_row_pairs < (1ull << 38)) {
+      set_wide_scales(A, cat, spare_items);
       A.diag_split = 1;
+      A.jit2 = (float)(std::ldexp(cat->max_d * cat->max_d, -24) * 1.01 + 1e-6);
+      A.eps0 = 5e-4f + 1e-6f * (float)n0;
+      A.eps1 = 5e-4f + 1e-6f * (float)n1;
+      pthr = polar_thresholds(rg);
+      TOS_TRY(ws->d_pthr.alloc(pthr.size()));
+      TOS_CUDA_TRY(cudaMemcpyAsync(ws->d_pthr.p, pthr.data(), pthr.size() * 8, cudaMemcpyHostToDevice, st));
+      A.thr_r2 = ws->d_pthr.p;
+      A.thr_mu2 = ws->d_pthr.p + n0 + 2;
       use_diag = true;
     }
   }

@@ -86,6 +86,7 @@ struct Workspace {
   DevBuf<uint32_t> d_gtb, d_gskew;
   DevBuf<uint2> d_gtabs;
   DevBuf<float4> d_edges;
+  DevBuf<double> d_pthr;                          // Polar bin thresholds
   DevBuf<double> d_gtz;
   DevBuf<unsigned char> d_cub_tmp;
   // the last completed per-cell run in d_acc
@@ -149,7 +150,7 @@ struct tos_catalog {
   tos::DevBuf<uint64_t> d_off;      // compact offset (per-pixel double/float arrays)
   tos::DevBuf<tos_pixel> d_raw;     // uploaded pixels, compact order
   tos::DevBuf<float> d_dist_pad, d_loglam_pad;
-  tos::DevBuf<tos::PixPack> d_pack;  // padded like d_dist_pad
+  tos::DevBuf<tos::PixPack> d_pix2;  // per sightline even pixels, odd pixels, padded (kParityPad)
   tos::DevBuf<double> d_wd;         // w*delta per pixel, exact in double
   tos::DevBuf<float> d_w;           // weight per pixel
   tos::DevBuf<double4> d_prefix;    // per sightline N+1 exclusive prefix sums of (w*delta, w, loglam)

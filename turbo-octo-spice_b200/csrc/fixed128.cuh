@@ -1,6 +1,6 @@
 // fixed128.cuh — reading the fixed-point sums of the accumulator rows
 // ([row][bin][kAccWords], the carry-free format described at kAccWords:
-// field f = hi * 2^32 + lo with lo at word f, hi at word 7 + f; the pair
+// field f = hi * 2^26 + lo with lo at word f, hi at word 7 + f; the pair
 // count at word 14).
 #pragma once
 
@@ -10,13 +10,13 @@ namespace tos {
 
 // Field f of one (row, bin) as a signed 128-bit integer.
 __device__ __forceinline__ __int128 acc128(const unsigned long long* base, int f) {
-  return (__int128)(long long)base[7 + f] * (__int128)4294967296ll + (__int128)base[f];
+  return (__int128)(long long)base[7 + f] * ((__int128)1 << kAccShift) + (__int128)base[f];
 }
 
-// Store v (|v| < 2^95) as field f of a row kept in the same format.
+// Store v (|v| < 2^89) as field f of a row kept in the same format.
 __device__ __forceinline__ void store128(unsigned long long* base, int f, __int128 v) {
-  base[f] = (unsigned long long)v & 0xFFFFFFFFull;
-  base[7 + f] = (unsigned long long)(long long)(v >> 32);
+  base[f] = (unsigned long long)v & kAccMask;
+  base[7 + f] = (unsigned long long)(long long)(v >> kAccShift);
 }
 
 // Signed 128-bit value as a double with one relative rounding (by magnitude).

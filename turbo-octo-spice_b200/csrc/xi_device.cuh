@@ -51,15 +51,17 @@ __device__ __forceinline__ void red_add(unsigned long long* p, unsigned long lon
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Add a signed value v (|v| < 2^95) to one field's sums {lo, hi} in the
-// carry-free format of kAccWords: lo += v mod 2^32, hi += floor(v / 2^32).
+// Add a signed value v (|v| < 2^89) to one field's sums {lo, hi} in the
+// carry-free format of kAccWords: lo += v mod 2^26, hi += floor(v / 2^26).
 __device__ __forceinline__ void add_wide(unsigned long long* lo, unsigned long long* hi, __int128 v) {
-  red_add(lo, (unsigned long long)v & 0xFFFFFFFFull);
-  const long long h = (long long)(v >> 32);
+  red_add(lo, (unsigned long long)v & kAccMask);
+  const long long h = (long long)(v >> kAccShift);
   if (h != 0) red_add(hi, (unsigned long long)h);
 }
 __device__ __forceinline__ void add128(unsigned long long* lo, unsigned long long* hi, long long q) {
-  add_wide(lo, hi, (__int128)q);
+  red_add(lo, (unsigned long long)q & kAccMask);
+  const long long h = q >> kAccShift;
+  if (h != 0) red_add(hi, (unsigned long long)h);
 }
 
 // ---- exact re-binning (reference expression order) returning the two axis

@@ -6,24 +6,84 @@
 // every few columns, so runs along rows are short.  Along a diagonal
 // (p1 + s, p2 + s) both distances grow together: r_par = d2 - d1 stays nearly
 // constant and r_perp grows slowly, so the key stays the same for tens to
-// hundreds of pairs.  A lane therefore owns one diagonal p2 - p1 = delta of
-// an item and walks it row by row: every pair is binned (FP32, with an FP64
-// re-evaluation of the reference's expression near an edge, as in the
-// pixel-pair kernel), and while the key stays the same the lane only adds
-// the two pair products w_i d_i w_j d_j and w_i w_j in FP64 registers.  The
-// other XiBin sums of a run of rows [s0, s1) on diagonal delta are
-// differences of the two sightlines' FP64 prefix sums:
+// hundreds of pairs.  A lane owns two neighbouring diagonals p2 - p1 = delta
+// and walks them in blocks of 16 rows without binning the pairs: it adds the
+// products w_i d_i w_j d_j and w_i w_j of the block in FP64 and keeps the
+// extremes of |d2 - d1| and of the FP32 r^2.  With them r and mu of every pair
+// of the block lie between bounds; when the bounds, widened by a margin over
+// every rounding of the reference's expression, fall into one key the block
+// has that key.  The other blocks (a key changes inside, about a tenth) are
+// queued per warp and swept pair by pair, 32 blocks at a time, one per lane,
+// each pair binned as in the pixel-pair kernel (FP32, FP64 near an edge).
+//
+// While the key stays the same a diagonal only adds its block sums.  The other
+// XiBin sums of a run of rows [s0, s1) are differences of the two sightlines'
+// FP64 prefix sums:
 //   di = P_i[s1] - P_i[s0],  dj = P_j[s1 + delta] - P_j[s0 + delta]  (w d, w, loglam).
-// When the key changes the run's sums go, as fixed-point values, to the
-// per-cell 128-bit sums.  The 32 lanes of a warp own 32 consecutive
-// diagonals, so a step reads one row value (broadcast) and 32 consecutive
-// column values.
+// Closed runs go through a per-warp queue, 32 at a time; eight lanes add a
+// run's eight sums to its 128-byte entry of the per-cell sums (one lane per
+// run would touch 32 lines with every add).
+//
+// A lane's two diagonals share each column (the second's column is the first's
+// one row later), and a sightline's pixels lie even ones first, then odd ones,
+// so that the lanes of a warp, two diagonals apart, read neighbouring entries.
+//
+// What bounds it: issue (52 % of cycles) and the shared-memory pipe (68 %);
+// about a third of the instructions are the block sums, a fifth each the block
+// keys and the pair-by-pair blocks (6.6 % of the pairs).
+//
+// Measured on a B200 against the version that binned every pair (one warp per
+// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 282 ms; five mocks
+// of 5,000 sightlines in all: 292 -> 167 ms; jackknife of 2,500 sightlines (its
+// few rows once went to the pixel-pair kernel: low words of 32 bits could have
+// wrapped after 2^32 adds): 363 -> 102 ms.  Block bounds from the extremes of
+// d1 d2 instead of r^2 sent twice the blocks pair by pair; one lane per run
+// with its own 15 adds touched 32 lines an add and took 30 of 46 shared-memory
+// and L1 cycles a step.
+#include "bulk_pipeline.cuh"
 #include "xi_device.cuh"
 
 namespace tos {
 namespace {
 
-constexpr int kDiagWarps = 8;  // warps per CTA
+constexpr int kDiagWarps = 8;  // warps per CTA; a CTA takes one item at a time
+constexpr int kDiagThreads = kDiagWarps * 32;
+constexpr int kDiagRows = 16;  // rows of a block
+constexpr int kDiagSpan = 64;  // diagonals of a warp's group
+constexpr int kQueue = 64;     // runs or blocks a warp holds (taken 32 at a time)
+
+// A warp's queues and the staging of the sums of 32 runs.
+struct WarpQ {
+  double didj[kQueue], wgt[kQueue];
+  double val[8][33];  // a row longer by one: a key's eight fields lie in different banks
+  uint32_t key[kQueue];
+  int s0[kQueue], s1[kQueue], delta[kQueue];
+  // blocks to sweep pair by pair (first row, diagonal), each with the run its
+  // diagonal had open before it
+  int2 block[kQueue];
+  uint32_t bkey[kQueue];
+  int bs0[kQueue];
+  double bdidj[kQueue], bwgt[kQueue];
+};
+
+// Per-item constants.
+struct DItem {
+  uint32_t cell, zb;
+  int ni, nj;
+  int dlo, groups;       // first diagonal and number of 64-diagonal groups (0: the end)
+  float ap;              // 2(1 - c)
+  double c;
+  const double4* prei;   // prefix sums of the two sightlines
+  const double4* prej;
+  const PixPack* rows;   // padded pixels of sightline i, even ones first
+  const PixPack* cols;   // padded pixels of sightline j, even ones first
+};
+
+// Entry of pixel p (0 of the even ones at kParityPad; kParityPad entries of
+// zero weight beside each half) in the even-first order of n pixels.
+__device__ __forceinline__ int parity_slot(int p, int n) {
+  return kParityPad + (p & 1) * (((n + 1) >> 1) + kParityPad) + (p >> 1);
+}
 
 // Row values of the pixel-pair kernel's Polar fast path (xi_kernels.cu
 // fast_bin): x1 = d1, A1 = d1 * 2(1 - c), dl1 = -(d1*d1 - fl(d1*d1)).
@@ -35,7 +95,8 @@ struct DRow {
 // whether it lies within 2^-K bins of an edge (or r^2 is tiny) and must be
 // re-binned in FP64.  The same decision as xi_kernels.cu fast_bin.
 template <bool MINPOS>
-__device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, float x2, bool& recheck) {
+__device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, float x2, bool& recheck, int& c0,
+                                              int& c1) {
   const float s = __fsub_rn(x2, R.x1);
   const float r2 = __fmaf_rn(s, s, __fmaf_rn(R.A1, x2, R.dl1));
   const float rs = rsqrt_approx(r2);
@@ -51,6 +112,8 @@ __device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, 
     coarse = coarse && (t0 > -2.0f) && (t1 > -2.0f);
   }
   int b0 = q0 >> A.k0, b1 = q1 >> A.k1;
+  c0 = b0;
+  c1 = b1;
   if (MINPOS) {
     b0 = max(b0, 0);
     b1 = max(b1, 0);
@@ -60,8 +123,61 @@ __device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, 
   return valid ? (((uint32_t)b0 << 16) | (uint32_t)b1) : kInvalidKey;
 }
 
+// Exact key of a pair near an edge whose FP32 codes are b0, b1 (each within
+// one of the exact code): the reference's r^2 against the smallest r^2 of each
+// r code (thr_r2), and |d2 - d1|^2 against thr_mu^2 r^2, where mu's rounding
+// cannot matter beyond 1e-14 relative; closer than that, or at a tiny r, the
+// reference's own expression decides.
+__device__ __noinline__ uint32_t polar_key_exact(const PairArgs& A, float d1, float d2, double c, int b0, int b1) {
+  const double r1_sq = (double)fmul(d1, d1);
+  const double two_r1_cos12 = dmul((double)fmul(2.0f, d1), c);
+  const double r_sq = dadd(r1_sq, dmul(dsub((double)d2, two_r1_cos12), (double)d2));
+  const double s = (double)fabsf(fsub(d1, d2)), s2 = s * s;
+  const int n0 = (int)A.g.n0, n1 = (int)A.g.n1;
+  const int a0 = min(max(b0, 0), n0), a1 = min(max(b1, 0), n1);
+  const int e0 = a0 - 1 + (r_sq >= A.thr_r2[a0] ? 1 : 0) + (r_sq >= A.thr_r2[a0 + 1] ? 1 : 0);
+  const double ma = A.thr_mu2[a1] * r_sq, mb = A.thr_mu2[a1 + 1] * r_sq;
+  const bool close = fabs(s2 - ma) <= 1e-14 * s2 || fabs(s2 - mb) <= 1e-14 * s2;
+  if (close || !(r_sq > 1e-6)) {
+    uint32_t p0 = 0, p1 = 0;
+    return exact_polar(d1, d2, c, A.g, &p0, &p1) ? ((p0 << 16) | p1) : kInvalidKey;
+  }
+  const int e1 = a1 - 1 + (s2 >= ma ? 1 : 0) + (s2 >= mb ? 1 : 0);
+  return (unsigned)e0 < (unsigned)n0 && (unsigned)e1 < (unsigned)n1 ? (((uint32_t)e0 << 16) | (uint32_t)e1)
+                                                                     : kInvalidKey;
+}
+
+// Key of every pair with slo <= |d2 - d1| <= shi and r2lo <= r^2 <= r2hi, r^2 =
+// (d2 - d1)^2 + 2(1 - c) d1 d2 in FP32: the packed key, kInvalidKey when no such
+// pair is binned, or kMixedKey when the bounds do not settle it.  The
+// reference's r^2 differs by the float rounding of d1*d1 (at most A.jit2);
+// 3e-6 relative and A.eps0, A.eps1 bins cover the FP32 evaluation here and the
+// rounding of the reference's.
+constexpr uint32_t kMixedKey = 0xFFFFFFFEu;
+template <bool MINPOS>
+__device__ __forceinline__ uint32_t block_key(const PairArgs& A, float slo, float shi, float r2lo, float r2hi) {
+  r2lo = __fmaf_rn(r2lo, 1.f - 3e-6f, -A.jit2);
+  r2hi = __fmaf_rn(r2hi, 1.f + 3e-6f, A.jit2);
+  if (!(r2lo >= A.r2_small)) return kMixedKey;
+  const float ia = rsqrt_approx(r2lo), ib = rsqrt_approx(r2hi);
+  const float t0a = __fmaf_rn(r2lo * ia, A.inv0f, A.off0f - A.eps0);
+  const float t0b = __fmaf_rn(r2hi * ib, A.inv0f, A.off0f + A.eps0);
+  if (t0a >= A.n0f) return kInvalidKey;
+  const float t1a = __fmaf_rn(slo * ib, A.inv1f, A.off1f - A.eps1);
+  const float t1b = __fmaf_rn(shi * ia, A.inv1f, A.off1f + A.eps1);
+  if (t1a >= A.n1f) return kInvalidKey;
+  bool ok = (t0b < A.n0f) && (t1b < A.n1f);
+  if (MINPOS) {
+    if (t0b <= -1.f || t1b <= -1.f) return kInvalidKey;
+    ok = ok && t0a > -1.f && t1a > -1.f;
+  }
+  const int b0 = (int)t0a, b1 = (int)t1a;  // toward zero: (-1, 0) is bin 0
+  ok = ok && b0 == (int)t0b && b1 == (int)t1b;
+  return ok ? (((uint32_t)b0 << 16) | (uint32_t)b1) : kMixedKey;
+}
+
 // Warp-sum the kernel's counters into A.counters[0] (evaluated pairs), [1]
-// (FP64 re-evaluations) and [12] (items taken, the same count in every lane).
+// (FP64 re-evaluations) and [12] (items taken).
 __device__ __forceinline__ void add_counters_diag(const PairArgs& A, int lane, unsigned long long n_eval,
                                                   unsigned long long n_recheck, unsigned long long n_taken) {
 #pragma unroll
@@ -76,127 +192,139 @@ __device__ __forceinline__ void add_counters_diag(const PairArgs& A, int lane, u
   }
 }
 
-// Per-item constants.
-struct DItem {
-  uint32_t cell, zb;
-  int ni, nj;
-  double c;
-  float ap;  // 2(1 - c)
-  const float* rowd;     // padded distances of sightline i
-  const double* rowwd;   // w*delta of i
-  const float* roww;     // w of i
-  const double4* prei;   // prefix sums of i
-  const float* cold;     // padded distances of sightline j
-  const double* colwd;
-  const float* colw;
-  const double4* prej;
-  const PixPack* rowp;   // padded (distance, weight, w*delta) of sightline i
-  const PixPack* colp;   // the same of sightline j
-};
-
-// Add the run [s0, s1) of diagonal delta with key `key` to row `cell`
-// (z index zb; prefix sums prei, prej of the item's two sightlines).
-__device__ __noinline__ void emit_diag(const PairArgs& A, uint32_t cell, uint32_t zb, const double4* prei,
-                                       const double4* prej, uint32_t key, int s0, int s1, int delta,
-                                       double didj, double wgt) {
-  const uint32_t b0 = key >> 16, b1 = key & 0xFFFFu;
-  const uint32_t idx = zb + (b1 + b0 * A.g.n1) * A.g.n2;  // as XiEstimator.cc:196-201
-  const unsigned long long m = (unsigned long long)(s1 - s0);
-  if (idx >= A.g.ntotal) {
-    atomicAdd(&A.counters[2], m);
-    return;
-  }
-  const double4 ia = prei[s0], ib = prei[s1];
-  const double4 ja = prej[s0 + delta], jb = prej[s1 + delta];
-  double v[7];
-  v[0] = didj;
-  v[1] = ib.x - ia.x;
-  v[2] = jb.x - ja.x;
-  v[3] = wgt;
-  v[4] = ib.y - ia.y;
-  v[5] = jb.y - ja.y;
-  v[6] = 0.5 * ((ib.z - ia.z) + (jb.z - ja.z));
-  unsigned long long* base = A.acc + ((size_t)cell * A.g.ntotal + idx) * kAccWords;
-#pragma unroll
-  for (int f = 0; f < 7; ++f) add128(base + f, base + 7 + f, to_fixed_wide(v[f], A.scale_hi[f]));
-  red_add(base + 14, m);
-}
-
-// A closed run of a diagonal, waiting in the warp's queue.
-struct DRun {
-  uint32_t key;
-  int s0, s1, delta;
-  double didj, wgt;
-};
-constexpr int kQueue = 64;  // runs per warp queue (drained 32 at a time)
-
-// Emit the queue entries [first, first + n) of the warp, one per lane.
-__device__ __forceinline__ void drain(const PairArgs& A, const DItem& it, const DRun* q, int first, int n,
-                                      int lane) {
+// Add the queue entries [first, first + n) of the warp to the item's row: a
+// lane works out the sums of one run, then eight lanes take a run, a field
+// each, so that the adds of a run fall into its one 128-byte entry.
+__device__ __noinline__ void drain(const PairArgs& A, const DItem& it, WarpQ& Q, int first, int n, int lane) {
   __syncwarp();
+  uint32_t at = 0xFFFFFFFFu;  // flat bin of the run
   if (lane < n) {
-    const DRun r = q[first + lane];
-    emit_diag(A, it.cell, it.zb, it.prei, it.prej, r.key, r.s0, r.s1, r.delta, r.didj, r.wgt);
+    const int e = first + lane;
+    const int delta = Q.delta[e];
+    const uint32_t key = Q.key[e];
+    // the rows of the run inside the matrix
+    const int s0 = max(Q.s0[e], -delta), s1 = min(min(Q.s1[e], it.ni), it.nj - delta);
+    if (s1 > s0) {
+      const double4 ia = it.prei[s0], ib = it.prei[s1];
+      const double4 ja = it.prej[s0 + delta], jb = it.prej[s1 + delta];
+      const uint32_t b0 = key >> 16, b1 = key & 0xFFFFu;
+      const uint32_t idx = it.zb + (b1 + b0 * A.g.n1) * A.g.n2;  // as XiEstimator.cc:196-201
+      if (idx < A.g.ntotal)
+        at = idx;
+      else
+        atomicAdd(&A.counters[2], (unsigned long long)(s1 - s0));
+      Q.val[0][lane] = Q.didj[e];
+      Q.val[1][lane] = ib.x - ia.x;
+      Q.val[2][lane] = jb.x - ja.x;
+      Q.val[3][lane] = Q.wgt[e];
+      Q.val[4][lane] = ib.y - ia.y;
+      Q.val[5][lane] = jb.y - ja.y;
+      Q.val[6][lane] = 0.5 * ((ib.z - ia.z) + (jb.z - ja.z));
+      Q.val[7][lane] = __longlong_as_double((long long)(s1 - s0));
+    }
+  }
+  __syncwarp();
+  const int f = lane & 7;
+  const double sh = A.scale_hi[min(f, 6)];
+  unsigned long long* row = A.acc + (size_t)it.cell * A.g.ntotal * kAccWords;
+#pragma unroll 2
+  for (int q = 0; q < 8; ++q) {
+    const int e = q * 4 + (lane >> 3);
+    const uint32_t idx = __shfl_sync(kFull, at, e);
+    if (idx == 0xFFFFFFFFu) continue;
+    unsigned long long* base = row + (size_t)idx * kAccWords;
+    const double v = Q.val[f][e];
+    if (f == 7)
+      red_add(base + 14, (unsigned long long)__double_as_longlong(v));
+    else
+      add128(base + f, base + 7 + f, to_fixed_wide(v, sh));
   }
   __syncwarp();
 }
 
-// Sweep diagonals delta0 .. delta0 + 31 (lane = delta - delta0) of an item
-// over the rows [s_lo, s_hi) that reach one of them.  Lanes close runs at
-// different rows, so a closed run goes to the warp's queue in shared memory
-// and the warp emits 32 of them at a time, one per lane.
+// Queue the runs of the lanes that close one; 32 waiting runs are added.
+__device__ __forceinline__ void push_run(const PairArgs& A, const DItem& it, WarpQ& Q, int& qn, bool close,
+                                         uint32_t key, int s0, int s1, int delta, double didj, double wgt, int lane) {
+  const unsigned cm = __ballot_sync(kFull, close);
+  if (cm == 0) return;
+  if (close) {
+    const int e = qn + __popc(cm & ((1u << lane) - 1u));
+    Q.key[e] = key;
+    Q.s0[e] = s0;
+    Q.s1[e] = s1;
+    Q.delta[e] = delta;
+    Q.didj[e] = didj;
+    Q.wgt[e] = wgt;
+  }
+  qn += __popc(cm);
+  if (qn >= 32) {
+    qn -= 32;
+    drain(A, it, Q, qn, 32, lane);
+  }
+}
+
+// Sweep the queued blocks [first, first + n) pair by pair, one per lane.  A
+// block usually closes one run: it is kept until the end of the block, when
+// the lanes' closed runs are queued together.
 template <bool MINPOS>
-__device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, int delta0, int dhi, int lane,
-                                           DRun* q, unsigned long long* stats) {
-  const int delta = delta0 + lane;
-  const bool lane_on = delta <= dhi;
-  const int s_lo = max(0, -(delta0 + 31));
-  const int s_hi = min(it.ni, it.nj - delta0);
-  const unsigned lt = (1u << lane) - 1u;
-  uint32_t cur = kInvalidKey;
-  int s0 = 0;
-  int qn = 0;  // queued runs (the same in every lane)
+__device__ __noinline__ void sweep_blocks(const PairArgs& A, const DItem& it, WarpQ& Q, int first, int n, int& qn,
+                                          int lane, unsigned& rech) {
+  __syncwarp();
+  int delta = 0, lo = 0, hi = 0, s0 = 0;
+  uint32_t cur = kInvalidKey;  // the run open before the block goes on in it
   double didj = 0.0, wgt = 0.0;
-  unsigned rech = 0;
-  unsigned n_eval = 0;  // at most one per row of the group
-#pragma unroll 1
-  for (int s = s_lo; s < s_hi; ++s) {
-    // p2 stays within the 32 sentinels on either side of the padded
-    // distances: p2 >= s_lo + delta0 >= -31 and p2 < s_hi + delta0 + 32 <= nj + 32
-    const int p2 = s + delta;
-    const bool in = lane_on && (unsigned)p2 < (unsigned)it.nj;
-    // one 16-byte load each: the row's (broadcast) and the lane's column's
-    // distance, weight and w*delta (padding: sentinel distance, zero weights)
-    const PixPack rp = it.rowp[s], cq = it.colp[p2];
+  if (lane < n) {
+    const int2 b = Q.block[first + lane];
+    delta = b.y;
+    lo = max(b.x, -delta);
+    hi = min(min(b.x + kDiagRows, it.ni), it.nj - delta);
+    cur = Q.bkey[first + lane];
+    s0 = Q.bs0[first + lane];
+    didj = Q.bdidj[first + lane];
+    wgt = Q.bwgt[first + lane];
+  }
+  const float ap = it.ap;
+  // rows lo, lo + 1, ... and columns lo + delta, ... alternate between the halves
+  const int oi = kParityPad + ((it.ni + 1) >> 1), oj = kParityPad + ((it.nj + 1) >> 1);
+  const PixPack* re = it.rows + kParityPad + (lo >> 1);
+  const PixPack* r0 = re + ((lo & 1) ? oi : 0);
+  const PixPack* r1 = re + ((lo & 1) ? 1 : oi);
+  const int c = lo + delta;
+  const PixPack* ce = it.cols + kParityPad + (c >> 1);
+  const PixPack* c0 = ce + ((c & 1) ? oj : 0);
+  const PixPack* c1 = ce + ((c & 1) ? 1 : oj);
+  uint32_t pkey = kInvalidKey;  // a closed run, not queued yet
+  int ps0 = 0, ps1 = 0;
+  double pd = 0.0, pw = 0.0;
+#pragma unroll 2
+  for (int k = 0; k < kDiagRows; ++k) {
+    const int s = lo + k;
+    const PixPack rp = (k & 1) ? r1[k >> 1] : r0[k >> 1];  // past `hi`: padding or the next pixels, not used
+    const PixPack cp = (k & 1) ? c1[k >> 1] : c0[k >> 1];
     DRow R;
-    R.d1 = rp.d;
-    R.x1 = R.d1;
+    R.x1 = R.d1 = rp.d;
     const float p = __fmul_rn(R.d1, R.d1);
     R.dl1 = -__fmaf_rn(R.d1, R.d1, -p);  // -(d1*d1 - fl(d1*d1)), exact
-    R.A1 = __fmul_rn(R.d1, it.ap);
-    const float x2 = cq.d;
+    R.A1 = __fmul_rn(R.d1, ap);
     bool recheck;
-    uint32_t key = polar_key<MINPOS>(A, R, x2, recheck);
-    recheck = recheck && in;
-    if (__any_sync(kFull, recheck)) {
-      if (recheck) {
-        uint32_t e0 = 0, e1 = 0;
-        key = exact_polar(R.d1, x2, it.c, A.g, &e0, &e1) ? ((e0 << 16) | e1) : kInvalidKey;
-        ++rech;
-      }
+    int b0, b1;
+    uint32_t key = polar_key<MINPOS>(A, R, cp.d, recheck, b0, b1);
+    const bool in = s < hi;
+    if (recheck && in) {
+      key = polar_key_exact(A, R.d1, cp.d, it.c, b0, b1);
+      ++rech;
     }
-    if (!in) key = kInvalidKey;
-    n_eval += in ? 1u : 0u;
-    const bool change = key != cur;
+    const bool change = in && key != cur;
     const bool close = change && cur != kInvalidKey;
-    const unsigned cm = __ballot_sync(kFull, close);
-    if (cm) {
-      if (close) q[qn + __popc(cm & lt)] = DRun{cur, s0, s, delta, didj, wgt};
-      qn += __popc(cm);
-      if (qn >= 32) {
-        qn -= 32;
-        drain(A, it, q, qn, 32, lane);
-      }
+    // a second run closed by this block: the first one is queued now
+    if (__any_sync(kFull, close && pkey != kInvalidKey))
+      push_run(A, it, Q, qn, close && pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
+    if (close) {
+      pkey = cur;
+      ps0 = s0;
+      ps1 = s;
+      pd = didj;
+      pw = wgt;
     }
     if (change) {
       cur = key;
@@ -204,116 +332,343 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, i
       didj = 0.0;
       wgt = 0.0;
     }
-    if (key != kInvalidKey) {  // binned: p2 is a pixel of sightline j
-      didj = __fma_rn(rp.wd, cq.wd, didj);
-      wgt = __fma_rn((double)rp.w, (double)cq.w, wgt);
+    if (in) {
+      didj = __fma_rn(rp.wd, cp.wd, didj);
+      wgt = __fma_rn((double)rp.w, (double)cp.w, wgt);
     }
   }
-  // runs still open at the last row, then the queue
-  const bool close = cur != kInvalidKey;
-  const unsigned cm = __ballot_sync(kFull, close);
-  if (close) q[qn + __popc(cm & lt)] = DRun{cur, s0, s_hi, delta, didj, wgt};
-  qn += __popc(cm);
-  if (qn >= 32) {
-    qn -= 32;
-    drain(A, it, q, qn, 32, lane);
+  push_run(A, it, Q, qn, pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
+  push_run(A, it, Q, qn, cur != kInvalidKey, cur, s0, hi, delta, didj, wgt, lane);
+}
+
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// The sums and bounds of one block of kDiagRows rows (from row sb, column c of
+// the lane's first diagonal) of a lane's two diagonals; MASKED: bit k of
+// mask[m] is set where row sb + k of diagonal m lies in the matrix (the others
+// read padding of zero weight).
+struct BlockSums {
+  double bd[2], bw[2];
+  float slo[2], shi[2], r2lo[2], r2hi[2];
+};
+template <bool MASKED>
+__device__ __forceinline__ void block_sums(const DItem& it, int sb, int c, const unsigned (&mask)[2], BlockSums& B) {
+  const int oi = kParityPad + ((it.ni + 1) >> 1), oj = kParityPad + ((it.nj + 1) >> 1);  // odd half after even
+  // rows sb + k and columns c + k + 1 by parity: one pointer each, a step per two rows
+  const PixPack* re = it.rows + kParityPad + (sb >> 1);
+  const PixPack* r0 = re + ((sb & 1) ? oi : 0);
+  const PixPack* r1 = re + ((sb & 1) ? 1 : oi);
+  const PixPack* ce = it.cols + kParityPad + (c >> 1);
+  const PixPack* c0 = ce + ((c & 1) ? 1 : oj);
+  const PixPack* c1 = ce + ((c & 1) ? oj + 1 : 1);
+  PixPack ca = ce[(c & 1) ? oj : 0];
+  double wa = (double)ca.w;
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    B.bd[m] = B.bw[m] = 0.0;
+    B.slo[m] = B.r2lo[m] = 3e38f;
+    B.shi[m] = B.r2hi[m] = 0.f;
   }
-  drain(A, it, q, 0, qn, lane);
-  stats[0] += (unsigned long long)n_eval;
+  float sp[2], rp[2];  // |d2 - d1| and r^2 of the even row, taken with the odd row's
+  // (a loop of four rows: fully unrolled, the kernel's code outgrows the instruction cache)
+#pragma unroll 1
+  for (int kk = 0; kk < kDiagRows; kk += 4, r0 += 2, r1 += 2, c0 += 2, c1 += 2)
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const PixPack r = (k & 1) ? r1[k >> 1] : r0[k >> 1];
+    const PixPack cb = (k & 1) ? c1[k >> 1] : c0[k >> 1];
+    const double w1 = (double)r.w, wb = (double)cb.w;
+    const float A1 = __fmul_rn(it.ap, r.d);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const float x2 = m ? cb.d : ca.d;
+      const float s = fabsf(__fsub_rn(x2, r.d));
+      const float r2 = __fmaf_rn(s, s, __fmul_rn(A1, x2));
+      if (MASKED) {
+        if ((mask[m] >> (kk + k)) & 1u) {
+          B.slo[m] = fminf(B.slo[m], s);
+          B.shi[m] = fmaxf(B.shi[m], s);
+          B.r2lo[m] = fminf(B.r2lo[m], r2);
+          B.r2hi[m] = fmaxf(B.r2hi[m], r2);
+        }
+      } else if (k & 1) {
+        B.slo[m] = fmin3(B.slo[m], sp[m], s);
+        B.shi[m] = fmax3(B.shi[m], sp[m], s);
+        B.r2lo[m] = fmin3(B.r2lo[m], rp[m], r2);
+        B.r2hi[m] = fmax3(B.r2hi[m], rp[m], r2);
+      } else {
+        sp[m] = s;
+        rp[m] = r2;
+      }
+      B.bd[m] = __fma_rn(r.wd, m ? cb.wd : ca.wd, B.bd[m]);
+      B.bw[m] = __fma_rn(w1, m ? wb : wa, B.bw[m]);
+    }
+    ca = cb;
+    wa = wb;
+  }
+}
+
+// One diagonal of a lane: the open run.
+struct DiagRun {
+  uint32_t cur;
+  int s0;
+  double didj, wgt;
+};
+
+// Sweep diagonals d0 .. d0 + 63 of an item: lane L takes d0 + 2 L and the next.
+// `it` is the item in registers, `sh` the same in shared memory for the
+// functions called now and then.
+template <bool MINPOS>
+__device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, const DItem& sh, int d0, int lane,
+                                           WarpQ& Q, unsigned long long* stats) {
+  const int ni = it.ni, nj = it.nj;
+  const int da = d0 + 2 * lane;  // diagonals da and da + 1
+  const int s_lo = max(0, -(d0 + kDiagSpan - 1));
+  const int s_hi = min(ni, nj - d0);
+  DiagRun run[2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) run[m] = DiagRun{kInvalidKey, 0, 0.0, 0.0};
+  int qn = 0, bn = 0;  // queued runs and blocks (the same in every lane)
+  unsigned rech = 0, n_eval = 0;
+#pragma unroll 1
+  for (int sb = s_lo; sb < s_hi; sb += kDiagRows) {
+    BlockSums B;
+    unsigned mask[2] = {0xFFFFu, 0xFFFFu};
+    if (sb + kDiagRows <= ni && sb + d0 >= 0 && sb + kDiagRows + d0 + kDiagSpan - 1 <= nj) {
+      block_sums<false>(it, sb, sb + da, mask, B);  // every pair of the 64 diagonals lies in the matrix
+      n_eval += 2 * kDiagRows;
+    } else {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int lo = max(0, -(da + m) - sb), hi = min(kDiagRows, min(ni, nj - (da + m)) - sb);
+        mask[m] = hi > lo ? (1u << hi) - (1u << lo) : 0u;
+        n_eval += __popc(mask[m]);
+      }
+      block_sums<true>(it, sb, sb + da, mask, B);
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const uint32_t key =
+          mask[m] ? block_key<MINPOS>(A, B.slo[m], B.shi[m], B.r2lo[m], B.r2hi[m]) : kInvalidKey;
+      // blocks to sweep pair by pair take the open run along
+      const bool mixed = key == kMixedKey;
+      const bool change = key != run[m].cur;
+      push_run(A, sh, Q, qn, change && !mixed && run[m].cur != kInvalidKey, run[m].cur, run[m].s0, sb, da + m,
+               run[m].didj, run[m].wgt, lane);
+      const unsigned xm = __ballot_sync(kFull, mixed);
+      if (mixed) {
+        const int e = bn + __popc(xm & ((1u << lane) - 1u));
+        Q.block[e] = make_int2(sb, da + m);
+        Q.bkey[e] = run[m].cur;
+        Q.bs0[e] = run[m].s0;
+        Q.bdidj[e] = run[m].didj;
+        Q.bwgt[e] = run[m].wgt;
+      }
+      if (change) {
+        run[m].cur = mixed ? kInvalidKey : key;
+        run[m].s0 = sb;
+        run[m].didj = 0.0;
+        run[m].wgt = 0.0;
+      }
+      run[m].didj += B.bd[m];
+      run[m].wgt += B.bw[m];
+      if (xm) {
+        bn += __popc(xm);
+        if (bn >= 32) {
+          bn -= 32;
+          sweep_blocks<MINPOS>(A, sh, Q, bn, 32, qn, lane, rech);
+        }
+      }
+    }
+  }
+  // runs still open at the last row, then the queues
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+    push_run(A, sh, Q, qn, run[m].cur != kInvalidKey, run[m].cur, run[m].s0, s_hi, da + m, run[m].didj, run[m].wgt,
+             lane);
+  if (bn) sweep_blocks<MINPOS>(A, sh, Q, 0, bn, qn, lane, rech);
+  drain(A, sh, Q, 0, qn, lane);
+  stats[0] += n_eval;
   stats[1] += rech;
 }
 
-// The arguments stay in the kernel's parameter space (__grid_constant__):
-// the inlined sweep reads them as constant-bank operands, and emit_diag
-// takes them by reference without a copy.
-template <bool MINPOS>
-__global__ void __launch_bounds__(kDiagWarps * 32, 3) diag_kernel(const __grid_constant__ PairArgs A) {
-  __shared__ DRun queue[kDiagWarps][kQueue];
-  const int lane = threadIdx.x & 31;
-  DRun* q = queue[threadIdx.x >> 5];
-  unsigned long long stats[2] = {0ull, 0ull};  // evaluated pairs, FP64 re-evaluations
-  unsigned long long n_taken = 0;
+// Prepare the next owned item into `h` (all lanes of one warp; SMEM: its
+// pixels into buf), arriving on `full`.
+template <bool SMEM>
+__device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next, PixPack* buf,
+                                          unsigned long long* full, int lane, unsigned long long& n_taken) {
+  DItem it;
+  it.groups = 0;
   for (;;) {
     unsigned long long idx = 0;
     if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
     idx = __shfl_sync(kFull, idx, 0);
     if (idx >= A.n_items) break;
+    if (item_owner(A, idx) != kOwnerDiag) continue;  // the pixel-pair kernel's item
+    ++n_taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
-    const double c = A.item_c[idx];
-    DItem it;
     it.ni = (int)A.npix[i];
     it.nj = (int)A.npix[j];
-    if (it.ni == 0 || it.nj == 0) continue;
-    const float4 ri = A.range[i], rj = A.range[j];
-    const float lsum_lo = __fadd_rn(ri.z, rj.z), lsum_hi = __fadd_rn(ri.w, rj.w);
-    const double zlo = dmul(dsub(dmul(0.5, (double)lsum_lo), A.g.min2), A.g.invn2);
-    const double zhi = dmul(dsub(dmul(0.5, (double)lsum_hi), A.g.min2), A.g.invn2);
-    it.zb = zbin_of_sum(lsum_lo, A.g);
-    if (!diag_item(A, zlo, zhi, it.zb, zbin_of_sum(lsum_hi, A.g))) continue;  // the pixel-pair kernel's item
-    ++n_taken;
-    it.c = c;
-    it.cell = dest_row(A, i, j);
-    const double a = 2.0 * dsub(1.0, c);
+    it.c = A.item_c[idx];
+    const double a = 2.0 * dsub(1.0, it.c);
     it.ap = (float)a;
-    const uint64_t oi = A.off[i] + (uint64_t)kPad * (i + 1), oj = A.off[j] + (uint64_t)kPad * (j + 1);
-    it.rowd = A.dist_pad + oi;
-    it.cold = A.dist_pad + oj;
-    it.rowwd = A.wd + A.off[i];
-    it.roww = A.w + A.off[i];
-    it.colwd = A.wd + A.off[j];
-    it.colw = A.w + A.off[j];
+    const float4 ri = A.range[i], rj = A.range[j];
+    it.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
+    it.cell = dest_row(A, i, j);
     it.prei = A.prefix + A.off[i] + i;
     it.prej = A.prefix + A.off[j] + j;
-    it.rowp = A.pack + oi;
-    it.colp = A.pack + oj;
     // Column window |d1 - d2| < lim of every row (the pixel-pair kernel's
     // Polar bound: r^2 >= (d2 - d1)^2 + 2(1 - c) dmin_i dmin_j - err), and
-    // from it the diagonals that reach it: delta in [dlo, dhi].
-    float lim = A.win_lim;
-    if (A.prune && ri.x > 0.f && rj.x > 0.f) {
-      const double q = A.polar_r2 - fmax(a, 0.0) * (double)ri.x * (double)rj.x * (1.0 - 1e-6) + A.polar_e2;
-      lim = fminf(lim, (float)(sqrt(fmax(q, 0.0)) * (1.0 + 1e-6) + 1e-3));
-    }
-    int dlo = 0x7FFFFFFF, dhi = -0x7FFFFFFF;
-    if (!A.prune) {  // no window: every diagonal
-      dlo = -(it.ni - 1);
-      dhi = it.nj - 1;
-    }
-    for (int r = lane; A.prune && r < it.ni; r += 32) {
-      const float x1 = it.rowd[r];
-      int lo = 0, hi = it.nj;  // first column with fl(x1 - x2) < lim
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__fsub_rn(x1, it.cold[mid]) < lim) hi = mid; else lo = mid + 1;
+    // from it the diagonals that reach it.
+    int dlo = -(it.ni - 1), dhi = it.nj - 1;
+    if (A.prune) {
+      float lim = A.win_lim;
+      if (ri.x > 0.f && rj.x > 0.f) {
+        const double q = A.polar_r2 - fmax(a, 0.0) * (double)ri.x * (double)rj.x * (1.0 - 1e-6) + A.polar_e2;
+        lim = fminf(lim, (float)(sqrt(fmax(q, 0.0)) * (1.0 + 1e-6) + 1e-3));
       }
-      int lo2 = lo, hi2 = it.nj;  // first column with x2 >= x1 and fl(x2 - x1) >= lim
-      while (lo2 < hi2) {
-        const int mid = (lo2 + hi2) >> 1;
-        const float x2 = it.cold[mid];
-        if (x2 >= x1 && __fsub_rn(x2, x1) >= lim) hi2 = mid; else lo2 = mid + 1;
+      const float* rowd = A.dist_pad + A.off[i] + (uint64_t)kPad * (i + 1);
+      const float* cold = A.dist_pad + A.off[j] + (uint64_t)kPad * (j + 1);
+      // over stretches of rows: the window's ends grow with the row, so the
+      // first row's lower end and the last row's upper end bound a stretch
+      const int step = (it.ni + 63) >> 6;
+      dlo = 0x7FFFFFFF;
+      dhi = -0x7FFFFFFF;
+      for (int r = lane * step; r < it.ni; r += 32 * step) {
+        const int re = min(r + step, it.ni) - 1;
+        const float xa = rowd[r], xb = rowd[re];
+        int lo = 0, hi = it.nj;  // first column with fl(xa - x2) < lim
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (__fsub_rn(xa, cold[mid]) < lim) hi = mid; else lo = mid + 1;
+        }
+        int lo2 = lo, hi2 = it.nj;  // first column with x2 >= xb and fl(x2 - xb) >= lim
+        while (lo2 < hi2) {
+          const int mid = (lo2 + hi2) >> 1;
+          const float x2 = cold[mid];
+          if (x2 >= xb && __fsub_rn(x2, xb) >= lim) hi2 = mid; else lo2 = mid + 1;
+        }
+        if (lo2 > lo) {
+          dlo = min(dlo, lo - re);
+          dhi = max(dhi, lo2 - 1 - r);
+        }
       }
-      if (lo2 > lo) {
-        dlo = min(dlo, lo - r);
-        dhi = max(dhi, lo2 - 1 - r);
+      dlo = __reduce_min_sync(kFull, dlo);
+      dhi = __reduce_max_sync(kFull, dhi);
+      if (dhi < dlo) continue;
+      dlo = max(dlo, -(it.ni - 1));
+      dhi = min(dhi, it.nj - 1);
+    }
+    it.dlo = dlo;
+    it.groups = (dhi - dlo) / kDiagSpan + 1;
+    const PixPack *gi = A.pix2 + A.off[i] + (uint64_t)(3 * kParityPad) * i,
+                  *gj = A.pix2 + A.off[j] + (uint64_t)(3 * kParityPad) * j;
+    const int len = A.max_np + 3 * kParityPad;
+    it.rows = SMEM ? buf : gi;
+    it.cols = SMEM ? buf + len : gj;
+    if (lane == 0) {
+      *h = it;
+      *next = 0;
+      if (SMEM) {
+        const uint32_t bi = (uint32_t)(it.ni + 3 * kParityPad) * 16u, bj = (uint32_t)(it.nj + 3 * kParityPad) * 16u;
+        bar_arrive_tx(full, bi + bj);
+        bulk_load(buf, gi, bi, full);
+        bulk_load(buf + len, gj, bj, full);
+      } else {
+        bar_arrive(full);
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      dlo = min(dlo, __shfl_xor_sync(kFull, dlo, o));
-      dhi = max(dhi, __shfl_xor_sync(kFull, dhi, o));
-    }
-    for (int d0 = dlo; d0 <= dhi; d0 += 32) diag_group<MINPOS>(A, it, d0, dhi, lane, q, stats);
+    __syncwarp();
+    return;
   }
+  if (lane == 0) {  // no item left
+    it.groups = 0;
+    *h = it;
+    bar_arrive(full);
+  }
+  __syncwarp();
+}
+
+// The arguments stay in the kernel's parameter space (__grid_constant__):
+// the inlined sweep reads them as constant-bank operands.  Two item buffers
+// per CTA, as in the band sweep (xi_grid.cu): warp 0 prepares the next item
+// before its share of this one, and each warp takes the item's groups from a
+// counter and goes on to the next item by itself.
+template <bool MINPOS, bool SMEM>
+__global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_constant__ PairArgs A) {
+  extern __shared__ PixPack diag_smem[];  // the item buffers, then the warps' queues
+  __shared__ DItem s_item[2];
+  __shared__ int s_next[2];
+  __shared__ unsigned long long s_full[2], s_empty[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int buf_len = 2 * (A.max_np + 3 * kParityPad);
+  WarpQ& Q = reinterpret_cast<WarpQ*>(diag_smem + (SMEM ? 2 * (size_t)buf_len : 0))[warp];
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b) {
+      bar_init(&s_full[b], 1);
+      bar_init(&s_empty[b], kDiagWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  unsigned long long stats[2] = {0ull, 0ull};  // evaluated pairs, FP64 re-evaluations
+  unsigned long long n_taken = 0;
+  bool ok = true, ended = false;
+  if (warp == 0) prepare_diag<SMEM>(A, &s_item[0], &s_next[0], diag_smem, &s_full[0], lane, n_taken);
+  for (uint32_t k = 0;; ++k) {
+    const uint32_t b = k & 1u;
+    ok = bar_wait(&s_full[b], (k >> 1) & 1u);
+    if (!ok) break;
+    DItem it = s_item[b];
+    if (it.groups == 0) break;
+    if (SMEM) {  // the same pointers, known to be in shared memory
+      it.rows = diag_smem + (size_t)b * buf_len;
+      it.cols = it.rows + A.max_np + 3 * kParityPad;
+    }
+    if (warp == 0 && !ended) {
+      const uint32_t nb = b ^ 1u;
+      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);  // item k - 1 is done by every warp
+      if (!ok) break;
+      prepare_diag<SMEM>(A, &s_item[nb], &s_next[nb], diag_smem + (SMEM ? (size_t)nb * buf_len : 0),
+                         &s_full[nb], lane, n_taken);
+      ended = s_item[nb].groups == 0;
+    }
+    for (;;) {
+      int q = 0;
+      if (lane == 0) q = atomicAdd(&s_next[b], 1);
+      q = __shfl_sync(kFull, q, 0);
+      if (q >= it.groups) break;
+      diag_group<MINPOS>(A, it, s_item[b], it.dlo + q * kDiagSpan, lane, Q, stats);
+    }
+    __syncwarp();
+    if (lane == 0) bar_arrive(&s_empty[b]);
+  }
+  if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
   add_counters_diag(A, lane, stats[0], stats[1], n_taken);
 }
 
+// Two items of two padded sightlines.
+size_t diag_smem_bytes(const PairArgs& a) { return (size_t)4 * (a.max_np + 3 * kParityPad) * sizeof(PixPack); }
+
 // Persistent launch: `ctas_per_sm` CTAs per SM (0 or above the occupancy
 // limit: as many as fit), or with `max_out` set only that limit.
-template <bool MINPOS>
+template <bool MINPOS, bool SMEM>
 cudaError_t launch_diag(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
+  const size_t smem = kDiagWarps * sizeof(WarpQ) + (SMEM ? diag_smem_bytes(a) : 0);  // two items of two sightlines
+  auto kern = diag_kernel<MINPOS, SMEM>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  const cudaError_t e =
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, diag_kernel<MINPOS>, kDiagWarps * 32, 0);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kDiagThreads, smem);
   if (e != cudaSuccess) return e;
   per_sm = per_sm > 0 ? per_sm : 1;
   if (max_out) {
@@ -321,16 +676,26 @@ cudaError_t launch_diag(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
     return cudaSuccess;
   }
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-  diag_kernel<MINPOS><<<num_sms * per_sm, kDiagWarps * 32, 0, stream>>>(a);
+  kern<<<num_sms * per_sm, kDiagThreads, smem, stream>>>(a);
   return cudaGetLastError();
+}
+
+// Items are staged in shared memory when two fit a CTA beside its queues.
+constexpr size_t kDiagSmem = 224 * 1024 - kDiagWarps * sizeof(WarpQ);
+
+template <bool MINPOS>
+cudaError_t launch_diag2(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
+  return diag_smem_bytes(a) <= kDiagSmem
+             ? launch_diag<MINPOS, true>(a, num_sms, ctas_per_sm, stream, max_out)
+             : launch_diag<MINPOS, false>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
 }  // namespace
 
 cudaError_t launch_diag_kernel(const PairArgs& a, bool minpos, int num_sms, int ctas_per_sm, cudaStream_t stream,
                                int* max_out) {
-  return minpos ? launch_diag<true>(a, num_sms, ctas_per_sm, stream, max_out)
-                : launch_diag<false>(a, num_sms, ctas_per_sm, stream, max_out);
+  return minpos ? launch_diag2<true>(a, num_sms, ctas_per_sm, stream, max_out)
+                : launch_diag2<false>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
 }  // namespace tos

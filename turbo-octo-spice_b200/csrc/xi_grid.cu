@@ -54,6 +54,7 @@
 // buffers filled by bulk copies, the grid's values in shared memory.
 #include <algorithm>
 
+#include "bulk_pipeline.cuh"
 #include "xi_sweep.cuh"
 
 namespace tos {
@@ -88,41 +89,6 @@ struct BandItem {
 // bands, starts the bulk copies of its prefix sums and row values) before its
 // share of item k; each warp goes from item to item on its own, so a warp
 // with fewer rows does not wait for the others unless it gets two items ahead.
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(unsigned long long* b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(unsigned long long* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void bar_arrive_tx(unsigned long long* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
-}
-// Wait for the phase of the given parity; false when kWaitLimit tries ran
-// out, each of which the hardware may suspend for about a microsecond.
-constexpr int kWaitLimit = 1 << 22;
-__device__ __forceinline__ bool bar_wait(unsigned long long* b, uint32_t parity) {
-  for (int k = 0; k < kWaitLimit; ++k) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(b)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
-// into shared memory, counted on barrier b.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* b) {
-  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(b))
-               : "memory");
-}
 
 // Row constants of the r_perp code of a row of distance d1.
 __device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, float d1) {

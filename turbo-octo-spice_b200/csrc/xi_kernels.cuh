@@ -43,13 +43,17 @@ constexpr int kWinWords = 19;
 constexpr int kSplit = 22;      // bits in each low word of the fixed-point split
 constexpr int kSigned = 3;      // fields 0..2 are signed (3 words), 3..6 positive (2 words)
 constexpr uint32_t kSlotCap = 1024u - 64u;  // contributions per slot before the window is emptied
-// u64 words per (row, bin): field f's sum is hi[f] * 2^32 + lo[f], where
-// lo[f] (word f) is the unsigned sum of the low 32 bits of every value added
-// and hi[f] (word 7 + f) the signed sum of the values shifted right by 32.
+// u64 words per (row, bin): field f's sum is hi[f] * 2^26 + lo[f], where
+// lo[f] (word f) is the unsigned sum of the low 26 bits of every value added
+// and hi[f] (word 7 + f) the signed sum of the values shifted right by 26.
 // The format carries nothing between words, so an add is two fire-and-forget
-// atomics; lo wraps after 2^32 adds to one (row, bin), which the host rules
-// out before a run (kMaxAddsPerItemBin).  Word 14: the pair count.
+// atomics; lo wraps after 2^38 adds to one (row, bin), which the host rules
+// out before a run (kMaxAddsPerItemBin; the diagonal sweep's adds are at most
+// a row's pixel pairs), and the values of a row are scaled so that hi does not
+// overflow.  Word 14: the pair count.
 constexpr int kAccWords = 16;
+constexpr int kAccShift = 26;
+constexpr unsigned long long kAccMask = (1ull << kAccShift) - 1ull;
 // Adds one sightline pair can make to one (row, bin, field), per pixel of its
 // primary: at most two codes of a run-sweep lane per row and side, or three
 // runs of one key per row (monotone segments) plus window flushes.
@@ -63,7 +67,8 @@ struct PairArgs {
   const uint32_t* npix;      // pixels per sightline
   const float* dist_pad;     // padded distances
   const float* loglam_pad;   // padded log10 wavelengths
-  const PixPack* pack;       // padded (distance, weight, w*delta)
+  const PixPack* pix2;       // (distance, weight, w*delta) per pixel: per sightline kParityPad zeros, its even
+                             // pixels, kParityPad zeros, its odd pixels, kParityPad zeros
   const double* wd;          // w * delta (exact double) per pixel
   const float* w;            // weight per pixel
   const double4* prefix;     // per sightline, N+1 exclusive prefix sums of (wd, w, loglam)
@@ -93,6 +98,10 @@ struct PairArgs {
   float r2_small;            // Polar: squared separations below this are re-binned in FP64
   float win_lim;             // |x1 - x2| >= win_lim (float) is always rejected
   double polar_r2;           // Polar: R^2 of the largest accepted r (with margin), or 0
+  float jit2;                // Polar: bound on the float rounding of d1^2
+  float eps0, eps1;          // Polar: margin (bins) of the diagonal sweep's block bounds
+  const double* thr_r2;      // Polar: [n0 + 2] smallest r^2 of r code >= k (the last: infinity)
+  const double* thr_mu2;     // Polar: [n1 + 2] square of the smallest mu of mu code >= m (0 for none, infinity last)
   double polar_e2;           // Polar: bound on the float rounding of d1^2, plus margin
   int prune;                 // sightlines sorted: restrict columns to the r_par window
   // accumulation
