@@ -556,43 +556,6 @@ std::vector<float4> code_edges(const RefGrid& g, int k1, double jit) {
   return e;
 }
 
-// Smallest double x >= 0 with reached(x) (monotone), near the guess g: 0 when
-// reached(0).
-template <class Pred>
-double first_double(double g, Pred reached) {
-  if (reached(0.0)) return 0.0;
-  double x = std::max(g, 1e-300), lo = 0.0;
-  for (int k = 0; k < 64 && !reached(x); ++k) {  // up in growing steps of the last place
-    lo = x;
-    x += std::ldexp(x, k / 2 - 52);
-  }
-  while (!reached(x)) {
-    lo = x;
-    x = x * 2 + 1;
-    if (!std::isfinite(x)) return INFINITY;
-  }
-  if (lo == 0.0)
-    for (int k = 0; k < 64; ++k) {
-      const double y = x - std::ldexp(x, k / 2 - 52);
-      if (!(y > 0) || !reached(y)) {
-        lo = std::max(y, 0.0);
-        break;
-      }
-      x = y;
-    }
-  uint64_t a, b;
-  std::memcpy(&a, &lo, 8);
-  std::memcpy(&b, &x, 8);
-  while (b - a > 1) {  // over the ordered bit patterns
-    const uint64_t m = a + (b - a) / 2;
-    double y;
-    std::memcpy(&y, &m, 8);
-    if (reached(y)) b = m; else a = m;
-  }
-  std::memcpy(&x, &b, 8);
-  return x;
-}
-
 // Thresholds of the Polar codes (PairArgs::thr_r2, thr_mu2): code >= k means
 // ref_u32((x - min) * inv) >= k with t > -1 (k = 0: t > -1).
 std::vector<double> polar_thresholds(const RefGrid& g) {
@@ -1026,6 +989,7 @@ void tos_engine_destroy(tos_engine* e) {
   {
     DeviceGuard g(e->device);
     cudaStreamSynchronize(e->stream);
+    e->brute.release();
     for (auto& ev : e->ev) cudaEventDestroy(ev);
     cudaStreamDestroy(e->stream);
   }

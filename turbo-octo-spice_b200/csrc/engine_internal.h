@@ -4,7 +4,9 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <functional>
 #include <map>
 #include <mutex>
@@ -62,9 +64,67 @@ struct DevBuf {
   size_t bytes() const { return p ? n * sizeof(T) : 0; }
 };
 
+// Smallest double x >= 0 with reached(x) (monotone), near the guess g: 0 when
+// reached(0).
+template <class Pred>
+inline double first_double(double g, Pred reached) {
+  if (reached(0.0)) return 0.0;
+  double x = std::max(g, 1e-300), lo = 0.0;
+  for (int k = 0; k < 64 && !reached(x); ++k) {  // up in growing steps of the last place
+    lo = x;
+    x += std::ldexp(x, k / 2 - 52);
+  }
+  while (!reached(x)) {
+    lo = x;
+    x = x * 2 + 1;
+    if (!std::isfinite(x)) return INFINITY;
+  }
+  if (lo == 0.0)
+    for (int k = 0; k < 64; ++k) {
+      const double y = x - std::ldexp(x, k / 2 - 52);
+      if (!(y > 0) || !reached(y)) {
+        lo = std::max(y, 0.0);
+        break;
+      }
+      x = y;
+    }
+  uint64_t a, b;
+  std::memcpy(&a, &lo, 8);
+  std::memcpy(&b, &x, 8);
+  while (b - a > 1) {  // over the ordered bit patterns
+    const uint64_t m = a + (b - a) / 2;
+    double y;
+    std::memcpy(&y, &m, 8);
+    if (reached(y)) b = m; else a = m;
+  }
+  std::memcpy(&x, &b, 8);
+  return x;
+}
+
 }  // namespace tos
 
 namespace tos {
+
+// Device scratch of tos_brute_run and tos_brute_tune, kept on the engine
+// between calls (used under its lock) as long as it is small.
+struct BruteScratch {
+  DevBuf<float> pts;
+  DevBuf<float4> pos;
+  DevBuf<double> wd, out, th;
+  DevBuf<unsigned long long> acc, misc;
+  size_t bytes() const {
+    return pts.bytes() + pos.bytes() + wd.bytes() + out.bytes() + th.bytes() + acc.bytes() + misc.bytes();
+  }
+  void release() {
+    pts.release();
+    pos.release();
+    wd.release();
+    out.release();
+    th.release();
+    acc.release();
+    misc.release();
+  }
+};
 
 // Device scratch of one pair count, kept between runs so that a caller that
 // runs again (a server slot, the catalogue's own runs) allocates only when a
@@ -110,6 +170,7 @@ struct tos_engine {
   // (kernel variant, warps per CTA)
   std::mutex tune_mu;
   std::map<int, std::pair<int, int>> brute_tuned;
+  tos::BruteScratch brute;
   // CTAs per SM of the dominant pair-count kernel picked by TOS_XI_TUNE, by
   // (coordinate type, total bins)
   std::map<std::pair<int, int>, int> xi_tuned;
