@@ -623,36 +623,111 @@ using namespace tos;
 // Common first-axis grid of a catalogue (grid sweep, xi_grid.cu)
 // ---------------------------------------------------------------------------
 
-// One warp per sightline: grid index of pixel 0 when the sightline's values
-// are consecutive entries of the sorted distinct values U, else kNoGrid.
-__global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint32_t* npix,
-                             size_t n_los, const float* U, int ng, uint32_t* gfirst,
-                             unsigned long long* n_ok) {
+constexpr uint32_t kGapMinPixels = 48, kGapMaxSpan = 3;  // see k_grid_first
+
+// First index of the sorted values U[0..ng) that is >= x.
+__device__ __forceinline__ int grid_index(const float* U, int ng, float x) {
+  int lo = 0, hi = ng;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (U[mid] < x) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// One warp per sightline: grid index of pixel 0 and the span of grid values
+// to its last pixel when its values strictly increase (U holds them all), else
+// kNoGrid.  Gapped sightlines of few pixels, or a span of many grid values a
+// pixel, stay with the pointer sweep: on the grid a row costs its span, on the
+// pointer sweep its pixels (ms, 82k Cartesian / 180k Observing items, grid |
+// pointers: 540 of 600 values 11.6 / 17.2 | 104 / 70, 204 of 600 10.8 / 16.9 |
+// 102 / 28, 150 of 600 25 / 22 | 60 / 21; 320k / 719k items of 64 of 128
+// values 10.9 / 20.0 | 19.0 / 21.3, 43 of 128 10.5 / 19.9 | 13.0 / 15.2, 16 of
+// 64 7.3 / 12.4 | 4.6 / 6.0).  count[0]: contiguous sightlines, count[1]:
+// those with gaps, count[2]: largest span.
+__global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint32_t* npix, size_t n_los,
+                             const float* U, int ng, uint32_t* gfirst, uint32_t* gspan, unsigned long long* count) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t s = warp; s < n_los; s += nwarps) {
     const uint32_t n = npix[s];
     const float* x = xpad + off[s] + (uint64_t)kPad * (s + 1);
-    uint32_t f = kNoGrid;
+    uint32_t f = kNoGrid, span = 0;
     if (n > 0) {
-      int lo = 0, hi = ng;  // first U >= x[0]
-      const float x0 = x[0];
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (U[mid] < x0)
-          lo = mid + 1;
-        else
-          hi = mid;
+      bool up = true;
+      for (uint32_t p = lane; p + 1 < n; p += 32) up = up && x[p + 1] > x[p];
+      if (__all_sync(kFull, up)) {
+        f = (uint32_t)grid_index(U, ng, x[0]);
+        span = (uint32_t)grid_index(U, ng, x[n - 1]) - f + 1;
+        if (span != n && (n < kGapMinPixels || span > kGapMaxSpan * n)) f = kNoGrid;
       }
-      bool ok = (uint64_t)lo + n <= (uint64_t)ng;
-      for (uint32_t p = lane; ok && p < n; p += 32) ok = U[lo + p] == x[p];
-      ok = __all_sync(kFull, ok);
-      if (ok) f = (uint32_t)lo;
     }
     if (lane == 0) {
       gfirst[s] = f;
-      if (f != kNoGrid) atomicAdd(n_ok, 1ull);
+      gspan[s] = f == kNoGrid ? 0u : span;
+      if (f != kNoGrid) {
+        atomicAdd(&count[span == n ? 0 : 1], 1ull);
+        atomicMax(&count[2], (unsigned long long)span);
+      }
+    }
+  }
+}
+
+// The on-grid sightlines' pixels at their grid entries (the arrays cleared
+// before): (wd, w) and (1, (loglam - lmid) / 2).
+__global__ void k_gap_rows(const float* xpad, const float* lpad, const uint64_t* off, const uint32_t* npix,
+                           size_t n_los, const double* wd, const float* w, const float* U, int ng,
+                           const uint32_t* gfirst, double lmid, const uint64_t* gap_off, double2* row, double2* one) {
+  const int lane = threadIdx.x & 31;
+  const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
+  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  for (size_t s = warp; s < n_los; s += nwarps) {
+    const uint32_t f = gfirst[s];
+    if (f == kNoGrid) continue;
+    const uint64_t po = off[s] + (uint64_t)kPad * (s + 1);
+    for (uint32_t p = lane; p < npix[s]; p += 32) {
+      const uint64_t e = gap_off[s] + (uint32_t)grid_index(U, ng, xpad[po + p]) - f;
+      row[e] = make_double2(wd[off[s] + p], (double)w[off[s] + p]);
+      one[e] = make_double2(1.0, 0.5 * ((double)lpad[po + p] - lmid));
+    }
+  }
+}
+
+// Exclusive prefix sums over each sightline's span.  Those of (wd, w) are the
+// pixels' own, so a stretch of zero weight adds exactly nothing.
+__global__ void k_gap_prefix(size_t n_los, const uint64_t* off, const double2* pre2, const uint32_t* gspan,
+                             const uint64_t* gap_off, const double2* one, double2* pre, double2* cnt) {
+  const int lane = threadIdx.x & 31;
+  const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
+  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  for (size_t s = warp; s < n_los; s += nwarps) {
+    const uint32_t n = gspan[s];
+    if (n == 0) continue;
+    const uint64_t o = gap_off[s], po = off[s] + s;
+    double base[2] = {0, 0};
+    if (lane == 0) pre[o] = cnt[o] = make_double2(0.0, 0.0);
+    for (uint32_t b = 0; b < n; b += 32) {
+      const uint32_t k = b + lane;
+      double v[2] = {0, 0};
+      if (k < n) {
+        const double2 m = one[o + k];
+        v[0] = m.x, v[1] = m.y;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const double u = __shfl_up_sync(kFull, v[q], d);
+          if (lane >= d) v[q] += u;
+        }
+        v[q] += base[q];
+        base[q] = __shfl_sync(kFull, v[q], 31);
+      }
+      if (k < n) {
+        pre[o + k + 1] = pre2[po + (uint32_t)v[0]];
+        cnt[o + k + 1] = make_double2(v[0], v[1]);
+      }
     }
   }
 }
@@ -660,19 +735,22 @@ __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint3
 // Loglam of every grid value, and whether it is a function of the value:
 // pass 0 writes the loglam of each on-grid pixel (equal values write the same
 // one, or some one of them), pass 1 counts the pixels that differ from it.
-__global__ void k_grid_loglam(int pass, const float* lpad, const uint64_t* off, const uint32_t* npix, size_t n_los,
-                              const uint32_t* gfirst, float* gl, unsigned long long* n_bad) {
+__global__ void k_grid_loglam(int pass, const float* xpad, const float* lpad, const uint64_t* off, const uint32_t* npix,
+                              size_t n_los, const float* U, int ng, const uint32_t* gfirst, const uint32_t* gspan,
+                              float* gl, unsigned long long* n_bad) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t s = warp; s < n_los; s += nwarps) {
     const uint32_t f = gfirst[s], n = npix[s];
     if (f == kNoGrid) continue;
-    const float* l = lpad + off[s] + (uint64_t)kPad * (s + 1);
+    const float *l = lpad + off[s] + (uint64_t)kPad * (s + 1), *x = xpad + off[s] + (uint64_t)kPad * (s + 1);
+    const bool gaps = gspan[s] != n;
     unsigned bad = 0;
     for (uint32_t p = lane; p < n; p += 32) {
-      if (pass == 0) gl[f + p] = l[p];
-      else if (gl[f + p] != l[p]) bad = 1;
+      const uint32_t g = gaps ? (uint32_t)grid_index(U, ng, x[p]) : f + p;
+      if (pass == 0) gl[g] = l[p];
+      else if (gl[g] != l[p]) bad = 1;
     }
     if (bad) atomicAdd(n_bad, 1ull);
   }
@@ -834,35 +912,65 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   TOS_TRY(cat->d_grid[w].alloc(ng));
   TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_grid[w].p, uniq.p, ng * sizeof(float), cudaMemcpyDeviceToDevice, st));
   TOS_TRY(cat->d_gfirst[w].alloc(cat->n_los));
-  TOS_CUDA_TRY(cudaMemsetAsync(nsel.p, 0, sizeof(int), st));
+  TOS_TRY(cat->d_gspan[w].alloc(cat->n_los));
   DevBuf<unsigned long long> nok;
-  TOS_TRY(nok.alloc(1));
-  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 8, st));
-  k_grid_first<<<grid_for(e, cat->n_los * 32, 256), 256, 0, st>>>(
-      x, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_grid[w].p, ng, cat->d_gfirst[w].p, nok.p);
+  TOS_TRY(nok.alloc(3));
+  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 24, st));
+  const int gw = grid_for(e, cat->n_los * 32, 256);
+  k_grid_first<<<gw, 256, 0, st>>>(x, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_grid[w].p, ng,
+                                   cat->d_gfirst[w].p, cat->d_gspan[w].p, nok.p);
   TOS_CUDA_TRY(cudaGetLastError());
-  unsigned long long h = 0;
-  TOS_CUDA_TRY(cudaMemcpyAsync(&h, nok.p, 8, cudaMemcpyDeviceToHost, st));
+  unsigned long long h[3] = {0, 0, 0};
+  TOS_CUDA_TRY(cudaMemcpyAsync(h, nok.p, 24, cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h == 0) return TOS_OK;
-  // the grid sweep takes a pixel's loglam from its grid value: not usable
-  // when two pixels of one value differ in it
+  if (h[0] + h[1] == 0) return TOS_OK;
+  // for contiguous sightlines the grid sweep takes a pixel's loglam from its
+  // grid value: not usable when two pixels of one value differ in it
   TOS_TRY(cat->d_gl[w].alloc(ng));
   TOS_TRY(cat->d_glp[w].alloc(ng + 1));
   TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gl[w].p, 0, ng * sizeof(float), st));
   TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 8, st));
   for (int pass = 0; pass < 2; ++pass)
-    k_grid_loglam<<<grid_for(e, cat->n_los * 32, 256), 256, 0, st>>>(pass, cat->d_loglam_pad.p, cat->d_off.p,
-                                                                    cat->d_npix.p, cat->n_los, cat->d_gfirst[w].p,
-                                                                    cat->d_gl[w].p, nok.p);
+    k_grid_loglam<<<gw, 256, 0, st>>>(pass, x, cat->d_loglam_pad.p, cat->d_off.p, cat->d_npix.p, cat->n_los,
+                                      cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->d_gspan[w].p, cat->d_gl[w].p,
+                                      nok.p);
   TOS_CUDA_TRY(cudaGetLastError());
   unsigned long long bad = 0;
   float lmid = 0.f;
   TOS_CUDA_TRY(cudaMemcpyAsync(&bad, nok.p, 8, cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaMemcpyAsync(&lmid, cat->d_gl[w].p + ng / 2, sizeof(float), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  if (bad) return TOS_OK;
+  cat->grid_geo[w] = bad == 0;
   cat->grid_lmid[w] = (double)lmid;
+  if (h[1] || bad) {  // sightlines laid out on the grid
+    std::vector<uint32_t> span(cat->n_los);
+    TOS_CUDA_TRY(cudaMemcpy(span.data(), cat->d_gspan[w].p, span.size() * 4, cudaMemcpyDeviceToHost));
+    std::vector<uint64_t> go(cat->n_los);
+    uint64_t tot = 0;
+    for (size_t s = 0; s < cat->n_los; ++s) {
+      go[s] = tot;
+      tot += (uint64_t)span[s] + 1;
+    }
+    // 64 bytes an entry: beyond 8 GiB of them the pointer sweep keeps the items
+    if (tot <= (8ull << 30) / 64) {
+      TOS_TRY(cat->d_gap_off[w].alloc(go.size()));
+      TOS_TRY(cat->d_gap_pre[w].alloc(tot));
+      TOS_TRY(cat->d_gap_cnt[w].alloc(tot));
+      TOS_TRY(cat->d_gap_row[w].alloc(tot));
+      TOS_TRY(cat->d_gap_one[w].alloc(tot));
+      TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_gap_off[w].p, go.data(), go.size() * 8, cudaMemcpyHostToDevice, st));
+      TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gap_row[w].p, 0, tot * sizeof(double2), st));
+      TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gap_one[w].p, 0, tot * sizeof(double2), st));
+      k_gap_rows<<<gw, 256, 0, st>>>(x, cat->d_loglam_pad.p, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_wd.p,
+                                     cat->d_w.p, cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->grid_lmid[w],
+                                     cat->d_gap_off[w].p, cat->d_gap_row[w].p, cat->d_gap_one[w].p);
+      k_gap_prefix<<<gw, 256, 0, st>>>(cat->n_los, cat->d_off.p, cat->d_pre2.p, cat->d_gspan[w].p,
+                                       cat->d_gap_off[w].p, cat->d_gap_one[w].p, cat->d_gap_pre[w].p,
+                                       cat->d_gap_cnt[w].p);
+      TOS_CUDA_TRY(cudaGetLastError());
+      TOS_CUDA_TRY(cudaStreamSynchronize(st));  // `go` is read until here
+    }
+  }
   k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, ng, (double)lmid, cat->d_glp[w].p);
   TOS_CUDA_TRY(cudaGetLastError());
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -870,7 +978,9 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   TOS_CUDA_TRY(cudaMemcpyAsync(&cat->grid_hi[w], cat->d_grid[w].p + ng - 1, sizeof(float), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   cat->grid_n[w] = ng;
-  cat->grid_los[w] = h;
+  cat->max_span[w] = (uint32_t)h[2];
+  cat->grid_los[w] = h[0];
+  cat->grid_gaps[w] = h[1];
   return TOS_OK;
 }
 
@@ -1386,7 +1496,9 @@ uint64_t catalog_data_bytes(const tos_catalog* c) {
                c->d_w.bytes() +
                c->d_prefix.bytes() + c->d_pre2.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
   for (int w = 0; w < 2; ++w)
-    b += c->d_grid[w].bytes() + c->d_gl[w].bytes() + c->d_glp[w].bytes() + c->d_gfirst[w].bytes();
+    b += c->d_grid[w].bytes() + c->d_gl[w].bytes() + c->d_glp[w].bytes() + c->d_gfirst[w].bytes() +
+         c->d_gspan[w].bytes() + c->d_gap_off[w].bytes() + c->d_gap_pre[w].bytes() + c->d_gap_cnt[w].bytes() +
+         c->d_gap_row[w].bytes() + c->d_gap_one[w].bytes();
   return b;
 }
 
@@ -1557,7 +1669,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // [0..3] kernel counters, [4] pair-kernel item counter, [5] candidates,
   // [6] window flushes, [7] run-kernel item counter, [8] run items, [9] grid
   // items, [10] grid-kernel item counter, [11] diagonal-kernel item counter,
-  // [12] diagonal items, [13] a grid-kernel wait ran out,
+  // [12] diagonal items, [13] a wait of a sweep ran out, [14] gap-kernel item counter,
   // [16] theta indices on an edge, [17..] their item numbers (4096 at most)
   unsigned long long* ctr = ws->d_counters.p;
   const double theta_min = G.axis[1].min, theta_inv = 1.0 / axis_width(G.axis[1]);
@@ -1828,7 +1940,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     // the boundary tables take 20 bytes per boundary and grid value; beyond
     // 2 GiB of them the pointer sweep takes the items
     const bool tables_fit = (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 20.0 < 2147483648.0;
-    if (ng > 0 && cat->grid_los[w] > 0 && tables_fit) {
+    if (ng > 0 && tables_fit) {
       const size_t nbd = 2 * ((size_t)n0 + 1);
       const int ngp = (ng + 7) / 4 * 4;
       TOS_TRY(ws->d_gtab.alloc(nbd * ngp));
@@ -1877,8 +1989,19 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       A.gfirst = cat->d_gfirst[w].p;
       A.ng = ng;
       A.ngp = ngp;
-      A.grid_split = 1;
-      use_grid = true;
+      A.gspan = cat->d_gspan[w].p;
+      A.max_span = (int)cat->max_np;
+      // contiguous sightlines on a grid that fixes loglam; the others with gaps
+      A.grid_split = cat->grid_geo[w] && cat->grid_los[w] > 1;
+      use_grid = A.grid_split != 0;
+      if (cat->d_gap_off[w].p) {
+        A.gap_off = cat->d_gap_off[w].p;
+        A.gap_pre = cat->d_gap_pre[w].p;
+        A.gap_cnt = cat->d_gap_cnt[w].p;
+        A.gap_row = cat->d_gap_row[w].p;
+        A.gap_one = cat->d_gap_one[w].p;
+        A.gap_split = 1;
+      }
     }
   }
   // --- diagonal sweep (Polar, sorted sightlines): every item whose z index is
@@ -2006,6 +2129,13 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     TOS_CUDA_TRY(cudaEventRecord(e->ev[7], st));
     if (use_grid) TOS_TRY(sweep(false, ctr + 10));
     TOS_CUDA_TRY(cudaEventRecord(e->ev[6], st));
+    if (A.gap_split) {
+      PairArgs R = A;
+      R.next_item = ctr + 14;
+      R.max_span = (int)cat->max_span[G.type == TOS_OBSERVING ? 1 : 0];
+      const cudaError_t ge2 = launch_gap_kernel(R, G.type, minpos, e->num_sms, st);
+      if (ge2 != cudaSuccess) return fail(TOS_ERR_CUDA, std::string("gap kernel: ") + cudaGetErrorString(ge2));
+    }
     if (use_runs) {
       PairArgs R = A;
       R.next_item = ctr + 7;

@@ -239,6 +239,14 @@ struct tos_catalog {
   double grid_lmid[2] = {0, 0};                        // loglam of the middle value
   float grid_lo[2] = {0, 0}, grid_hi[2] = {0, 0};      // smallest and largest value
   tos::DevBuf<uint32_t> d_gfirst[2];                   // per sightline grid index of pixel 0 or kNoGrid
+  tos::DevBuf<uint32_t> d_gspan[2];                    // grid values from its first to its last pixel
+  uint32_t max_span[2] = {0, 0};
+  bool grid_geo[2] = {false, false};                   // loglam is a function of the grid value
+  uint64_t grid_gaps[2] = {0, 0};                      // sightlines on the grid with gaps
+  // the sightlines laid out on the grid (PairArgs::gap_*), when some have gaps
+  // or loglam is not a function of the grid value
+  tos::DevBuf<uint64_t> d_gap_off[2];
+  tos::DevBuf<double2> d_gap_pre[2], d_gap_cnt[2], d_gap_row[2], d_gap_one[2];
   // the workspace of tos_xi_run on this catalogue; its per-cell sums stay
   // there after the run for the covariance calls
   tos::Workspace run;

@@ -114,12 +114,6 @@ __device__ __forceinline__ bool run_item(const PairArgs& A, double c, bool zcons
   return zconst && dmul(2.0, dsub(1.0, c)) >= A.run_amin;
 }
 
-// Run items whose sightlines are both contiguous on the common grid: the
-// grid-sweep kernel's share when A.grid_split is set.
-__device__ __forceinline__ bool grid_item(const PairArgs& A, uint32_t i, uint32_t j) {
-  return A.grid_split && A.gfirst[i] != kNoGrid && A.gfirst[j] != kNoGrid;
-}
-
 __device__ __forceinline__ uint32_t zbin_of_sum(float lsum, const RefGrid& g) {
   return ref_u32(dmul(dsub(dmul(0.5, (double)lsum), g.min2), g.invn2));
 }
@@ -134,10 +128,9 @@ __device__ __forceinline__ bool diag_item(const PairArgs& A, double zlo, double 
 }
 
 // The kernel that takes item idx, from the predicates above as each kernel
-// applies them (load_item and grid_item for the sweeps, the pixel-pair
-// kernel's own test): one lane per item, so that a kernel can claim a batch
+// applies them (load_item for the sweeps, the pixel-pair kernel's own test): one lane per item, so that a kernel can claim a batch
 // of items and skip the others' without loading each one warp-wide.
-enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerRun, kOwnerDiag, kOwnerPair };
+enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerPair };
 __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long idx) {
   const uint32_t i = A.item_i[idx], j = A.item_j[idx];
   if (A.npix[i] == 0 || A.npix[j] == 0) return kOwnerNone;
@@ -147,7 +140,13 @@ __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long 
   const double zhi = dmul(dsub(dmul(0.5, (double)lsum_hi), A.g.min2), A.g.invn2);
   const uint32_t zb_lo = zbin_of_sum(lsum_lo, A.g), zb_hi = zbin_of_sum(lsum_hi, A.g);
   const bool zconst = zlo > -1.0 && zhi < 2147483648.0 && zb_lo == zb_hi;
-  if (A.run_split && run_item(A, A.item_c[idx], zconst)) return grid_item(A, i, j) ? kOwnerGrid : kOwnerRun;
+  if (A.run_split && run_item(A, A.item_c[idx], zconst)) {
+    if ((A.grid_split || A.gap_split) && A.gfirst[i] != kNoGrid && A.gfirst[j] != kNoGrid) {
+      if (A.grid_split && A.gspan[i] == A.npix[i] && A.gspan[j] == A.npix[j]) return kOwnerGrid;
+      if (A.gap_split) return kOwnerGaps;
+    }
+    return kOwnerRun;
+  }
   if (diag_item(A, zlo, zhi, zb_lo, zb_hi)) return kOwnerDiag;
   return kOwnerPair;
 }

@@ -32,7 +32,9 @@
 // loop (V) evaluates no bin at all: a lane owns boundary t and adds, row by
 // row, six products of its row's (w*delta, w) and sightline j's prefix sums at
 // one column.  The z sums and pair counts of a stretch of rows depend on the
-// grid alone and come from prefix tables over the rows.
+// grid alone and come from prefix tables over the rows.  Where a sightline has
+// gaps (GAPS) its missing pixels have zero weight, and pixel counts and loglam
+// sums are two more products of row values and column prefix sums.
 //
 // What bounds it: shared-memory reads and the latency of the table reads
 // around the inner loop (LSU data pipe 63 %, issue 41 %, most stalled cycles on
@@ -53,6 +55,7 @@
 // boundaries read from a skewed table (one sector for four lanes), two item
 // buffers filled by bulk copies, the grid's values in shared memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "bulk_pipeline.cuh"
 #include "xi_sweep.cuh"
@@ -60,16 +63,19 @@
 namespace tos {
 namespace {
 
-constexpr int kGridWarps = 4;  // warps per CTA; a CTA takes one item at a time
-constexpr int kGridThreads = kGridWarps * 32;
+// Warps per CTA; a CTA has two items in flight.  Sightlines with gaps take twice
+// the shared memory an item, so twice the warps share a CTA's items there.
+template <bool GAPS>
+constexpr int kGridWarps = GAPS ? 8 : 4;
 constexpr int kBandsPerWarp = 31;  // 32 boundaries
 
 // Sums of a stretch of rows: w d w d, w d, w d, w w, w, w (didj, di, dj, wgt,
 // wi, wj), the centred z sum and the pair count.
+template <bool GAPS>
 struct BandSums {
   double s[6];
   double z;
-  uint32_t n;
+  std::conditional_t<GAPS, double, uint32_t> n;
 };
 
 // One item as its warps see it.
@@ -81,6 +87,10 @@ struct BandItem {
   const double2* P;    // prefix sums (w*delta, w) of sightline j, by column
   const double2* R;    // (w*delta, w) of sightline i, by row
   const double4* Ri;   // prefix sums of sightline i
+  // sightlines with gaps (PairArgs::gap_*): column prefix sums of (pixels,
+  // l'/2), row values (1 where there is a pixel, l'/2), and the prefix sums of
+  // sightline i
+  const double2 *C, *M, *Pi, *Ci;
   Dest d;
 };
 
@@ -101,11 +111,10 @@ __device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, float d1) 
   return R;
 }
 
-// First column in [lo, hi) of row R with code >= m (hi when there is none),
-// eb = the edge's bounds without the margin
-// for the row's rounding term, which is part of u here: columns are compared
-// in FP32 with the edge, and the few within its margin are binned as the
-// pixel-pair kernel does.
+// First column in [lo, hi) of row R with code >= m (hi when there is none).
+// eb: the edge's bounds without the margin for the row's rounding term, which
+// is part of u here.  Columns are compared in FP32 with the edge, and the few
+// within its margin are binned as the pixel-pair kernel does.
 template <bool MINPOS>
 __device__ __forceinline__ int edge_column(const PairArgs& A, const RowV& R, const float* colx, double c,
                                            int lo, int hi, int m, float2 eb, unsigned& rech) {
@@ -123,39 +132,62 @@ __device__ __forceinline__ int edge_column(const PairArgs& A, const RowV& R, con
 // The six sums of band t in code c evaluated row by row from differences of
 // prefix sums, for a bin whose telescoped sums cancel to rounding level: a
 // bin all of whose weights are zero sums to exactly zero this way.
-template <int COORD, bool MINPOS>
-__device__ __noinline__ void band_by_rows(const PairArgs& A, const double2* P, const double2* R, const float* U, int fi, int fj,
-                                          int nj, double c, float ap, const uint16_t* tt, int g0, int g1, int code,
-                                          double* out) {
+template <int COORD, bool MINPOS, bool GAPS>
+__device__ __noinline__ void band_by_rows(const PairArgs& A, const BandItem& it, const float* U, const uint16_t* tt,
+                                          int g0, int g1, int code, double* out) {
   double s[6] = {0, 0, 0, 0, 0, 0};
   unsigned rech = 0;
+  const int fi = it.fi, fj = it.fj, nj = it.nj;
   for (int g = g0; g < g1; ++g) {
     int lo = min(max((int)tt[g] - fj, 0), nj), hi = min(max((int)tt[A.ngp + g] - fj, 0), nj);
     if (COORD == kCart) {
-      const RowV V = code_row(A, ap, U[g]);
+      const RowV V = code_row(A, it.ap, U[g]);
       const float4 e1 = A.edges[code + 1], e0 = A.edges[code];
-      const int e = edge_column<MINPOS>(A, V, U + fj, c, lo, hi, code + 1, make_float2(e1.z, e1.w), rech);
-      lo = edge_column<MINPOS>(A, V, U + fj, c, lo, e, code, make_float2(e0.z, e0.w), rech);
+      const int e = edge_column<MINPOS>(A, V, U + fj, it.c, lo, hi, code + 1, make_float2(e1.z, e1.w), rech);
+      lo = edge_column<MINPOS>(A, V, U + fj, it.c, lo, e, code, make_float2(e0.z, e0.w), rech);
       hi = e;
     }
     if (hi <= lo) continue;
-    const double2 a = P[lo], b = P[hi], r = R[g - fi];
-    const double m = (double)(hi - lo), dwd = b.x - a.x, dw = b.y - a.y;
+    const double2 a = it.P[lo], b = it.P[hi], r = it.R[g - fi];
+    const double m = GAPS ? it.C[hi].x - it.C[lo].x : (double)(hi - lo), dwd = b.x - a.x, dw = b.y - a.y;
+    const double one = GAPS ? it.M[g - fi].x : 1.0;
     s[0] += r.x * dwd;
     s[1] += r.x * m;
-    s[2] += dwd;
+    s[2] += one * dwd;
     s[3] += r.y * dw;
     s[4] += r.y * m;
-    s[5] += dw;
+    s[5] += one * dw;
   }
 #pragma unroll
   for (int f = 0; f < 6; ++f) out[f] = s[f];
 }
 
+// Add the row values r (and m: with gaps) times the column sums p (and c).
+__device__ __forceinline__ void add_gap_row(double (&a)[8], double2 r, double2 m, double2 p, double2 c) {
+  a[0] = __fma_rn(r.x, p.x, a[0]);
+  a[1] = __fma_rn(r.x, c.x, a[1]);
+  a[2] = __fma_rn(m.x, p.x, a[2]);
+  a[3] = __fma_rn(r.y, p.y, a[3]);
+  a[4] = __fma_rn(r.y, c.x, a[4]);
+  a[5] = __fma_rn(m.x, p.y, a[5]);
+  a[6] = __fma_rn(m.y, c.x, __fma_rn(m.x, c.y, a[6]));
+  a[7] = __fma_rn(m.x, c.x, a[7]);
+}
+
+// The same into X_t, of one row or of the sums of several.
+__device__ __forceinline__ void add_gap_row(BandSums<true>& x, double2 r, double2 m, double2 p, double2 c) {
+  double a[8] = {x.s[0], x.s[1], x.s[2], x.s[3], x.s[4], x.s[5], x.z, x.n};
+  add_gap_row(a, r, m, p, c);
+#pragma unroll
+  for (int f = 0; f < 6; ++f) x.s[f] = a[f];
+  x.z = a[6];
+  x.n = a[7];
+}
+
 // Add grid row g's part of X_t (edge column q; from the row `rho` on less the
 // columns below b0, which V_t no longer holds).
 __device__ __forceinline__ void add_edge_row(const PairArgs& A, const BandItem& it, int g, int q, int b0, bool past,
-                                             double lpj, BandSums& x) {
+                                             double lpj, BandSums<false>& x) {
   double2 p = it.P[q];
   const double2 r = it.R[g - it.fi];
   double bd = (double)q, l = A.glp[it.fj + q] - lpj;
@@ -178,9 +210,22 @@ __device__ __forceinline__ void add_edge_row(const PairArgs& A, const BandItem& 
   x.n += (uint32_t)bn;
 }
 
+__device__ __forceinline__ void add_edge_row(const PairArgs&, const BandItem& it, int g, int q, int b0, bool past,
+                                             double, BandSums<true>& x) {
+  double2 p = it.P[q], c = it.C[q];
+  if (past) {
+    const double2 p0 = it.P[b0], c0 = it.C[b0];
+    p.x -= p0.x;
+    p.y -= p0.y;
+    c.x -= c0.x;
+    c.y -= c0.y;
+  }
+  add_gap_row(x, it.R[g - it.fi], it.M[g - it.fi], p, c);
+}
+
 // Bands t0 .. t0 + m - 1 of an item; lane = boundary t0 + lane (lane <= m).
 // U: the grid's values (in shared memory where the kernel stages them).
-template <int COORD, bool MINPOS>
+template <int COORD, bool MINPOS, bool GAPS>
 __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it, const float* U, int t0, int m,
                                            int lane, unsigned long long* stats) {
   const int n0 = (int)A.g.n0, n1 = (int)A.g.n1;
@@ -195,7 +240,7 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
   const uint16_t* inv = A.ginv + tr;   // first row with B_t >= column
   const double* tz = A.gtz + tr;       // prefix sums over the rows
   const uint32_t* tb = A.gtb + tr;
-  const double lpj = A.glp[fj], dfj = (double)fj;
+  const double lpj = GAPS ? 0.0 : A.glp[fj], dfj = (double)fj;
   // rows with 0 < b_t < nj: [z, y)
   const int z = bound ? min(max((int)inv[fj + 1], fi), ge) : fi;
   const int y = bound ? min(max((int)inv[fj + nj], fi), ge) : fi;
@@ -225,7 +270,7 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     if (top) ++mtop;
     if (m0 > mtop) m0 = mtop;  // no edge crosses the group
   }
-  if (owner && z1 < y) {  // pairs of the band, whatever their code
+  if (!GAPS && owner && z1 < y) {  // pairs of the band, whatever their code
     const uint32_t nt = (tb[y] - tb[z]) - (uint32_t)fj * (uint32_t)(y - z);
     const uint32_t* tb1 = tb + (A.ng + 1);
     const uint32_t nt1 = (tb1[y1] - tb1[z1]) - (uint32_t)fj * (uint32_t)(y1 - z1) + (uint32_t)nj * (uint32_t)(y - y1);
@@ -242,9 +287,14 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
   };
   unsigned rech = 0;
   int cur = z, rho = row_bound(m0);
-  double tzc = tz[z], lpc = A.glp[z];
-  uint32_t tbc = tb[z];
-  BandSums xp;  // X_t of the edge before
+  double tzc = 0.0, lpc = 0.0;
+  uint32_t tbc = 0u;
+  if (!GAPS) {
+    tzc = tz[z];
+    lpc = A.glp[z];
+    tbc = tb[z];
+  }
+  BandSums<GAPS> xp;  // X_t of the edge before
 #pragma unroll
   for (int f = 0; f < 6; ++f) xp.s[f] = 0.0;
   xp.z = 0.0;
@@ -254,8 +304,13 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
   for (int e = m0; e <= mtop; ++e) {
     const bool last = COORD == kObs || (top && e == mtop);
     // loads of this edge's row and the next edge's bound, used after the loop
-    const double tzr = tz[rho], lpr = A.glp[rho];
-    const uint32_t tbr = tb[rho];
+    double tzr = 0.0, lpr = 0.0;
+    uint32_t tbr = 0u;
+    if (!GAPS) {
+      tzr = tz[rho];
+      lpr = A.glp[rho];
+      tbr = tb[rho];
+    }
     const int rho_next = e < mtop ? row_bound(e + 1) : y;
     // V: rows [cur, rho), four at a time.  A lane's row and column advance
     // together, so the banks that eight lanes read side by side (one 128-byte
@@ -263,7 +318,9 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     // starting in a row of residue m l mod 8 (m odd) its columns have the
     // residues m l + (column - row), and m = 1, 3, 5 or 7 is taken for the most
     // different ones.  A lane idles through the rows before cur.
-    double a[6] = {0, 0, 0, 0, 0, 0};
+    double a[GAPS ? 8 : 6];
+#pragma unroll
+    for (int f = 0; f < (GAPS ? 8 : 6); ++f) a[f] = 0.0;
     {
       const int l8 = lane & 7;
       const int lag = rho > cur ? (int)tt[cur] - cur : l8;
@@ -300,6 +357,10 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
         for (int q = 0; q < 4; ++q) {
           if (g + q >= cur && g + q < rho) {
             const double2 p = pj[x[q]], r = rp[q];
+            if constexpr (GAPS) {
+              add_gap_row(a, r, it.M[g + q - fi], p, it.C[(int)x[q] - fj]);
+              continue;
+            }
             const double b = __hiloint2double(0x43300000, (int)x[q]) - bias;  // the column as a double
             a[0] = __fma_rn(r.x, p.x, a[0]);
             a[1] = __fma_rn(r.x, b, a[1]);
@@ -313,7 +374,7 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     }
     // X: rows from rho1 in which the edge crosses the band
     const int rho1 = __shfl_down_sync(kFull, rho, 1);
-    BandSums x;
+    BandSums<GAPS> x;
 #pragma unroll
     for (int f = 0; f < 6; ++f) x.s[f] = 0.0;
     x.z = 0.0;
@@ -321,7 +382,13 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     if (owner) {
       if (last) {
         // the band's end: rows [y1, y) with every column from b_t on
-        if (y > y1) {
+        if constexpr (GAPS) {
+          if (y > y1) {
+            const double2 pa = it.Pi[y1 - fi], pb = it.Pi[y - fi], ca = it.Ci[y1 - fi], cb = it.Ci[y - fi];
+            add_gap_row(x, make_double2(pb.x - pa.x, pb.y - pa.y), make_double2(cb.x - ca.x, cb.y - ca.y), it.P[nj],
+                        it.C[nj]);
+          }
+        } else if (y > y1) {
           const double2 p = it.P[nj];
           const double4 ra = it.Ri[y1 - fi], rb = it.Ri[y - fi];
           const double dn = (double)nj, dr = (double)(y - y1);
@@ -350,15 +417,21 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
         }
       }
     }
-    // z sum and pair count of the rows [cur, rho)
-    const double vz = (tzr - tzc) - 0.5 * (dfj * (lpr - lpc) + lpj * (double)(rho - cur));
-    const uint32_t vn = (tbr - tbc) - (uint32_t)fj * (uint32_t)(rho - cur);
     // the bin of the codes between this edge and the one before: boundary
     // t + 1 less boundary t, and the edges' rows
     const int code = (COORD == kObs) ? 0 : e - 1;
     FAcc F;
-    F.n = __shfl_down_sync(kFull, vn, 1) - vn + x.n - xp.n;
-    const double zc = __shfl_down_sync(kFull, vz, 1) - vz + x.z - xp.z;
+    double zc;
+    if constexpr (GAPS) {
+      F.n = (uint32_t)(__shfl_down_sync(kFull, a[7], 1) - a[7] + x.n - xp.n);
+      zc = __shfl_down_sync(kFull, a[6], 1) - a[6] + x.z - xp.z;
+    } else {
+      // z sum and pair count of the rows [cur, rho)
+      const double vz = (tzr - tzc) - 0.5 * (dfj * (lpr - lpc) + lpj * (double)(rho - cur));
+      const uint32_t vn = (tbr - tbc) - (uint32_t)fj * (uint32_t)(rho - cur);
+      F.n = __shfl_down_sync(kFull, vn, 1) - vn + x.n - xp.n;
+      zc = __shfl_down_sync(kFull, vz, 1) - vz + x.z - xp.z;
+    }
     bool tiny = false;
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
@@ -371,12 +444,13 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     if (owner && F.n != 0u && code >= 0) {
       if (tiny) {
         double s[6];
-        band_by_rows<COORD, MINPOS>(A, it.P, it.R, U, fi, fj, nj, it.c, ap, tt, min(z1, y), y, code, s);
+        band_by_rows<COORD, MINPOS, GAPS>(A, it, U, tt, min(z1, y), y, code, s);
 #pragma unroll
         for (int f = 0; f < 6; ++f) F.s[f] = s[f];
       }
       F.s[6] = __fma_rn(A.lmid, (double)F.n, zc);
       F.code = code;
+      if (GAPS) stats[0] += F.n;
       add_bin<COORD>(A, it.d, (t < n0) ? n0 - 1 - t : t - n0 - 1, code, F);
     }
     xp = x;
@@ -391,9 +465,9 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
 
 // Prepare the next owned item into `h` (all lanes of one warp; SMEM: its data
 // into buf, arriving on `full`).
-template <int COORD, bool SMEM>
-__device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double2* buf, unsigned long long* full,
-                                             int lane, unsigned long long& n_taken) {
+template <int COORD, bool SMEM, bool GAPS>
+__device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, int* next, double2* buf,
+                                          unsigned long long* full, int lane, unsigned long long& n_taken) {
   const int nb = 2 * (int)A.g.n0 + 1;
   BandItem it;
   it.bands = 0;
@@ -402,11 +476,11 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double
     if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
     idx = __shfl_sync(kFull, idx, 0);
     if (idx >= A.n_items) break;
-    if (item_owner(A, idx) != kOwnerGrid) continue;  // another kernel's item
+    if (item_owner(A, idx) != (GAPS ? kOwnerGaps : kOwnerGrid)) continue;  // another kernel's item
     ++n_taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
-    it.ni = (int)A.npix[i];
-    it.nj = (int)A.npix[j];
+    it.ni = (int)A.gspan[i];
+    it.nj = (int)A.gspan[j];
     it.fi = (int)A.gfirst[i];
     it.fj = (int)A.gfirst[j];
     // bands that hold a pair: b_{t+1} > 0 in the last row, b_t < nj in the first
@@ -426,11 +500,25 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double
     it.c = A.item_c[idx];
     const double a = 2.0 * dsub(1.0, it.c);
     it.ap = (float)(a * A.g.inv1 * A.g.inv1);
-    it.Ri = A.prefix + A.off[i] + i;
-    const double2* gP = A.pre2 + A.off[j] + j;
-    const double2* gR = A.row2 + A.off[i];
+    const int len = A.max_span + 1;
+    const double2 *gP, *gR, *gC = nullptr, *gM = nullptr;
+    if (GAPS) {
+      const uint64_t oi = A.gap_off[i], oj = A.gap_off[j];
+      gP = A.gap_pre + oj;
+      gC = A.gap_cnt + oj;
+      gR = A.gap_row + oi;
+      gM = A.gap_one + oi;
+      it.Pi = A.gap_pre + oi;
+      it.Ci = A.gap_cnt + oi;
+    } else {
+      it.Ri = A.prefix + A.off[i] + i;
+      gP = A.pre2 + A.off[j] + j;
+      gR = A.row2 + A.off[i];
+    }
     it.P = SMEM ? buf : gP;
-    it.R = SMEM ? buf + A.max_np + 1 : gR;
+    it.R = SMEM ? buf + len : gR;
+    it.C = SMEM ? buf + 2 * len : gC;
+    it.M = SMEM ? buf + 3 * len : gM;
     const float4 ri = A.range[i], rj = A.range[j];
     it.d.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
     it.d.cell = dest_row(A, i, j);
@@ -441,11 +529,16 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double
     it.per = (it.bands + groups - 1) / groups;
     if (lane == 0) {
       *h = it;
+      *next = 0;
       if (SMEM) {
         const uint32_t bp = (uint32_t)(it.nj + 1) * 16u, br = (uint32_t)it.ni * 16u;
-        bar_arrive_tx(full, bp + br);
+        bar_arrive_tx(full, GAPS ? 2 * (bp + br) : bp + br);
         bulk_load(buf, gP, bp, full);
-        bulk_load(buf + A.max_np + 1, gR, br, full);
+        bulk_load(buf + len, gR, br, full);
+        if (GAPS) {
+          bulk_load(buf + 2 * len, gC, bp, full);
+          bulk_load(buf + 3 * len, gM, br, full);
+        }
       } else {
         bar_arrive(full);
       }
@@ -462,23 +555,24 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, double
 
 // The arguments stay in the kernel's parameter space (__grid_constant__):
 // the inlined sweep reads them as constant-bank operands.
-template <int COORD, bool MINPOS, bool SMEM>
-__global__ void __launch_bounds__(kGridThreads, 4) grid_kernel(const __grid_constant__ PairArgs A) {
+template <int COORD, bool MINPOS, bool SMEM, bool GAPS>
+__global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kernel(const __grid_constant__ PairArgs A) {
   extern __shared__ double2 band_smem[];
   __shared__ BandItem s_item[2];
+  __shared__ int s_next[2];  // GAPS: next group of each item
   __shared__ unsigned long long s_full[2], s_empty[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int buf_len = 2 * A.max_np + 1;
+  const int len = A.max_span + 1, buf_len = (GAPS ? 4 : 2) * len;
   const float* U = A.gU;
   if (SMEM) {
     float* u = reinterpret_cast<float*>(band_smem + 2 * (size_t)buf_len);
-    for (int g = tid; g < A.ng; g += kGridThreads) u[g] = A.gU[g];
+    for (int g = tid; g < A.ng; g += kGridWarps<GAPS> * 32) u[g] = A.gU[g];
     U = u;
   }
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
-      bar_init(&s_empty[b], kGridWarps);
+      bar_init(&s_empty[b], kGridWarps<GAPS>);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -486,7 +580,8 @@ __global__ void __launch_bounds__(kGridThreads, 4) grid_kernel(const __grid_cons
   unsigned long long stats[2] = {0ull, 0ull};  // pairs in bands, FP64 re-evaluations
   unsigned long long n_taken = 0;
   bool ok = true, ended = false;
-  if (warp == 0) prepare_item<COORD, SMEM>(A, &s_item[0], band_smem, &s_full[0], lane, n_taken);
+  if (warp == 0)
+    prepare_item<COORD, SMEM, GAPS>(A, &s_item[0], &s_next[0], band_smem, &s_full[0], lane, n_taken);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u, parity = (k >> 1) & 1u;
     ok = bar_wait(&s_full[b], parity);
@@ -495,37 +590,51 @@ __global__ void __launch_bounds__(kGridThreads, 4) grid_kernel(const __grid_cons
     if (it.bands == 0) break;
     if (SMEM) {  // the same pointers, known to be in shared memory
       it.P = band_smem + (size_t)b * buf_len;
-      it.R = it.P + A.max_np + 1;
+      it.R = it.P + len;
+      it.C = it.P + 2 * len;
+      it.M = it.P + 3 * len;
     }
     if (warp == 0 && !ended) {
       const uint32_t nb = b ^ 1u;
       // item k - 1 (the other buffer's) is done by every warp
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
       if (!ok) break;
-      prepare_item<COORD, SMEM>(A, &s_item[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0), &s_full[nb], lane,
-                                n_taken);
+      prepare_item<COORD, SMEM, GAPS>(A, &s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
+                                      &s_full[nb], lane, n_taken);
       ended = s_item[nb].bands == 0;
     }
-    for (int q = warp; q * it.per < it.bands; q += kGridWarps)
-      band_group<COORD, MINPOS>(A, it, U, it.tf + q * it.per, min(it.per, it.bands - q * it.per), lane, stats);
+    for (int q = warp;; q += kGridWarps<GAPS>) {
+      if (GAPS) {  // more warps than an item has groups: from a counter
+        if (lane == 0) q = atomicAdd(&s_next[b], 1);
+        q = __shfl_sync(kFull, q, 0);
+      }
+      if (q * it.per >= it.bands) break;
+      band_group<COORD, MINPOS, GAPS>(A, it, U, it.tf + q * it.per, min(it.per, it.bands - q * it.per), lane, stats);
+    }
     __syncwarp();
     if (lane == 0) bar_arrive(&s_empty[b]);
   }
   if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
-  add_counters(A, lane, stats[0], stats[1], n_taken, 9);
+  add_counters(A, lane, stats[0], stats[1], n_taken, GAPS ? 8 : 9);
+}
+
+// Two items and the grid's values.
+template <bool GAPS>
+size_t band_smem_bytes(const PairArgs& a) {
+  return 2 * (size_t)(GAPS ? 4 : 2) * (a.max_span + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float);
 }
 
 // Persistent launch: `ctas_per_sm` CTAs per SM (0 or above the occupancy
 // limit: as many as fit), or with `max_out` set only that limit.
-template <int COORD, bool MINPOS, bool SMEM>
+template <int COORD, bool MINPOS, bool SMEM, bool GAPS>
 cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  // two items and the grid's values
-  const size_t smem = SMEM ? 2 * (size_t)(2 * a.max_np + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float) : 0;
-  auto kern = grid_kernel<COORD, MINPOS, SMEM>;
+  constexpr int threads = kGridWarps<GAPS> * 32;
+  const size_t smem = SMEM ? band_smem_bytes<GAPS>(a) : 0;
+  auto kern = grid_kernel<COORD, MINPOS, SMEM, GAPS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
   if (e != cudaSuccess) return e;
   per_sm = std::max(per_sm, 1);
   if (max_out) {
@@ -533,30 +642,40 @@ cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
     return cudaSuccess;
   }
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-  kern<<<num_sms * per_sm, kGridThreads, smem, stream>>>(a);
+  kern<<<num_sms * per_sm, threads, smem, stream>>>(a);
   return cudaGetLastError();
 }
 
-// Items and the grid's values are staged in shared memory when two items'
-// prefix sums and row values and the values fit a CTA (227 KB), the usual
-// case: 622-pixel forests on 1,800 values take 47 KB.
+// Items and the grid's values are staged in shared memory when two items and
+// the values fit a CTA (227 KB), the usual case: 622-pixel forests on 1,800
+// values take 47 KB (87 KB with gaps).
 constexpr size_t kBandSmem = 224 * 1024;
 
-template <int COORD, bool MINPOS>
+template <int COORD, bool MINPOS, bool GAPS>
 cudaError_t launch_grid2(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  const bool fits = 2 * (size_t)(2 * a.max_np + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float) <= kBandSmem;
-  return fits ? launch_grid<COORD, MINPOS, true>(a, num_sms, ctas_per_sm, stream, max_out)
-              : launch_grid<COORD, MINPOS, false>(a, num_sms, ctas_per_sm, stream, max_out);
+  return band_smem_bytes<GAPS>(a) <= kBandSmem
+             ? launch_grid<COORD, MINPOS, true, GAPS>(a, num_sms, ctas_per_sm, stream, max_out)
+             : launch_grid<COORD, MINPOS, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
+}
+
+template <bool GAPS>
+cudaError_t launch_grid3(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm, cudaStream_t stream,
+                         int* max_out) {
+  if (coord == TOS_CARTESIAN)
+    return minpos ? launch_grid2<kCart, true, GAPS>(a, num_sms, ctas_per_sm, stream, max_out)
+                  : launch_grid2<kCart, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
+  return launch_grid2<kObs, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
 }  // namespace
 
 cudaError_t launch_grid_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm,
                                cudaStream_t stream, int* max_out) {
-  if (coord == TOS_CARTESIAN)
-    return minpos ? launch_grid2<kCart, true>(a, num_sms, ctas_per_sm, stream, max_out)
-                  : launch_grid2<kCart, false>(a, num_sms, ctas_per_sm, stream, max_out);
-  return launch_grid2<kObs, false>(a, num_sms, ctas_per_sm, stream, max_out);
+  return launch_grid3<false>(a, coord, minpos, num_sms, ctas_per_sm, stream, max_out);
+}
+
+cudaError_t launch_gap_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream) {
+  return launch_grid3<true>(a, coord, minpos, num_sms, 0, stream, nullptr);
 }
 
 }  // namespace tos

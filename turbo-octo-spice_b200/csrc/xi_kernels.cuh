@@ -33,7 +33,7 @@
 namespace tos {
 
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
-constexpr uint32_t kNoGrid = 0xFFFFFFFFu;  // sightline not contiguous on the common grid
+constexpr uint32_t kNoGrid = 0xFFFFFFFFu;  // sightline not on the common grid
 constexpr int kPairWarps = 16;  // warps per CTA of the pair kernel
 // u32 words per window slot: the three signed sums (didj, di, dj) as 22+22+rest
 // bit words of a 62-bit fixed-point value, the four positive sums (wgt, wi,
@@ -131,6 +131,13 @@ struct PairArgs {
   const float* gl;           // [ng]: loglam of each grid value
   const double* glp;         // [ng + 1]: exclusive prefix sums of l' = loglam - lmid
   const uint32_t* gfirst;    // per sightline: grid index of pixel 0, or kNoGrid
+  const uint32_t* gspan;     // per sightline: grid values from its first to its last pixel
+  int max_span;              // largest of the launched items' sightlines
+  // the sightlines laid out on the grid, entry c of a sightline the grid value
+  // gfirst + c (missing pixels zero), at gap_off: prefix sums (span + 1
+  // entries) of (wd, w) and of (1, l'/2), and the values themselves
+  const uint64_t* gap_off;
+  const double2 *gap_pre, *gap_cnt, *gap_row, *gap_one;
   const double2* pre2;       // prefix sums (wd, w) alone, laid out as `prefix`
   const double2* row2;       // (w*delta, w) per pixel
   double lmid;               // loglam near the middle of the grid
@@ -146,7 +153,8 @@ struct PairArgs {
   float lev_scale, lev_off;
   int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
   int max_np;                // longest sightline
-  int grid_split;            // the grid kernel takes the run items whose sightlines are on the grid
+  int grid_split;            // the grid kernel takes the run items whose sightlines are contiguous on the grid
+  int gap_split;             // its variant for gaps takes the other run items whose sightlines are on the grid
   int diag_split;            // Polar: the diagonal-sweep kernel takes the items whose z index is
                              // constant; the pixel-pair kernel evaluates the rest exactly
   int win_w1;                // window width along axis 1 (Cartesian)
@@ -178,11 +186,14 @@ cudaError_t launch_pair_kernel(const PairArgs& a, int coord, bool exact0, bool m
 size_t pair_kernel_smem(int win_slots);
 
 // Launch the persistent grid-sweep kernel (xi_grid.cu) over the items that
-// run_item() accepts and whose two sightlines lie on the common grid.
+// run_item() accepts and whose two sightlines are contiguous on the common grid.
 // ctas_per_sm: CTAs per SM (0: as many as fit); with max_out set, only
 // report that limit.
 cudaError_t launch_grid_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm,
                                cudaStream_t stream, int* max_out = nullptr);
+
+// The same for the items with gapped sightlines (item_owner: kOwnerGaps).
+cudaError_t launch_gap_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream);
 
 // Launch the persistent diagonal-sweep kernel (xi_diag.cu) over the Polar
 // items that diag_item() accepts (every field on the wide scale).

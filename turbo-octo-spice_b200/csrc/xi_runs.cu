@@ -1,6 +1,7 @@
 // xi_runs.cu — pointer-sweep kernel of the XiEstimator pair count (Cartesian
 // and observing coordinates): the run sweep of xi_sweep.cuh for sorted
-// sightlines that are not contiguous on a common coordinate grid.
+// sightlines that are not on a common coordinate grid (values repeated within
+// a sightline, or too many or too scattered values for one).
 //
 // A lane owns one (side, bin k) task and walks the rows with two column
 // pointers, the first columns that pass the boundary predicates of T[k] and
@@ -118,7 +119,6 @@ __global__ void __launch_bounds__(kRunWarps * 32, 4) run_kernel(PairArgs args) {
       todo &= todo - 1;
       SweepItem it;
       if (!load_item<COORD>(A, idx, tmax, it)) continue;  // another kernel's item
-      if (grid_item(A, it.i, it.j)) continue;              // the grid sweep's item
       ++n_taken;
       if (it.r_hi <= it.r_lo) continue;
       for (int t0 = 0; t0 < 2 * n0; t0 += 32) run_group<COORD, MINPOS>(A, it, t0, lane, stats);
