@@ -8,9 +8,14 @@
 
 namespace tos {
 
-// Field f of one (row, bin) as a signed 128-bit integer.
+// A field's two words as a signed 128-bit integer.
+__device__ __forceinline__ __int128 acc128_of(unsigned long long lo, unsigned long long hi) {
+  return (__int128)(long long)hi * ((__int128)1 << kAccShift) + (__int128)lo;
+}
+
+// Field f of one (row, bin).
 __device__ __forceinline__ __int128 acc128(const unsigned long long* base, int f) {
-  return (__int128)(long long)base[7 + f] * ((__int128)1 << kAccShift) + (__int128)base[f];
+  return acc128_of(base[f], base[7 + f]);
 }
 
 // Store v (|v| < 2^89) as field f of a row kept in the same format.

@@ -79,12 +79,6 @@ struct DItem {
   const PixPack* cols;   // padded pixels of sightline j, even ones first
 };
 
-// Entry of pixel p (0 of the even ones at kParityPad; kParityPad entries of
-// zero weight beside each half) in the even-first order of n pixels.
-__device__ __forceinline__ int parity_slot(int p, int n) {
-  return kParityPad + (p & 1) * (((n + 1) >> 1) + kParityPad) + (p >> 1);
-}
-
 // Row values of the pixel-pair kernel's Polar fast path (xi_kernels.cu
 // fast_bin): x1 = d1, A1 = d1 * 2(1 - c), dl1 = -(d1*d1 - fl(d1*d1)).
 struct DRow {
