@@ -183,9 +183,7 @@ tos_status sample_covariance(tos_engine* e, double* dX, const double* dw, uint32
   TOS_CUDA_TRY(cudaGetLastError());
   if (mean_out)
     TOS_CUDA_TRY(cudaMemcpyAsync(mean_out, dmean.p, (size_t)nb * 8, cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaMemcpyAsync(cov_out, dC.p, (size_t)nb * nb * 8, cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  return TOS_OK;
+  return copy_out(e, cov_out, dC.p, (size_t)nb * nb * 8);
 }
 
 tos_status check_last_run(tos_engine* e, tos_catalog* cat) {

@@ -1080,6 +1080,7 @@ void tos_engine_destroy(tos_engine* e) {
     DeviceGuard g(e->device);
     cudaStreamSynchronize(e->stream);
     e->brute.release();
+    e->stage.release();
     for (auto& ev : e->ev) cudaEventDestroy(ev);
     cudaStreamDestroy(e->stream);
   }
@@ -2162,9 +2163,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
                                cudaMemcpyDeviceToHost, st));
   unsigned long long hc[14];
   TOS_CUDA_TRY(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, st));
-  if (n_rows)
-    TOS_CUDA_TRY(cudaMemcpyAsync(out_cells, ws->d_out.p + nb, n_rows * nb * sizeof(tos_xibin),
-                                 cudaMemcpyDeviceToHost, st));
+  if (n_rows) TOS_TRY(copy_out(e, out_cells, ws->d_out.p + nb, n_rows * nb * sizeof(tos_xibin)));
   TOS_CUDA_TRY(cudaEventRecord(e->ev[4], st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   if (hc[13]) return fail(TOS_ERR_TIMEOUT, "a wait of the grid sweep ran out");

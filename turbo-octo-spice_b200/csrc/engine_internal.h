@@ -159,6 +159,24 @@ struct Workspace {
 
 }  // namespace tos
 
+namespace tos {
+
+// Pinned staging of copy_out (4 MiB), kept by the engine under its mutex.
+struct HostStage {
+  static constexpr int kSlots = 8;
+  static constexpr size_t kSlotBytes = 512 * 1024;
+  unsigned char* p = nullptr;
+  cudaEvent_t ev[kSlots] = {};
+  bool ready();  // allocates on the first call; false where that fails
+  void release();
+};
+
+// Copies `bytes` from the device to the host after the work on the engine's
+// stream, and waits for them (engine mutex held).
+tos_status copy_out(tos_engine* e, void* dst, const void* src, size_t bytes);
+
+}  // namespace tos
+
 struct tos_engine {
   int device = 0;
   int num_sms = 0;
@@ -171,6 +189,7 @@ struct tos_engine {
   std::mutex tune_mu;
   std::map<int, std::pair<int, int>> brute_tuned;
   tos::BruteScratch brute;
+  tos::HostStage stage;
   // CTAs per SM of the dominant pair-count kernel picked by TOS_XI_TUNE, by
   // (coordinate type, total bins)
   std::map<std::pair<int, int>, int> xi_tuned;
