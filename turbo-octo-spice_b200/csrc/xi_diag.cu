@@ -33,11 +33,13 @@
 // keys and the pair-by-pair blocks (6.6 % of the pairs).
 //
 // Measured on a B200 against the version that binned every pair (one warp per
-// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 282 ms; five mocks
-// of 5,000 sightlines in all: 292 -> 167 ms; jackknife of 2,500 sightlines (its
+// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 266 ms; five mocks
+// of 5,000 sightlines in all: 292 -> 158 ms; jackknife of 2,500 sightlines (its
 // few rows once went to the pixel-pair kernel: low words of 32 bits could have
-// wrapped after 2^32 adds): 363 -> 102 ms.  Block bounds from the extremes of
-// d1 d2 instead of r^2 sent twice the blocks pair by pair; one lane per run
+// wrapped after 2^32 adds): 363 -> 96 ms.  Block bounds from the extremes of
+// d1 d2 instead of r^2 sent twice the blocks pair by pair; functions that are
+// not inlined and read the arguments through the kernel's parameters cost 6 % (now
+// copied to shared memory); one lane per run
 // with its own 15 adds touched 32 lines an add and took 30 of 46 shared-memory
 // and L1 cycles a step.
 #include "bulk_pipeline.cuh"
@@ -54,8 +56,9 @@ constexpr int kQueue = 64;     // runs or blocks a warp holds (taken 32 at a tim
 
 // A warp's queues and the staging of the sums of 32 runs.
 struct WarpQ {
+  unsigned long long rech;  // FP64 re-evaluations
   double didj[kQueue], wgt[kQueue];
-  double val[8][33];  // a row longer by one: a key's eight fields lie in different banks
+  double val[8][34];  // (rows longer by two: eight fields of two runs lie in different banks)
   uint32_t key[kQueue];
   int s0[kQueue], s1[kQueue], delta[kQueue];
   // blocks to sweep pair by pair (first row, diagonal), each with the run its
@@ -78,6 +81,12 @@ struct DItem {
   const PixPack* rows;   // padded pixels of sightline i, even ones first
   const PixPack* cols;   // padded pixels of sightline j, even ones first
 };
+
+// The CTA's two items and the launch's arguments for the functions that are
+// not inlined: through a reference to the kernel's parameters they would read
+// them by generic loads.
+__shared__ DItem s_item[2];
+__shared__ PairArgs s_args;
 
 // Row values of the pixel-pair kernel's Polar fast path (xi_kernels.cu
 // fast_bin): x1 = d1, A1 = d1 * 2(1 - c), dl1 = -(d1*d1 - fl(d1*d1)).
@@ -189,7 +198,9 @@ __device__ __forceinline__ void add_counters_diag(const PairArgs& A, int lane, u
 // Add the queue entries [first, first + n) of the warp to the item's row: a
 // lane works out the sums of one run, then eight lanes take a run, a field
 // each, so that the adds of a run fall into its one 128-byte entry.
-__device__ __noinline__ void drain(const PairArgs& A, const DItem& it, WarpQ& Q, int first, int n, int lane) {
+__device__ __noinline__ void drain(int buf, WarpQ& Q, int first, int n, int lane) {
+  const PairArgs& A = s_args;
+  const DItem& it = s_item[buf];
   __syncwarp();
   uint32_t at = 0xFFFFFFFFu;  // flat bin of the run
   if (lane < n) {
@@ -237,7 +248,7 @@ __device__ __noinline__ void drain(const PairArgs& A, const DItem& it, WarpQ& Q,
 }
 
 // Queue the runs of the lanes that close one; 32 waiting runs are added.
-__device__ __forceinline__ void push_run(const PairArgs& A, const DItem& it, WarpQ& Q, int& qn, bool close,
+__device__ __forceinline__ void push_run(int buf, WarpQ& Q, int& qn, bool close,
                                          uint32_t key, int s0, int s1, int delta, double didj, double wgt, int lane) {
   const unsigned cm = __ballot_sync(kFull, close);
   if (cm == 0) return;
@@ -253,16 +264,18 @@ __device__ __forceinline__ void push_run(const PairArgs& A, const DItem& it, War
   qn += __popc(cm);
   if (qn >= 32) {
     qn -= 32;
-    drain(A, it, Q, qn, 32, lane);
+    drain(buf, Q, qn, 32, lane);
   }
 }
 
 // Sweep the queued blocks [first, first + n) pair by pair, one per lane.  A
 // block usually closes one run: it is kept until the end of the block, when
-// the lanes' closed runs are queued together.
+// the lanes' closed runs are queued together.  Returns the runs in the queue.
 template <bool MINPOS>
-__device__ __noinline__ void sweep_blocks(const PairArgs& A, const DItem& it, WarpQ& Q, int first, int n, int& qn,
-                                          int lane, unsigned& rech) {
+__device__ __noinline__ int sweep_blocks(int buf, WarpQ& Q, int first, int n, int qn, int lane) {
+  const PairArgs& A = s_args;
+  const DItem& it = s_item[buf];
+  unsigned rech = 0;
   __syncwarp();
   int delta = 0, lo = 0, hi = 0, s0 = 0;
   uint32_t cur = kInvalidKey;  // the run open before the block goes on in it
@@ -312,7 +325,7 @@ __device__ __noinline__ void sweep_blocks(const PairArgs& A, const DItem& it, Wa
     const bool close = change && cur != kInvalidKey;
     // a second run closed by this block: the first one is queued now
     if (__any_sync(kFull, close && pkey != kInvalidKey))
-      push_run(A, it, Q, qn, close && pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
+      push_run(buf, Q, qn, close && pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
     if (close) {
       pkey = cur;
       ps0 = s0;
@@ -331,8 +344,11 @@ __device__ __noinline__ void sweep_blocks(const PairArgs& A, const DItem& it, Wa
       wgt = __fma_rn((double)rp.w, (double)cp.w, wgt);
     }
   }
-  push_run(A, it, Q, qn, pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
-  push_run(A, it, Q, qn, cur != kInvalidKey, cur, s0, hi, delta, didj, wgt, lane);
+  push_run(buf, Q, qn, pkey != kInvalidKey, pkey, ps0, ps1, delta, pd, pw, lane);
+  push_run(buf, Q, qn, cur != kInvalidKey, cur, s0, hi, delta, didj, wgt, lane);
+  rech = __reduce_add_sync(kFull, rech);
+  if (lane == 0) Q.rech += rech;
+  return qn;
 }
 
 __device__ __forceinline__ float fmin3(float a, float b, float c) {
@@ -419,11 +435,10 @@ struct DiagRun {
 };
 
 // Sweep diagonals d0 .. d0 + 63 of an item: lane L takes d0 + 2 L and the next.
-// `it` is the item in registers, `sh` the same in shared memory for the
-// functions called now and then.
+// `it` is s_item[buf] in registers.
 template <bool MINPOS>
-__device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, const DItem& sh, int d0, int lane,
-                                           WarpQ& Q, unsigned long long* stats) {
+__device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, int buf, int d0, int lane, WarpQ& Q,
+                                           unsigned long long& n_eval_sum) {
   const int ni = it.ni, nj = it.nj;
   const int da = d0 + 2 * lane;  // diagonals da and da + 1
   const int s_lo = max(0, -(d0 + kDiagSpan - 1));
@@ -432,7 +447,7 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, c
 #pragma unroll
   for (int m = 0; m < 2; ++m) run[m] = DiagRun{kInvalidKey, 0, 0.0, 0.0};
   int qn = 0, bn = 0;  // queued runs and blocks (the same in every lane)
-  unsigned rech = 0, n_eval = 0;
+  unsigned n_eval = 0;
 #pragma unroll 1
   for (int sb = s_lo; sb < s_hi; sb += kDiagRows) {
     BlockSums B;
@@ -456,7 +471,7 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, c
       // blocks to sweep pair by pair take the open run along
       const bool mixed = key == kMixedKey;
       const bool change = key != run[m].cur;
-      push_run(A, sh, Q, qn, change && !mixed && run[m].cur != kInvalidKey, run[m].cur, run[m].s0, sb, da + m,
+      push_run(buf, Q, qn, change && !mixed && run[m].cur != kInvalidKey, run[m].cur, run[m].s0, sb, da + m,
                run[m].didj, run[m].wgt, lane);
       const unsigned xm = __ballot_sync(kFull, mixed);
       if (mixed) {
@@ -479,7 +494,7 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, c
         bn += __popc(xm);
         if (bn >= 32) {
           bn -= 32;
-          sweep_blocks<MINPOS>(A, sh, Q, bn, 32, qn, lane, rech);
+          qn = sweep_blocks<MINPOS>(buf, Q, bn, 32, qn, lane);
         }
       }
     }
@@ -487,19 +502,19 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, c
   // runs still open at the last row, then the queues
 #pragma unroll
   for (int m = 0; m < 2; ++m)
-    push_run(A, sh, Q, qn, run[m].cur != kInvalidKey, run[m].cur, run[m].s0, s_hi, da + m, run[m].didj, run[m].wgt,
+    push_run(buf, Q, qn, run[m].cur != kInvalidKey, run[m].cur, run[m].s0, s_hi, da + m, run[m].didj, run[m].wgt,
              lane);
-  if (bn) sweep_blocks<MINPOS>(A, sh, Q, 0, bn, qn, lane, rech);
-  drain(A, sh, Q, 0, qn, lane);
-  stats[0] += n_eval;
-  stats[1] += rech;
+  if (bn) qn = sweep_blocks<MINPOS>(buf, Q, 0, bn, qn, lane);
+  drain(buf, Q, 0, qn, lane);
+  n_eval_sum += n_eval;
 }
 
 // Prepare the next owned item into `h` (all lanes of one warp; SMEM: its
-// pixels into buf), arriving on `full`.
+// pixels into buf), arriving on `full`.  Returns the items taken.
 template <bool SMEM>
-__device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next, PixPack* buf,
-                                          unsigned long long* full, int lane, unsigned long long& n_taken) {
+__device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsigned long long* full, int lane) {
+  const PairArgs& A = s_args;
+  int taken = 0;
   DItem it;
   it.groups = 0;
   for (;;) {
@@ -508,7 +523,7 @@ __device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next
     idx = __shfl_sync(kFull, idx, 0);
     if (idx >= A.n_items) break;
     if (item_owner(A, idx) != kOwnerDiag) continue;  // the pixel-pair kernel's item
-    ++n_taken;
+    ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
     it.ni = (int)A.npix[i];
     it.nj = (int)A.npix[j];
@@ -582,7 +597,7 @@ __device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next
       }
     }
     __syncwarp();
-    return;
+    return taken;
   }
   if (lane == 0) {  // no item left
     it.groups = 0;
@@ -590,6 +605,7 @@ __device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next
     bar_arrive(full);
   }
   __syncwarp();
+  return taken;
 }
 
 // The arguments stay in the kernel's parameter space (__grid_constant__):
@@ -600,13 +616,14 @@ __device__ __noinline__ void prepare_diag(const PairArgs& A, DItem* h, int* next
 template <bool MINPOS, bool SMEM>
 __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_constant__ PairArgs A) {
   extern __shared__ PixPack diag_smem[];  // the item buffers, then the warps' queues
-  __shared__ DItem s_item[2];
   __shared__ int s_next[2];
   __shared__ unsigned long long s_full[2], s_empty[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int buf_len = 2 * (A.max_np + 3 * kParityPad);
   WarpQ& Q = reinterpret_cast<WarpQ*>(diag_smem + (SMEM ? 2 * (size_t)buf_len : 0))[warp];
+  if (lane == 0) Q.rech = 0ull;
   if (tid == 0) {
+    s_args = A;
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
       bar_init(&s_empty[b], kDiagWarps);
@@ -614,10 +631,10 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  unsigned long long stats[2] = {0ull, 0ull};  // evaluated pairs, FP64 re-evaluations
+  unsigned long long n_eval = 0;
   unsigned long long n_taken = 0;
   bool ok = true, ended = false;
-  if (warp == 0) prepare_diag<SMEM>(A, &s_item[0], &s_next[0], diag_smem, &s_full[0], lane, n_taken);
+  if (warp == 0) n_taken += prepare_diag<SMEM>(&s_item[0], &s_next[0], diag_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u;
     ok = bar_wait(&s_full[b], (k >> 1) & 1u);
@@ -632,8 +649,8 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
       const uint32_t nb = b ^ 1u;
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);  // item k - 1 is done by every warp
       if (!ok) break;
-      prepare_diag<SMEM>(A, &s_item[nb], &s_next[nb], diag_smem + (SMEM ? (size_t)nb * buf_len : 0),
-                         &s_full[nb], lane, n_taken);
+      n_taken += prepare_diag<SMEM>(&s_item[nb], &s_next[nb], diag_smem + (SMEM ? (size_t)nb * buf_len : 0),
+                                    &s_full[nb], lane);
       ended = s_item[nb].groups == 0;
     }
     for (;;) {
@@ -641,13 +658,14 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
       if (lane == 0) q = atomicAdd(&s_next[b], 1);
       q = __shfl_sync(kFull, q, 0);
       if (q >= it.groups) break;
-      diag_group<MINPOS>(A, it, s_item[b], it.dlo + q * kDiagSpan, lane, Q, stats);
+      diag_group<MINPOS>(A, it, (int)b, it.dlo + q * kDiagSpan, lane, Q, n_eval);
     }
     __syncwarp();
     if (lane == 0) bar_arrive(&s_empty[b]);
   }
   if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
-  add_counters_diag(A, lane, stats[0], stats[1], n_taken);
+  __syncwarp();
+  add_counters_diag(A, lane, n_eval, lane == 0 ? Q.rech : 0ull, n_taken);
 }
 
 // Two items of two padded sightlines.
