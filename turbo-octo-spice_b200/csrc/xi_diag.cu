@@ -38,10 +38,9 @@
 // few rows once went to the pixel-pair kernel: low words of 32 bits could have
 // wrapped after 2^32 adds): 363 -> 96 ms.  Block bounds from the extremes of
 // d1 d2 instead of r^2 sent twice the blocks pair by pair; functions that are
-// not inlined and read the arguments through the kernel's parameters cost 6 % (now
-// copied to shared memory); one lane per run
-// with its own 15 adds touched 32 lines an add and took 30 of 46 shared-memory
-// and L1 cycles a step.
+// not inlined and read the arguments through the kernel's parameters cost 6 %;
+// one lane per run with its own 15 adds touched 32 lines an add and took 30 of
+// 46 shared-memory and L1 cycles a step.
 #include "bulk_pipeline.cuh"
 #include "xi_device.cuh"
 

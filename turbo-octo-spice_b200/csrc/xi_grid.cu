@@ -45,11 +45,13 @@
 //
 // Measured on a B200 against the version that evaluated the r_perp code at
 // every boundary of every row and bisected each split run (one warp per item):
-//                                            that  bands  + tables, pipeline
-//   16,000 sightlines at 16/deg^2, 50 x 50   970   306    237 ms
-//   2,000 sightlines on 100 deg^2            125   39.9   30.9
-//   48 sightlines (one wave)                 1.58  0.17   0.18
-//   observing, 500 sightlines                11.3  7.3    6.4
+//                                            that  bands  + tables,  + arguments
+//                                                         pipeline   in shared
+//   16,000 sightlines at 16/deg^2, 50 x 50   970   306    237        228 ms
+//   2,000 sightlines on 100 deg^2            125   39.9   32.3       29.8
+//   48 sightlines (one wave)                 1.58  0.17   0.18       0.17
+//   observing, 500 sightlines                11.3  7.3    6.5        6.4
+//   1,201 masked (pointer sweep: 133)                     21.0       19.5
 // "Tables, pipeline": rows of code edges from a level table instead of a
 // bisection (the bisection and its dependent reads took a fifth of the time),
 // boundaries read from a skewed table (one sector for four lanes), two item
@@ -94,6 +96,16 @@ struct BandItem {
   Dest d;
 };
 
+// The CTA's two items and the launch's arguments for the functions that are
+// not inlined: through a reference to the kernel's parameters they would read
+// them by generic loads.
+__shared__ BandItem s_item[2];
+__shared__ PairArgs s_args;
+
+struct Sums6 {
+  double a, b, c, d, e, f;
+};
+
 // ---- the item pipeline ----------------------------------------------------
 // Two item buffers per CTA.  Warp 0 prepares item k + 1 (claims it, finds its
 // bands, starts the bulk copies of its prefix sums and row values) before its
@@ -133,8 +145,9 @@ __device__ __forceinline__ int edge_column(const PairArgs& A, const RowV& R, con
 // prefix sums, for a bin whose telescoped sums cancel to rounding level: a
 // bin all of whose weights are zero sums to exactly zero this way.
 template <int COORD, bool MINPOS, bool GAPS>
-__device__ __noinline__ void band_by_rows(const PairArgs& A, const BandItem& it, const float* U, const uint16_t* tt,
-                                          int g0, int g1, int code, double* out) {
+__device__ __noinline__ Sums6 band_by_rows(const BandItem& it, const float* U, const uint16_t* tt, int g0, int g1,
+                                           int code) {
+  const PairArgs& A = s_args;
   double s[6] = {0, 0, 0, 0, 0, 0};
   unsigned rech = 0;
   const int fi = it.fi, fj = it.fj, nj = it.nj;
@@ -158,8 +171,7 @@ __device__ __noinline__ void band_by_rows(const PairArgs& A, const BandItem& it,
     s[4] += r.y * m;
     s[5] += one * dw;
   }
-#pragma unroll
-  for (int f = 0; f < 6; ++f) out[f] = s[f];
+  return Sums6{s[0], s[1], s[2], s[3], s[4], s[5]};
 }
 
 // Add the row values r (and m: with gaps) times the column sums p (and c).
@@ -227,7 +239,7 @@ __device__ __forceinline__ void add_edge_row(const PairArgs&, const BandItem& it
 // U: the grid's values (in shared memory where the kernel stages them).
 template <int COORD, bool MINPOS, bool GAPS>
 __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it, const float* U, int t0, int m,
-                                           int lane, unsigned long long* stats) {
+                                           int lane, int buf, unsigned long long* stats) {
   const int n0 = (int)A.g.n0, n1 = (int)A.g.n1;
   const int t = t0 + min(lane, m);
   const bool bound = lane <= m;           // this lane owns a boundary
@@ -443,10 +455,11 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
     }
     if (owner && F.n != 0u && code >= 0) {
       if (tiny) {
-        double s[6];
-        band_by_rows<COORD, MINPOS, GAPS>(A, it, U, tt, min(z1, y), y, code, s);
-#pragma unroll
-        for (int f = 0; f < 6; ++f) F.s[f] = s[f];
+        // (observing: by the caller's copy, which then lives in memory and leaves
+        // the sweep its registers: 7.3 -> 6.4 ms for 500 sightlines)
+        const Sums6 q =
+            band_by_rows<COORD, MINPOS, GAPS>(COORD == kObs ? it : s_item[buf], U, tt, min(z1, y), y, code);
+        F.s[0] = q.a, F.s[1] = q.b, F.s[2] = q.c, F.s[3] = q.d, F.s[4] = q.e, F.s[5] = q.f;
       }
       F.s[6] = __fma_rn(A.lmid, (double)F.n, zc);
       F.code = code;
@@ -466,8 +479,9 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
 // Prepare the next owned item into `h` (all lanes of one warp; SMEM: its data
 // into buf, arriving on `full`).
 template <int COORD, bool SMEM, bool GAPS>
-__device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, int* next, double2* buf,
-                                          unsigned long long* full, int lane, unsigned long long& n_taken) {
+__device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, unsigned long long* full, int lane) {
+  const PairArgs& A = s_args;
+  int taken = 0;
   const int nb = 2 * (int)A.g.n0 + 1;
   BandItem it;
   it.bands = 0;
@@ -477,7 +491,7 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, int* n
     idx = __shfl_sync(kFull, idx, 0);
     if (idx >= A.n_items) break;
     if (item_owner(A, idx) != (GAPS ? kOwnerGaps : kOwnerGrid)) continue;  // another kernel's item
-    ++n_taken;
+    ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
     it.ni = (int)A.gspan[i];
     it.nj = (int)A.gspan[j];
@@ -544,13 +558,14 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, int* n
       }
     }
     __syncwarp();
-    return;
+    return taken;
   }
   if (lane == 0) {  // no item left
     *h = it;
     bar_arrive(full);
   }
   __syncwarp();
+  return taken;
 }
 
 // The arguments stay in the kernel's parameter space (__grid_constant__):
@@ -558,7 +573,6 @@ __device__ __noinline__ void prepare_item(const PairArgs& A, BandItem* h, int* n
 template <int COORD, bool MINPOS, bool SMEM, bool GAPS>
 __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kernel(const __grid_constant__ PairArgs A) {
   extern __shared__ double2 band_smem[];
-  __shared__ BandItem s_item[2];
   __shared__ int s_next[2];  // GAPS: next group of each item
   __shared__ unsigned long long s_full[2], s_empty[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -570,6 +584,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
     U = u;
   }
   if (tid == 0) {
+    s_args = A;
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
       bar_init(&s_empty[b], kGridWarps<GAPS>);
@@ -581,7 +596,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
   unsigned long long n_taken = 0;
   bool ok = true, ended = false;
   if (warp == 0)
-    prepare_item<COORD, SMEM, GAPS>(A, &s_item[0], &s_next[0], band_smem, &s_full[0], lane, n_taken);
+    n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[0], &s_next[0], band_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u, parity = (k >> 1) & 1u;
     ok = bar_wait(&s_full[b], parity);
@@ -599,8 +614,8 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
       // item k - 1 (the other buffer's) is done by every warp
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
       if (!ok) break;
-      prepare_item<COORD, SMEM, GAPS>(A, &s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
-                                      &s_full[nb], lane, n_taken);
+      n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
+                                                 &s_full[nb], lane);
       ended = s_item[nb].bands == 0;
     }
     for (int q = warp;; q += kGridWarps<GAPS>) {
@@ -609,7 +624,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
         q = __shfl_sync(kFull, q, 0);
       }
       if (q * it.per >= it.bands) break;
-      band_group<COORD, MINPOS, GAPS>(A, it, U, it.tf + q * it.per, min(it.per, it.bands - q * it.per), lane, stats);
+      band_group<COORD, MINPOS, GAPS>(A, it, U, it.tf + q * it.per, min(it.per, it.bands - q * it.per), lane, (int)b, stats);
     }
     __syncwarp();
     if (lane == 0) bar_arrive(&s_empty[b]);
