@@ -33,10 +33,10 @@
 // keys and the pair-by-pair blocks (6.6 % of the pairs).
 //
 // Measured on a B200 against the version that binned every pair (one warp per
-// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 266 ms; five mocks
-// of 5,000 sightlines in all: 292 -> 158 ms; jackknife of 2,500 sightlines (its
+// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 264 ms; five mocks
+// of 5,000 sightlines in all: 292 -> 156 ms; jackknife of 2,500 sightlines (its
 // few rows once went to the pixel-pair kernel: low words of 32 bits could have
-// wrapped after 2^32 adds): 363 -> 96 ms.  Block bounds from the extremes of
+// wrapped after 2^32 adds): 363 -> 95 ms.  Block bounds from the extremes of
 // d1 d2 instead of r^2 sent twice the blocks pair by pair; functions that are
 // not inlined and read the arguments through the kernel's parameters cost 6 %;
 // one lane per run with its own 15 adds touched 32 lines an add and took 30 of
@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
   __syncthreads();
   unsigned long long n_eval = 0;
   unsigned long long n_taken = 0;
-  bool ok = true, ended = false;
+  bool ok = true;
   if (warp == 0) n_taken += prepare_diag<SMEM>(&s_item[0], &s_next[0], diag_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u;
@@ -644,13 +644,12 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
       it.rows = diag_smem + (size_t)b * buf_len;
       it.cols = it.rows + A.max_np + 3 * kParityPad;
     }
-    if (warp == 0 && !ended) {
+    if (((warp - (int)k) & (kDiagWarps - 1)) == 0) {  // the warps take turns
       const uint32_t nb = b ^ 1u;
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);  // item k - 1 is done by every warp
       if (!ok) break;
       n_taken += prepare_diag<SMEM>(&s_item[nb], &s_next[nb], diag_smem + (SMEM ? (size_t)nb * buf_len : 0),
                                     &s_full[nb], lane);
-      ended = s_item[nb].groups == 0;
     }
     for (;;) {
       int q = 0;

@@ -45,13 +45,13 @@
 //
 // Measured on a B200 against the version that evaluated the r_perp code at
 // every boundary of every row and bisected each split run (one warp per item):
-//                                            that  bands  + tables,  + arguments
-//                                                         pipeline   in shared
-//   16,000 sightlines at 16/deg^2, 50 x 50   970   306    237        228 ms
-//   2,000 sightlines on 100 deg^2            125   39.9   32.3       29.8
+//                                            that  bands  + tables,  + arguments in
+//                                                         pipeline   shared, turns
+//   16,000 sightlines at 16/deg^2, 50 x 50   970   306    237        216 ms
+//   2,000 sightlines on 100 deg^2            125   39.9   32.3       28.2
 //   48 sightlines (one wave)                 1.58  0.17   0.18       0.17
-//   observing, 500 sightlines                11.3  7.3    6.5        6.4
-//   1,201 masked (pointer sweep: 133)                     21.0       19.5
+//   observing, 500 sightlines                11.3  7.3    6.5        5.5
+//   1,201 masked (pointer sweep: 133)                     21.0       19.4
 // "Tables, pipeline": rows of code edges from a level table instead of a
 // bisection (the bisection and its dependent reads took a fifth of the time),
 // boundaries read from a skewed table (one sector for four lanes), two item
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
   __syncthreads();
   unsigned long long stats[2] = {0ull, 0ull};  // pairs in bands, FP64 re-evaluations
   unsigned long long n_taken = 0;
-  bool ok = true, ended = false;
+  bool ok = true;
   if (warp == 0)
     n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[0], &s_next[0], band_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
@@ -609,16 +609,19 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
       it.C = it.P + 2 * len;
       it.M = it.P + 3 * len;
     }
-    if (warp == 0 && !ended) {
+    // groups go round the warps from item to item, and the warp with the last
+    // one, often none, prepares the next item (2,000 sightlines: 29.8 ms with a
+    // fixed producer, 28.3; 328,000 pairs of 16-pixel sightlines: 4.9 ms, 2.7)
+    const int q0 = (warp - (int)k) & (kGridWarps<GAPS> - 1);
+    if (q0 == kGridWarps<GAPS> - 1) {
       const uint32_t nb = b ^ 1u;
       // item k - 1 (the other buffer's) is done by every warp
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
       if (!ok) break;
       n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
                                                  &s_full[nb], lane);
-      ended = s_item[nb].bands == 0;
     }
-    for (int q = warp;; q += kGridWarps<GAPS>) {
+    for (int q = q0;; q += kGridWarps<GAPS>) {
       if (GAPS) {  // more warps than an item has groups: from a counter
         if (lane == 0) q = atomicAdd(&s_next[b], 1);
         q = __shfl_sync(kFull, q, 0);
