@@ -878,8 +878,8 @@ extern "C" tos_status tos_brute_tune(tos_engine* e, const float* points, size_t 
 // Some callers cannot allocate device memory while they count pairs: code
 // that manages every byte of the GPU through its own pool, code that runs
 // where a cudaMalloc would synchronise the device or is not allowed, or
-// service loops that must not touch the allocator at all.  tos_brute_run allocates its
-// scratch on every call; tos_brute_run_noalloc takes its inputs and outputs
+// service loops that must not touch the allocator at all.  tos_brute_run keeps its
+// scratch with the engine and grows it; tos_brute_run_noalloc takes its inputs and outputs
 // in device memory and keeps all scratch in one statically sized device
 // array that the library reserves on every GPU that loads it, until exit.
 // ============================================================================

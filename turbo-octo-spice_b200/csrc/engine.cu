@@ -1489,7 +1489,7 @@ size_t Workspace::bytes() const {
          d_item_off.bytes() + d_item_i.bytes() + d_item_j.bytes() + d_item_sep.bytes() +
          d_item_c.bytes() + d_cell_pairs.bytes() + d_acc.bytes() + d_out.bytes() +
          d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_ginv.bytes() + d_gtb.bytes() +
-         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_pthr.bytes() + d_pthr.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
+         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_pthr.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
 }
 
 // Counter words of a run: kernel counters [0, 16), the theta-edge flags of

@@ -248,7 +248,7 @@ struct tos_catalog {
   double min_gap = 0;               // smallest positive distance step within a sightline (lower bound)
   uint32_t max_np = 0;
   // common first-axis grids (0: distance, 1: loglam), built on first use
-  std::mutex grid_mu;                                  // guards the grid build
+  mutable std::mutex grid_mu;                                  // guards the grid build
   bool grid_built[2] = {false, false};
   int grid_n[2] = {0, 0};                              // distinct values (0: no usable grid)
   uint64_t grid_los[2] = {0, 0};                       // sightlines contiguous on the grid

@@ -86,7 +86,15 @@ uint64_t workspace_estimate(const tos_catalog* cat, const tos_grid& g, double sc
   bytes += pairs * 20.0;                                      // items (i, j, cos, theta index)
   bytes += n * 24.0;                                          // per primary counts and offsets
   bytes += nc * (near_cells + 12.0) * 4.0;                    // cell neighbours
-  bytes += 4192.0 * 8 + 2.0 * 65536 * (g.axis[0].nbins + 1.0) + 1e6;  // counters, tables, cub
+  // boundary tables of the grid sweep: 22 bytes a boundary and grid value
+  double tables = 2.0 * 65536 * (g.axis[0].nbins + 1.0);
+  {
+    const int w = g.type == TOS_OBSERVING ? 1 : 0;
+    std::lock_guard<std::mutex> lock(cat->grid_mu);
+    if (g.type != TOS_POLAR && cat->grid_built[w])
+      tables = std::max(tables, 2.0 * (g.axis[0].nbins + 1.0) * (cat->grid_n[w] + 64.0) * 24.0);
+  }
+  bytes += 4192.0 * 8 + tables + 1e6;  // counters, tables, cub
   return (uint64_t)bytes;
 }
 
