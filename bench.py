@@ -423,11 +423,11 @@ def engine_arm(args, D):
         value = D.world * pairs * args.steps / (ms_max / 1e3)
         e2e_value = D.world * pairs * args.steps / D.max(wall)
         kernel_ms = ms / args.steps
-        kernel_name = "brute_kernel"
+        kernel_name = "line_kernel"  # the grid's points come in lines of equal steps
         evaluated = pairs
         h2d = pts.nbytes
         d2h = 102 * 24
-        launches = 3 * args.steps
+        launches = 6 * args.steps  # bounds, two line checks, preparation, pairs, finish
         st = {}
         par = None
         if D.rank == 0 and D.world == 1 and not args.no_parity:
