@@ -162,7 +162,7 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
 // max_ang + r_A + r_B (caps bound every member).  Only cells of A's own
 // sightline group are searched.
 // One warp per cell; a cell's neighbours are in ascending order.  (2,028 cells,
-// both passes: 1.5 ms with one thread a cell, 0.05 ms.)
+// both passes: 1.5 ms with one thread a cell, 0.07 ms.)
 __global__ void k_cell_neighbours(const double4* cap, const uint2* grange, uint32_t n_cells,
                                   double max_ang, const uint32_t* start, uint32_t* count,
                                   uint32_t* out) {
@@ -375,7 +375,8 @@ __global__ void k_expand(const uint32_t* members, uint32_t n_members, const uint
 // Eight lanes take a bin, a field each, so that a cell's 128-byte entry is read
 // by one group of lanes; the loads of eight cells are in flight while the sums
 // stay in order.  Bound by the bytes of the entries: 2,028 cells of 2,500 bins
-// (649 MB) took 6 ms with one thread a bin, whose loads waited for each other.
+// (649 MB) take 0.5 ms; 6 ms with one thread a bin, whose loads waited for each
+// other.
 static_assert(sizeof(tos_xibin) == 64 && offsetof(tos_xibin, num_pairs) == 56, "eight 8-byte fields");
 __global__ void __launch_bounds__(128) k_combine(const unsigned long long* acc, const uint32_t* gstart,
                                                  uint32_t n_groups, uint32_t n_cells, uint32_t nb, double4 inv_a,
