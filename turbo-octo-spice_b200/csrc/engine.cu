@@ -537,6 +537,20 @@ std::vector<float4> code_edges(const RefGrid& g, int k1, double jit) {
   return e;
 }
 
+// Smallest FP32 r^2 at which the FP32 codes of a Polar pair are within half of
+// their 2^-k windows of the reference's t.  r^2 = (d2 - d1)^2 + (2(1 - c) d1 d2 -
+// err), where err, the rounding of the reference's float d1^2, is up to J =
+// 2^-24 D^2 (D the largest distance): the two cancel near r = 0, and the
+// product's relative 2^-23 leaves an error e of up to 2^-23 J in r^2 whatever its
+// size.  t0 = r inv0 then moves by inv0 e / (2 r) and t1 = mu inv1 by at most
+// t1 e / (2 r^2); both bounds are taken twice.  (D = 8,000 and 50 mu bins: 0.37.)
+float polar_r2_small(const RefGrid& g, double max_d, int k0, int k1) {
+  const double e = std::ldexp(max_d * max_d, -47);
+  const double t1 = std::min(g.inv1, (double)g.n1 + 2.0 + std::fabs(g.min1 * g.inv1));
+  const double r0 = 2.0 * std::ldexp(g.inv0 * e, k0);
+  return (float)std::max({1e-4, r0 * r0, 2.0 * std::ldexp(t1 * e, k1)});
+}
+
 // Thresholds of the Polar codes (PairArgs::thr_r2, thr_mu2): code >= k means
 // ref_u32((x - min) * inv) >= k with t > -1 (k = 0: t > -1).
 std::vector<double> polar_thresholds(const RefGrid& g) {
@@ -1825,7 +1839,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   A.mag1 = std::ldexp(1.5f, 23 - A.k1);
   std::memcpy(&A.bits0, &A.mag0, 4);
   std::memcpy(&A.bits1, &A.mag1, 4);
-  A.r2_small = 1e-4f;
+  A.r2_small = G.type == TOS_POLAR ? polar_r2_small(rg, cat->max_d, A.k0, A.k1) : 1e-4f;
   const bool exact0 = (G.type != TOS_POLAR) && rg.min0 == 0.0 && is_pow2(rg.inv0);
   const bool minpos = (rg.min0 > 0.0) || (G.type != TOS_OBSERVING && rg.min1 > 0.0) ||
                       (rg.min0 < 0.0) || (G.type != TOS_OBSERVING && rg.min1 < 0.0);

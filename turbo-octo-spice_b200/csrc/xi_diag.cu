@@ -95,7 +95,9 @@ struct DRow {
 
 // FP32 Polar key of one pixel pair (packed b0 << 16 | b1, or kInvalidKey) and
 // whether it lies within 2^-K bins of an edge (or r^2 is tiny) and must be
-// re-binned in FP64.  The same decision as xi_kernels.cu fast_bin.
+// re-binned in FP64.  The same decision as xi_kernels.cu fast_bin.  c0, c1: its
+// codes, or kNoCode in c0 below r2_small, where they are no guide.
+constexpr int kNoCode = -0x40000000;
 template <bool MINPOS>
 __device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, float x2, bool& recheck, int& c0,
                                               int& c1) {
@@ -114,7 +116,7 @@ __device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, 
     coarse = coarse && (t0 > -2.0f) && (t1 > -2.0f);
   }
   int b0 = q0 >> A.k0, b1 = q1 >> A.k1;
-  c0 = b0;
+  c0 = small ? kNoCode : b0;
   c1 = b1;
   if (MINPOS) {
     b0 = max(b0, 0);
@@ -128,8 +130,8 @@ __device__ __forceinline__ uint32_t polar_key(const PairArgs& A, const DRow& R, 
 // Exact key of a pair near an edge whose FP32 codes are b0, b1 (each within
 // one of the exact code): the reference's r^2 against the smallest r^2 of each
 // r code (thr_r2), and |d2 - d1|^2 against thr_mu^2 r^2, where mu's rounding
-// cannot matter beyond 1e-14 relative; closer than that, or at a tiny r, the
-// reference's own expression decides.
+// cannot matter beyond 1e-14 relative; closer than that, or without codes
+// (kNoCode: a tiny r), the reference's own expression decides.
 __device__ __noinline__ uint32_t polar_key_exact(const PairArgs& A, float d1, float d2, double c, int b0, int b1) {
   const double r1_sq = (double)fmul(d1, d1);
   const double two_r1_cos12 = dmul((double)fmul(2.0f, d1), c);
@@ -140,7 +142,7 @@ __device__ __noinline__ uint32_t polar_key_exact(const PairArgs& A, float d1, fl
   const int e0 = a0 - 1 + (r_sq >= A.thr_r2[a0] ? 1 : 0) + (r_sq >= A.thr_r2[a0 + 1] ? 1 : 0);
   const double ma = A.thr_mu2[a1] * r_sq, mb = A.thr_mu2[a1 + 1] * r_sq;
   const bool close = fabs(s2 - ma) <= 1e-14 * s2 || fabs(s2 - mb) <= 1e-14 * s2;
-  if (close || !(r_sq > 1e-6)) {
+  if (close || b0 == kNoCode) {
     uint32_t p0 = 0, p1 = 0;
     return exact_polar(d1, d2, c, A.g, &p0, &p1) ? ((p0 << 16) | p1) : kInvalidKey;
   }

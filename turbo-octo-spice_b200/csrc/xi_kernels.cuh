@@ -95,7 +95,7 @@ struct PairArgs {
   float mag0, mag1;          // 1.5 * 2^(23-K) for the two axes
   int k0, k1;                // fractional bits kept (edge half-width 2^-K)
   int bits0, bits1;          // bit patterns of mag0/mag1
-  float r2_small;            // Polar: squared separations below this are re-binned in FP64
+  float r2_small;            // Polar: squared separations below this are re-binned in FP64 (polar_r2_small)
   float win_lim;             // |x1 - x2| >= win_lim (float) is always rejected
   double polar_r2;           // Polar: R^2 of the largest accepted r (with margin), or 0
   float jit2;                // Polar: bound on the float rounding of d1^2
