@@ -73,13 +73,14 @@ struct BruteArgs {
   int exact_diff;         // differences of coordinates are exact in FP32
   int wshift;             // log2 of the copies of a window slot (lane l adds to copy l mod 2^wshift)
   int copies;             // copies of the global sums, to spread the adds over (k_brute_finish adds them up)
+  int carry;              // the global sums are 128-bit integers with a carry (brute_args)
   // line_kernel: Q lines of P points, step (sx, sy, sz)
   int P, Q, eblocks;      // eblocks: offset blocks per unit
   float sx, sy, sz;
   const double2* val;     // (w*delta, w), point z of line l at z Q + l
   const float4* base;     // first point of each line
   const double* th;       // [nbins + 3] exact-index thresholds on r^2 (brute_thresholds)
-  unsigned long long* acc;       // [nbins + 2][kBWin] 128-bit carry-free sums and counts
+  unsigned long long* acc;       // [copies][nbins + 2][kBWin] sums and counts
   unsigned long long* next;      // diagonal-group counter
   unsigned long long* counters;  // [0] FP64 re-binnings
 };
@@ -150,7 +151,10 @@ __device__ __forceinline__ void window_add(const BruteArgs& A, int* win, int S, 
 }
 
 // Add the warp window to the global sums (carry-free: low 32 bits and the
-// signed rest of each value) and clear it.
+// signed rest of each value; CARRY: 128-bit integers) and clear it.  (A
+// template: with the choice made at run time the scattered points' kernel took
+// 4 to 10 % longer.)
+template <bool CARRY>
 __device__ __noinline__ void brute_flush(const BruteArgs& A, int* win, int S, int lane) {
   __syncwarp();
   const int step = S << A.wshift;
@@ -172,8 +176,12 @@ __device__ __noinline__ void brute_flush(const BruteArgs& A, int* win, int S, in
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       const __int128 v = ((__int128)part[f][2] << 42) + ((__int128)part[f][1] << 21) + (__int128)part[f][0];
-      atomicAdd(&g[2 * f], (unsigned long long)v & 0xFFFFFFFFull);
-      const long long h = (long long)(v >> 32);
+      const unsigned long long lo = CARRY ? (unsigned long long)v : (unsigned long long)v & 0xFFFFFFFFull;
+      long long h = (long long)(v >> (CARRY ? 64 : 32));
+      if (CARRY)
+        h += atomicAdd(&g[2 * f], lo) > ~lo;  // the low word's carry
+      else
+        atomicAdd(&g[2 * f], lo);
       if (h != 0) atomicAdd(&g[2 * f + 1], (unsigned long long)h);
     }
     atomicAdd(&g[4], cnt);
@@ -186,7 +194,7 @@ __device__ __noinline__ void brute_flush(const BruteArgs& A, int* win, int S, in
 // 1 + g * 32K + K L + m, m = 0 .. K-1; segment s is the rows [s seg, (s + 1) seg).
 // A diagonal's runs end at a segment's end, whatever K is, so that the sums
 // do not depend on the launch shape.
-template <int K>
+template <int K, bool CARRY>
 __global__ void __launch_bounds__(kBruteWarpsMax * 32, K == 1 ? 2 : 1) brute_kernel(const __grid_constant__ BruteArgs A) {
   extern __shared__ int bsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -284,7 +292,7 @@ __global__ void __launch_bounds__(kBruteWarpsMax * 32, K == 1 ? 2 : 1) brute_ker
           // lane adds the run it keeps (scattered points: 32 runs a row)
           if (__any_sync(kFull, close && pm[m] != 0u)) {
             if (adds + per > kBruteAdds) {
-              brute_flush(A, win, S, lane);
+              brute_flush<CARRY>(A, win, S, lane);
               adds = 0;
             }
             if (pm[m] != 0u) window_add(A, win, S, lane, pbin[m], pm[m], pd[m], pw[m]);
@@ -324,7 +332,7 @@ __global__ void __launch_bounds__(kBruteWarpsMax * 32, K == 1 ? 2 : 1) brute_ker
 #pragma unroll
     for (int m = 0; m < K; ++m) {
       if (adds + 2 * per > kBruteAdds) {
-        brute_flush(A, win, S, lane);
+        brute_flush<CARRY>(A, win, S, lane);
         adds = 0;
       }
       if (pm[m] != 0u) window_add(A, win, S, lane, pbin[m], pm[m], pd[m], pw[m]);
@@ -333,7 +341,7 @@ __global__ void __launch_bounds__(kBruteWarpsMax * 32, K == 1 ? 2 : 1) brute_ker
       adds += 2 * per;
     }
   }
-  brute_flush(A, win, S, lane);
+  brute_flush<CARRY>(A, win, S, lane);
   for (int o = 16; o > 0; o >>= 1) n_recheck += __shfl_xor_sync(kFull, n_recheck, o);
   if (lane == 0) atomicAdd(&A.counters[0], n_recheck);
 }
@@ -387,6 +395,7 @@ __global__ void k_brute_bounds(const float* pts, int n, unsigned long long* out)
 // costs one 16-byte read per lane and a broadcast for 2 kLineE FP64 FMAs.
 // Values are stored by z, then line.
 constexpr int kLineE = 8;
+template <bool CARRY>
 __global__ void __launch_bounds__(kBruteWarpsMax * 32) line_kernel(const __grid_constant__ BruteArgs A) {
   extern __shared__ int bsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(kBruteWarpsMax * 32) line_kernel(const __grid_
         }
       }
       if (adds + per > kBruteAdds) {
-        brute_flush(A, win, S, lane);
+        brute_flush<CARRY>(A, win, S, lane);
         adds = 0;
       }
       adds += per;
@@ -463,7 +472,7 @@ __global__ void __launch_bounds__(kBruteWarpsMax * 32) line_kernel(const __grid_
       }
     }
   }
-  brute_flush(A, win, S, lane);
+  brute_flush<CARRY>(A, win, S, lane);
   for (int o = 16; o > 0; o >>= 1) n_recheck += __shfl_xor_sync(kFull, n_recheck, o);
   if (lane == 0) atomicAdd(&A.counters[0], n_recheck);
 }
@@ -514,15 +523,19 @@ __global__ void k_brute_prep(const float* pts, int n, float4* pos, double* wd) {
 }
 
 // 128-bit sums -> the caller's dsum, wsum (FP64) and counts.
-__global__ void k_brute_finish(const unsigned long long* acc, int nb2, int copies, double inv0, double inv1, double* dsum,
-                               double* wsum, uint64_t* counts) {
+__device__ __forceinline__ __int128 brute_sum(const unsigned long long* g, int carry) {
+  return carry ? (__int128)(((unsigned __int128)g[1] << 64) | g[0])
+               : (__int128)(long long)g[1] * (__int128)4294967296ll + (__int128)g[0];
+}
+__global__ void k_brute_finish(const unsigned long long* acc, int nb2, int copies, int carry, double inv0, double inv1,
+                               double* dsum, double* wsum, uint64_t* counts) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb2; b += gridDim.x * blockDim.x) {
     __int128 v0 = 0, v1 = 0;
     uint64_t m = 0;
     for (int c = 0; c < copies; ++c) {
       const unsigned long long* g = acc + ((size_t)c * nb2 + b) * kBWin;
-      v0 += (__int128)(long long)g[1] * (__int128)4294967296ll + (__int128)g[0];
-      v1 += (__int128)(long long)g[3] * (__int128)4294967296ll + (__int128)g[2];
+      v0 += brute_sum(g, carry);
+      v1 += brute_sum(g + 2, carry);
       m += g[4];
     }
     dsum[b] = i128_double(v0) * inv0;
@@ -542,9 +555,12 @@ struct BruteBounds {
 // The kernel's variants, by diagonals per lane.
 struct BruteVariant {
   int k;
-  void (*fn)(BruteArgs);
+  void (*fn[2])(BruteArgs);  // by BruteArgs::carry
 };
-const BruteVariant kVariants[] = {{1, brute_kernel<1>}, {2, brute_kernel<2>}, {4, brute_kernel<4>}};
+const BruteVariant kVariants[] = {{1, {brute_kernel<1, false>, brute_kernel<1, true>}},
+                                  {2, {brute_kernel<2, false>, brute_kernel<2, true>}},
+                                  {4, {brute_kernel<4, false>, brute_kernel<4, true>}}};
+const BruteVariant kLineVariant = {1, {line_kernel<false>, line_kernel<true>}};
 
 // Copies of window slots are made while a block stays below this much shared
 // memory, so that three blocks share an SM.
@@ -582,6 +598,12 @@ void brute_args(BruteArgs& A, int n, int nbins, double min, double max, const Br
     // units of one (line, 32 lines) where there are many, else of one offset block
     A.eblocks = (double)A.Q * A.Q >= 1e6 ? 1 << 20 : 1;
   }
+  // Carry-free sums hold a bin that takes every pair while its values, below
+  // 2^62 for A.seg pairs, add up to less than 2^94 and its flushes (at least
+  // 2^11 pairs each, but for the last ones) to less than 2^32.  Beyond that the
+  // low word's add returns its carry.
+  const double pairs = 0.5 * n * ((double)n - 1.0);
+  A.carry = pairs > 4294967296.0 * A.seg || pairs > 1099511627776.0 /* 2^40 */ ? 1 : 0;
   A.copies = std::max(1, std::min(64, kBruteAccBins / (nbins + 2)));
   A.n = n;
   A.nbins = nbins;
@@ -697,12 +719,12 @@ tos_status brute_launch_shape(tos_engine* e, BruteArgs A, cudaStream_t st, int v
   int warps = 0;
   size_t smem = 0;
   TOS_TRY(brute_shape(e, A.nbins, warps_max, &warps, &A.wshift, &smem));
-  const BruteVariant v = A.P ? BruteVariant{1, line_kernel} : kVariants[vi];
-  TOS_CUDA_TRY(cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const auto fn = (A.P ? kLineVariant : kVariants[vi]).fn[A.carry];
+  TOS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  TOS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.fn, warps * 32, smem));
+  TOS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem));
   TOS_CUDA_TRY(cudaEventRecord(e->ev[4], st));
-  v.fn<<<e->num_sms * std::max(1, per_sm), warps * 32, smem, st>>>(A);
+  fn<<<e->num_sms * std::max(1, per_sm), warps * 32, smem, st>>>(A);
   TOS_CUDA_TRY(cudaGetLastError());
   TOS_CUDA_TRY(cudaEventRecord(e->ev[5], st));
   return TOS_OK;
@@ -810,8 +832,8 @@ extern "C" tos_status tos_brute_run(tos_engine* e, const float* points, size_t n
   TOS_TRY(brute_setup(e, points, n, min, max, nbins, &A));
   TOS_TRY(brute_launch(e, A, st));
   double* out = e->brute.out.p;  // dsum, wsum, counts
-  k_brute_finish<<<(nb2 + 127) / 128, 128, 0, st>>>(A.acc, nb2, A.copies, brute_inv_scale(A, 0), brute_inv_scale(A, 1), out,
-                                                   out + nb2, reinterpret_cast<uint64_t*>(out + 2 * nb2));
+  k_brute_finish<<<(nb2 + 127) / 128, 128, 0, st>>>(A.acc, nb2, A.copies, A.carry, brute_inv_scale(A, 0),
+                                                   brute_inv_scale(A, 1), out, out + nb2, reinterpret_cast<uint64_t*>(out + 2 * nb2));
   TOS_CUDA_TRY(cudaGetLastError());
   std::vector<double> h((size_t)3 * nb2);
   TOS_CUDA_TRY(cudaMemcpyAsync(h.data(), out, h.size() * 8, cudaMemcpyDeviceToHost, st));
@@ -973,8 +995,8 @@ extern "C" tos_status tos_brute_run_noalloc(tos_engine* e, const float* d_points
   A.next = misc;
   A.counters = misc + 1;
   TOS_TRY(brute_launch(e, A, st));
-  k_brute_finish<<<(nb2 + 127) / 128, 128, 0, st>>>(acc, nb2, A.copies, brute_inv_scale(A, 0), brute_inv_scale(A, 1),
-                                                   d_dsum, d_wsum, d_counts);
+  k_brute_finish<<<(nb2 + 127) / 128, 128, 0, st>>>(acc, nb2, A.copies, A.carry, brute_inv_scale(A, 0),
+                                                   brute_inv_scale(A, 1), d_dsum, d_wsum, d_counts);
   TOS_CUDA_TRY(cudaGetLastError());
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   if (ms_kernel) {
