@@ -86,6 +86,7 @@ struct DItem {
 // them by generic loads.
 __shared__ DItem s_item[2];
 __shared__ PairArgs s_args;
+__shared__ Claim s_claim;  // of the warp that prepares an item
 
 // Row values of the pixel-pair kernel's Polar fast path (xi_kernels.cu
 // fast_bin): x1 = d1, A1 = d1 * 2(1 - c), dl1 = -(d1*d1 - fl(d1*d1)).
@@ -520,10 +521,7 @@ __device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsi
   it.groups = 0;
   for (;;) {
     unsigned long long idx = 0;
-    if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
-    idx = __shfl_sync(kFull, idx, 0);
-    if (idx >= A.n_items) break;
-    if (item_owner(A, idx) != kOwnerDiag) continue;  // the pixel-pair kernel's item
+    if (!claim_item(A, kOwnerDiag, s_claim, lane, idx)) break;
     ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
     it.ni = (int)A.npix[i];
@@ -625,6 +623,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
   if (lane == 0) Q.rech = 0ull;
   if (tid == 0) {
     s_args = A;
+    s_claim.todo = 0u;
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
       bar_init(&s_empty[b], kDiagWarps);

@@ -101,6 +101,7 @@ struct BandItem {
 // them by generic loads.
 __shared__ BandItem s_item[2];
 __shared__ PairArgs s_args;
+__shared__ Claim s_claim;  // of the warp that prepares an item
 
 struct Sums6 {
   double a, b, c, d, e, f;
@@ -487,10 +488,7 @@ __device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, u
   it.bands = 0;
   for (;;) {
     unsigned long long idx = 0;
-    if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
-    idx = __shfl_sync(kFull, idx, 0);
-    if (idx >= A.n_items) break;
-    if (item_owner(A, idx) != (GAPS ? kOwnerGaps : kOwnerGrid)) continue;  // another kernel's item
+    if (!claim_item(A, GAPS ? kOwnerGaps : kOwnerGrid, s_claim, lane, idx)) break;
     ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
     it.ni = (int)A.gspan[i];
@@ -585,6 +583,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
   }
   if (tid == 0) {
     s_args = A;
+    s_claim.todo = 0u;
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
       bar_init(&s_empty[b], kGridWarps<GAPS>);
