@@ -639,7 +639,8 @@ __device__ __forceinline__ int grid_index(const float* U, int ng, float x) {
 // 102 / 28, 150 of 600 25 / 22 | 60 / 21; 320k / 719k items of 64 of 128
 // values 10.9 / 20.0 | 19.0 / 21.3, 43 of 128 10.5 / 19.9 | 13.0 / 15.2, 16 of
 // 64 7.3 / 12.4 | 4.6 / 6.0).  count[0]: contiguous sightlines, count[1]:
-// those with gaps, count[2]: largest span.
+// those with gaps, count[2]: largest span, count[3]: contiguous ones of at most
+// kShortPixels pixels.
 __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint32_t* npix, size_t n_los,
                              const float* U, int ng, uint32_t* gfirst, uint32_t* gspan, unsigned long long* count) {
   const int lane = threadIdx.x & 31;
@@ -664,6 +665,7 @@ __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint3
       if (f != kNoGrid) {
         atomicAdd(&count[span == n ? 0 : 1], 1ull);
         atomicMax(&count[2], (unsigned long long)span);
+        if (span == n && n <= kShortPixels) atomicAdd(&count[3], 1ull);
       }
     }
   }
@@ -909,14 +911,14 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   TOS_TRY(cat->d_gfirst[w].alloc(cat->n_los));
   TOS_TRY(cat->d_gspan[w].alloc(cat->n_los));
   DevBuf<unsigned long long> nok;
-  TOS_TRY(nok.alloc(3));
-  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 24, st));
+  TOS_TRY(nok.alloc(4));
+  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 32, st));
   const int gw = grid_for(e, cat->n_los * 32, 256);
   k_grid_first<<<gw, 256, 0, st>>>(x, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_grid[w].p, ng,
                                    cat->d_gfirst[w].p, cat->d_gspan[w].p, nok.p);
   TOS_CUDA_TRY(cudaGetLastError());
-  unsigned long long h[3] = {0, 0, 0};
-  TOS_CUDA_TRY(cudaMemcpyAsync(h, nok.p, 24, cudaMemcpyDeviceToHost, st));
+  unsigned long long h[4] = {0, 0, 0, 0};
+  TOS_CUDA_TRY(cudaMemcpyAsync(h, nok.p, 32, cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   if (h[0] + h[1] == 0) return TOS_OK;
   // for contiguous sightlines the grid sweep takes a pixel's loglam from its
@@ -975,6 +977,7 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   cat->grid_n[w] = ng;
   cat->max_span[w] = (uint32_t)h[2];
   cat->grid_los[w] = h[0];
+  cat->grid_short[w] = h[3];
   cat->grid_gaps[w] = h[1];
   return TOS_OK;
 }
@@ -1513,7 +1516,9 @@ size_t Workspace::bytes() const {
 constexpr int kChunkCounters = 4128;
 constexpr int kMaxChunks = 64;
 constexpr uint64_t kChunkItemsMin = 131072;  // tens of ms per chunk: the launch tail stays small
-constexpr size_t kCounterWords = kChunkCounters + kMaxChunks;
+// sweeps that a request runs in chunks
+enum SweepKind { kSweepDiag = 0, kSweepGrid, kSweepShort, kSweepKinds };
+constexpr size_t kCounterWords = kChunkCounters + kSweepKinds * kMaxChunks;
 
 // Host callback after a shared-GPU sweep chunk: hands the SMs back.
 static void CUDART_CB sweep_chunk_done(void* share) { static_cast<SweepShare*>(share)->release(); }
@@ -1665,7 +1670,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // [0..3] kernel counters, [4] pair-kernel item counter, [5] candidates,
   // [6] window flushes, [7] run-kernel item counter, [8] run items, [9] grid
   // items, [10] grid-kernel item counter, [11] diagonal-kernel item counter,
-  // [12] diagonal items, [13] a wait of a sweep ran out, [14] gap-kernel item counter,
+  // [12] diagonal items, [13] a wait of a sweep ran out, [14] gap-kernel item counter, [15] short-item kernel's,
   // [16] theta indices on an edge, [17..] their item numbers (4096 at most)
   unsigned long long* ctr = ws->d_counters.p;
   const double theta_min = G.axis[1].min, theta_inv = 1.0 / axis_width(G.axis[1]);
@@ -1927,7 +1932,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     }
   }
   // --- grid sweep: catalogues whose first-axis values lie on a small common grid
-  bool use_grid = false;
+  bool use_grid = false, use_short = false;
   std::vector<float4> edges;  // kept until the stream sync
   if (use_runs) {
     const int w = (G.type == TOS_OBSERVING) ? 1 : 0;
@@ -1989,7 +1994,8 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       A.max_span = (int)cat->max_np;
       // contiguous sightlines on a grid that fixes loglam; the others with gaps
       A.grid_split = cat->grid_geo[w] && cat->grid_los[w] > 1;
-      use_grid = A.grid_split != 0;
+      use_grid = A.grid_split && cat->grid_los[w] > cat->grid_short[w];
+      use_short = A.grid_split && cat->grid_short[w] > 1;
       if (cat->d_gap_off[w].p) {
         A.gap_off = cat->d_gap_off[w].p;
         A.gap_pre = cat->d_gap_pre[w].p;
@@ -2073,21 +2079,27 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     TOS_CUDA_TRY(cudaMemsetAsync(ctr, 0, 4 * 8, st));          // evaluated, rechecks, overflow, direct
     TOS_CUDA_TRY(cudaMemsetAsync(ctr + 6, 0, 7 * 8, st));      // flushes, item counters, taken
   }
-  // Dominant kernel (grid or diagonal sweep): one persistent launch, or for
-  // a shared GPU (SweepShare) a chain of chunk launches, each with its own
-  // item counter (ctr[kChunkCounters + k], after the theta-edge flags of
-  // observing grids at ctr[16 ..]) and its CTA count asked just before launch.
-  auto sweep = [&](bool diag, unsigned long long* counter) -> tos_status {
-    auto launch = [&](const PairArgs& R, int per_sm) -> cudaError_t {
-      return diag ? launch_diag_kernel(R, minpos, e->num_sms, per_sm, st)
-                  : launch_grid_kernel(R, G.type, minpos, e->num_sms, per_sm, st);
+  // A sweep: one persistent launch, or for a shared GPU (SweepShare) a chain
+  // of chunk launches, each with its own item counter (ctr[kChunkCounters ..],
+  // after the theta-edge flags of observing grids at ctr[16 ..]) and its CTA
+  // count asked just before launch.
+  static const char* const sweep_name[kSweepKinds] = {"diagonal", "grid", "short"};
+  auto sweep = [&](SweepKind kind, unsigned long long* counter) -> tos_status {
+    auto launch = [&](PairArgs& R, int per_sm) -> cudaError_t {
+      switch (kind) {
+        case kSweepDiag: return launch_diag_kernel(R, minpos, e->num_sms, per_sm, st);
+        case kSweepGrid: return launch_grid_kernel(R, G.type, minpos, e->num_sms, per_sm, st);
+        default:
+          R.max_span = std::min(R.max_span, (int)kShortPixels);
+          return launch_short_kernel(R, G.type, minpos, e->num_sms, st);
+      }
     };
     if (!share) {
       PairArgs R = A;
       R.next_item = counter;
       const cudaError_t ke = launch(R, ctas_per_sm);
       if (ke != cudaSuccess)
-        return fail(TOS_ERR_CUDA, std::string(diag ? "diagonal" : "grid") + " kernel: " + cudaGetErrorString(ke));
+        return fail(TOS_ERR_CUDA, std::string(sweep_name[kind]) + " kernel: " + cudaGetErrorString(ke));
       return TOS_OK;
     }
     const uint64_t chunks = std::max<uint64_t>(
@@ -2102,13 +2114,13 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       R.item_c = A.item_c + a;
       R.item_sep = (G.type == TOS_OBSERVING) ? A.item_sep + a : A.item_sep;
       R.n_items = b - a;
-      R.next_item = ctr + kChunkCounters + c;
+      R.next_item = ctr + kChunkCounters + kind * kMaxChunks + c;
       const uint64_t remaining = (uint64_t)((double)n_pixel_pairs * (double)(n_items - a) / (double)n_items);
       const int per_sm = share->acquire(remaining);
       const cudaError_t ke = launch(R, per_sm);
       if (ke != cudaSuccess) {
         share->release();
-        return fail(TOS_ERR_CUDA, std::string(diag ? "diagonal" : "grid") + " kernel: " + cudaGetErrorString(ke));
+        return fail(TOS_ERR_CUDA, std::string(sweep_name[kind]) + " kernel: " + cudaGetErrorString(ke));
       }
       const cudaError_t he = cudaLaunchHostFunc(st, sweep_chunk_done, const_cast<SweepShare*>(share));
       if (he != cudaSuccess) {
@@ -2121,9 +2133,10 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   };
   if (n_items > 0) {
     TOS_CUDA_TRY(cudaEventRecord(e->ev[2], st));
-    if (use_diag) TOS_TRY(sweep(true, ctr + 11));
+    if (use_diag) TOS_TRY(sweep(kSweepDiag, ctr + 11));
     TOS_CUDA_TRY(cudaEventRecord(e->ev[7], st));
-    if (use_grid) TOS_TRY(sweep(false, ctr + 10));
+    if (use_grid) TOS_TRY(sweep(kSweepGrid, ctr + 10));
+    if (use_short) TOS_TRY(sweep(kSweepShort, ctr + 15));
     TOS_CUDA_TRY(cudaEventRecord(e->ev[6], st));
     if (A.gap_split) {
       PairArgs R = A;

@@ -252,6 +252,7 @@ struct tos_catalog {
   bool grid_built[2] = {false, false};
   int grid_n[2] = {0, 0};                              // distinct values (0: no usable grid)
   uint64_t grid_los[2] = {0, 0};                       // sightlines contiguous on the grid
+  uint64_t grid_short[2] = {0, 0};                     // those of at most kShortPixels pixels
   tos::DevBuf<float> d_grid[2];                        // sorted distinct values
   tos::DevBuf<float> d_gl[2];                          // loglam of each value
   tos::DevBuf<double> d_glp[2];                        // exclusive prefix sums of loglam - lmid

@@ -130,7 +130,7 @@ __device__ __forceinline__ bool diag_item(const PairArgs& A, double zlo, double 
 // The kernel that takes item idx, from the predicates above as each kernel
 // applies them (load_item for the sweeps, the pixel-pair kernel's own test): one lane per item, so that a kernel can claim a batch
 // of items and skip the others' without loading each one warp-wide.
-enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerPair };
+enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerShort, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerPair };
 __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long idx) {
   const uint32_t i = A.item_i[idx], j = A.item_j[idx];
   if (A.npix[i] == 0 || A.npix[j] == 0) return kOwnerNone;
@@ -142,7 +142,8 @@ __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long 
   const bool zconst = zlo > -1.0 && zhi < 2147483648.0 && zb_lo == zb_hi;
   if (A.run_split && run_item(A, A.item_c[idx], zconst)) {
     if ((A.grid_split || A.gap_split) && A.gfirst[i] != kNoGrid && A.gfirst[j] != kNoGrid) {
-      if (A.grid_split && A.gspan[i] == A.npix[i] && A.gspan[j] == A.npix[j]) return kOwnerGrid;
+      if (A.grid_split && A.gspan[i] == A.npix[i] && A.gspan[j] == A.npix[j])
+        return max(A.npix[i], A.npix[j]) <= kShortPixels ? kOwnerShort : kOwnerGrid;
       if (A.gap_split) return kOwnerGaps;
     }
     return kOwnerRun;
@@ -164,20 +165,25 @@ struct Claim {
 };
 
 // The next item of kernel `owner` (one warp; false: none left).  A claim takes
-// one item, so that long items spread over the CTAs; after one of another
-// kernel it takes 2, 4, ... up to kClaimItems, until it holds one of its own: a
+// one item, so that long items spread over the CTAs (`size` items, up to
+// kClaimItems, where they are short); after those of another kernel it takes
+// twice as many, up to kClaimItems, until it holds one of its own: a
 // sweep that owns few of the items goes through the others 32 at a time.  (8.0e6
 // items of 4,000 contiguous sightlines, one of them masked: the gap sweep scanned
 // them in 52 ms one by one, now in 2.)
-__device__ __forceinline__ bool claim_item(const PairArgs& A, int owner, Claim& C, int lane, unsigned long long& idx) {
+__device__ __forceinline__ bool claim_item(const PairArgs& A, int owner, Claim& C, int lane, unsigned long long& idx,
+                                           int size = 1) {
   unsigned todo = C.todo;
   if (todo == 0u) {
     idx = 0;
-    if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
-    idx = __shfl_sync(kFull, idx, 0);
-    if (idx >= A.n_items) return false;
-    if (item_owner(A, idx) == owner) return true;
-    for (int size = 2; todo == 0u; size = min(2 * size, kClaimItems)) {
+    if (size == 1) {
+      if (lane == 0) idx = atomicAdd(A.next_item, 1ull);
+      idx = __shfl_sync(kFull, idx, 0);
+      if (idx >= A.n_items) return false;
+      if (item_owner(A, idx) == owner) return true;
+      size = 2;
+    }
+    for (; todo == 0u; size = min(2 * size, kClaimItems)) {
       if (lane == 0) idx = atomicAdd(A.next_item, (unsigned long long)size);
       idx = __shfl_sync(kFull, idx, 0);
       if (idx >= A.n_items) return false;

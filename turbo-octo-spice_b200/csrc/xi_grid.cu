@@ -67,8 +67,25 @@ namespace {
 
 // Warps per CTA; a CTA has two items in flight.  Sightlines with gaps take twice
 // the shared memory an item, so twice the warps share a CTA's items there.
-template <bool GAPS>
-constexpr int kGridWarps = GAPS ? 8 : 4;
+// Short items (kShortPixels) are bound by the chain of reads that prepares
+// them, so each has one warp to itself, 16 CTAs an SM, and a claim takes up to
+// 16 of them (neighbouring items add to the same bins: from one warp these adds
+// do not meet).  Measured against four warps an item and the sweep before the
+// band sweep, which had a warp an item (ms):
+//                                               before   four   one
+//   328,000 Cartesian items of 16 pixels          1.60   2.68   1.35
+//   of 40                                         3.13   3.11   1.63
+//   of 128                                       13.0    5.94   4.37
+//   of 4 (the chain is longer than it was)        0.83   2.27   1.07
+//   719,000 observing items of 16                 3.56   5.11   1.82
+//   of 40                                         6.39   7.23   2.85
+//   of 128                                       16.8   17.6    6.71
+// With room for sightlines of 300 pixels fewer CTAs fit (16 pixels 2.3 ms, 128
+// pixels 6.5): the limit is the longest for which 16 do.
+enum Layout { kWhole, kShort, kGaps };
+template <int L>
+constexpr int kGridWarps = L == kGaps ? 8 : L == kShort ? 1 : 4;
+constexpr int kShortClaim = 16;
 constexpr int kBandsPerWarp = 31;  // 32 boundaries
 
 // Sums of a stretch of rows: w d w d, w d, w d, w w, w, w (didj, di, dj, wgt,
@@ -479,8 +496,9 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
 
 // Prepare the next owned item into `h` (all lanes of one warp; SMEM: its data
 // into buf, arriving on `full`).
-template <int COORD, bool SMEM, bool GAPS>
+template <int COORD, bool SMEM, int L>
 __device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, unsigned long long* full, int lane) {
+  constexpr bool GAPS = L == kGaps;
   const PairArgs& A = s_args;
   int taken = 0;
   const int nb = 2 * (int)A.g.n0 + 1;
@@ -488,7 +506,8 @@ __device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, u
   it.bands = 0;
   for (;;) {
     unsigned long long idx = 0;
-    if (!claim_item(A, GAPS ? kOwnerGaps : kOwnerGrid, s_claim, lane, idx)) break;
+    if (!claim_item(A, GAPS ? kOwnerGaps : L == kShort ? kOwnerShort : kOwnerGrid, s_claim, lane, idx,
+                    L == kShort ? A.short_claim : 1)) break;
     ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
     it.ni = (int)A.gspan[i];
@@ -568,17 +587,18 @@ __device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, u
 
 // The arguments stay in the kernel's parameter space (__grid_constant__):
 // the inlined sweep reads them as constant-bank operands.
-template <int COORD, bool MINPOS, bool SMEM, bool GAPS>
-__global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kernel(const __grid_constant__ PairArgs A) {
+template <int COORD, bool MINPOS, bool SMEM, int L>
+__global__ void __launch_bounds__(kGridWarps<L> * 32, L == kGaps ? 2 : 16 / kGridWarps<L>) grid_kernel(const __grid_constant__ PairArgs A) {
+  constexpr bool GAPS = L == kGaps;
   extern __shared__ double2 band_smem[];
   __shared__ int s_next[2];  // GAPS: next group of each item
   __shared__ unsigned long long s_full[2], s_empty[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int len = A.max_span + 1, buf_len = (GAPS ? 4 : 2) * len;
   const float* U = A.gU;
-  if (SMEM) {
+  if (SMEM && L != kShort) {
     float* u = reinterpret_cast<float*>(band_smem + 2 * (size_t)buf_len);
-    for (int g = tid; g < A.ng; g += kGridWarps<GAPS> * 32) u[g] = A.gU[g];
+    for (int g = tid; g < A.ng; g += kGridWarps<L> * 32) u[g] = A.gU[g];
     U = u;
   }
   if (tid == 0) {
@@ -586,7 +606,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
     s_claim.todo = 0u;
     for (int b = 0; b < 2; ++b) {
       bar_init(&s_full[b], 1);
-      bar_init(&s_empty[b], kGridWarps<GAPS>);
+      bar_init(&s_empty[b], kGridWarps<L>);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -595,7 +615,7 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
   unsigned long long n_taken = 0;
   bool ok = true;
   if (warp == 0)
-    n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[0], &s_next[0], band_smem, &s_full[0], lane);
+    n_taken += prepare_item<COORD, SMEM, L>(&s_item[0], &s_next[0], band_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u, parity = (k >> 1) & 1u;
     ok = bar_wait(&s_full[b], parity);
@@ -610,17 +630,17 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
     }
     // groups go round the warps from item to item, and the warp with the last
     // one, often none, prepares the next item (2,000 sightlines: 29.8 ms with a
-    // fixed producer, 28.3; 328,000 pairs of 16-pixel sightlines: 4.9 ms, 2.7)
-    const int q0 = (warp - (int)k) & (kGridWarps<GAPS> - 1);
-    if (q0 == kGridWarps<GAPS> - 1) {
+    // fixed producer, 28.3; one warp alone is always that one)
+    const int q0 = (warp - (int)k) & (kGridWarps<L> - 1);
+    if (q0 == kGridWarps<L> - 1) {
       const uint32_t nb = b ^ 1u;
       // item k - 1 (the other buffer's) is done by every warp
       if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
       if (!ok) break;
-      n_taken += prepare_item<COORD, SMEM, GAPS>(&s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
+      n_taken += prepare_item<COORD, SMEM, L>(&s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
                                                  &s_full[nb], lane);
     }
-    for (int q = q0;; q += kGridWarps<GAPS>) {
+    for (int q = q0;; q += kGridWarps<L>) {
       if (GAPS) {  // more warps than an item has groups: from a counter
         if (lane == 0) q = atomicAdd(&s_next[b], 1);
         q = __shfl_sync(kFull, q, 0);
@@ -635,19 +655,20 @@ __global__ void __launch_bounds__(kGridWarps<GAPS> * 32, GAPS ? 2 : 4) grid_kern
   add_counters(A, lane, stats[0], stats[1], n_taken, GAPS ? 8 : 9);
 }
 
-// Two items and the grid's values.
-template <bool GAPS>
+// Two items and (but for short ones, which read few of them) the grid's values.
+template <int L>
 size_t band_smem_bytes(const PairArgs& a) {
-  return 2 * (size_t)(GAPS ? 4 : 2) * (a.max_span + 1) * sizeof(double2) + (size_t)a.ng * sizeof(float);
+  return 2 * (size_t)(L == kGaps ? 4 : 2) * (a.max_span + 1) * sizeof(double2) +
+         (L == kShort ? 0 : (size_t)a.ng * sizeof(float));
 }
 
 // Persistent launch: `ctas_per_sm` CTAs per SM (0 or above the occupancy
 // limit: as many as fit), or with `max_out` set only that limit.
-template <int COORD, bool MINPOS, bool SMEM, bool GAPS>
+template <int COORD, bool MINPOS, bool SMEM, int L>
 cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  constexpr int threads = kGridWarps<GAPS> * 32;
-  const size_t smem = SMEM ? band_smem_bytes<GAPS>(a) : 0;
-  auto kern = grid_kernel<COORD, MINPOS, SMEM, GAPS>;
+  constexpr int threads = kGridWarps<L> * 32;
+  const size_t smem = SMEM ? band_smem_bytes<L>(a) : 0;
+  auto kern = grid_kernel<COORD, MINPOS, SMEM, L>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -659,7 +680,11 @@ cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
     return cudaSuccess;
   }
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-  kern<<<num_sms * per_sm, threads, smem, stream>>>(a);
+  PairArgs b = a;
+  // (as many as leave each CTA several claims)
+  b.short_claim = (int)std::min<unsigned long long>(
+      kShortClaim, std::max<unsigned long long>(1, a.n_items / (4ull * num_sms * per_sm)));
+  kern<<<num_sms * per_sm, threads, smem, stream>>>(b);
   return cudaGetLastError();
 }
 
@@ -668,31 +693,40 @@ cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
 // values take 47 KB (87 KB with gaps).
 constexpr size_t kBandSmem = 224 * 1024;
 
-template <int COORD, bool MINPOS, bool GAPS>
+static_assert(2 * 2 * (kShortPixels + 1) * sizeof(double2) <= kBandSmem / 16, "short items: 16 CTAs an SM");
+
+template <int COORD, bool MINPOS, int L>
 cudaError_t launch_grid2(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStream_t stream, int* max_out) {
-  return band_smem_bytes<GAPS>(a) <= kBandSmem
-             ? launch_grid<COORD, MINPOS, true, GAPS>(a, num_sms, ctas_per_sm, stream, max_out)
-             : launch_grid<COORD, MINPOS, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
+  if constexpr (L == kShort)
+    return launch_grid<COORD, MINPOS, true, L>(a, num_sms, ctas_per_sm, stream, max_out);
+  else
+    return band_smem_bytes<L>(a) <= kBandSmem
+               ? launch_grid<COORD, MINPOS, true, L>(a, num_sms, ctas_per_sm, stream, max_out)
+               : launch_grid<COORD, MINPOS, false, L>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
-template <bool GAPS>
+template <int L>
 cudaError_t launch_grid3(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm, cudaStream_t stream,
                          int* max_out) {
   if (coord == TOS_CARTESIAN)
-    return minpos ? launch_grid2<kCart, true, GAPS>(a, num_sms, ctas_per_sm, stream, max_out)
-                  : launch_grid2<kCart, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
-  return launch_grid2<kObs, false, GAPS>(a, num_sms, ctas_per_sm, stream, max_out);
+    return minpos ? launch_grid2<kCart, true, L>(a, num_sms, ctas_per_sm, stream, max_out)
+                  : launch_grid2<kCart, false, L>(a, num_sms, ctas_per_sm, stream, max_out);
+  return launch_grid2<kObs, false, L>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
 }  // namespace
 
 cudaError_t launch_grid_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm,
                                cudaStream_t stream, int* max_out) {
-  return launch_grid3<false>(a, coord, minpos, num_sms, ctas_per_sm, stream, max_out);
+  return launch_grid3<kWhole>(a, coord, minpos, num_sms, ctas_per_sm, stream, max_out);
+}
+
+cudaError_t launch_short_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream) {
+  return launch_grid3<kShort>(a, coord, minpos, num_sms, 0, stream, nullptr);
 }
 
 cudaError_t launch_gap_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream) {
-  return launch_grid3<true>(a, coord, minpos, num_sms, 0, stream, nullptr);
+  return launch_grid3<kGaps>(a, coord, minpos, num_sms, 0, stream, nullptr);
 }
 
 }  // namespace tos

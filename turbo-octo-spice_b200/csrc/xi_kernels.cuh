@@ -34,6 +34,9 @@ namespace tos {
 
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
 constexpr uint32_t kNoGrid = 0xFFFFFFFFu;  // sightline not on the common grid
+// Pairs of contiguous sightlines of at most this many pixels: the band sweep's
+// layout for short items (xi_grid.cu).
+constexpr uint32_t kShortPixels = 128;
 constexpr int kPairWarps = 16;  // warps per CTA of the pair kernel
 // u32 words per window slot: the three signed sums (didj, di, dj) as 22+22+rest
 // bit words of a 62-bit fixed-point value, the four positive sums (wgt, wi,
@@ -153,6 +156,7 @@ struct PairArgs {
   float lev_scale, lev_off;
   int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
   int max_np;                // longest sightline
+  int short_claim;           // items a claim of the short layout takes
   int grid_split;            // the grid kernel takes the run items whose sightlines are contiguous on the grid
   int gap_split;             // its variant for gaps takes the other run items whose sightlines are on the grid
   int diag_split;            // Polar: the diagonal-sweep kernel takes the items whose z index is
@@ -186,11 +190,15 @@ cudaError_t launch_pair_kernel(const PairArgs& a, int coord, bool exact0, bool m
 size_t pair_kernel_smem(int win_slots);
 
 // Launch the persistent grid-sweep kernel (xi_grid.cu) over the items that
-// run_item() accepts and whose two sightlines are contiguous on the common grid.
+// run_item() accepts and whose two sightlines are contiguous on the common grid
+// (item_owner: kOwnerGrid).
 // ctas_per_sm: CTAs per SM (0: as many as fit); with max_out set, only
 // report that limit.
 cudaError_t launch_grid_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, int ctas_per_sm,
                                cudaStream_t stream, int* max_out = nullptr);
+
+// The same for the items of two short sightlines (item_owner: kOwnerShort).
+cudaError_t launch_short_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream);
 
 // The same for the items with gapped sightlines (item_owner: kOwnerGaps).
 cudaError_t launch_gap_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream);
