@@ -142,6 +142,11 @@ int tos_abi_version(void);
 tos_status tos_engine_create(int device, tos_engine** out);
 void tos_engine_destroy(tos_engine* engine);
 
+/* The longest a kernel of this engine's calls waits on a barrier for a copy or
+ * another warp before it gives up and the call returns TOS_ERR_TIMEOUT (the
+ * engine stays usable).  Default 10 s; 0: no wait at all. */
+tos_status tos_engine_set_wait_limit(tos_engine* engine, double seconds);
+
 /* ---- catalogue (sightlines + pixels resident on the device) --------------- */
 
 /* Upload sightlines and pixels, and bin sightlines into HEALPix RING cells of

@@ -1092,6 +1092,13 @@ tos_status tos_engine_create(int device, tos_engine** out) {
   return TOS_OK;
 }
 
+tos_status tos_engine_set_wait_limit(tos_engine* e, double seconds) {
+  if (!e || !(seconds >= 0 && seconds <= 3600)) return fail(TOS_ERR_INVALID_ARG, "need an engine and 0 <= seconds <= 3600");
+  std::lock_guard<std::mutex> lock(e->mu);
+  e->wait_ms = (uint32_t)std::ceil(seconds * 1e3);
+  return TOS_OK;
+}
+
 void tos_engine_destroy(tos_engine* e) {
   if (!e) return;
   {
@@ -1799,6 +1806,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   A.item_sep = ws->d_item_sep.p;
   A.n_items = n_items;
   A.next_item = ctr + 4;
+  A.wait_ms = e->wait_ms;
   A.g = rg;
   A.acc = ws->d_acc.p;
   A.counters = ctr;
@@ -2194,7 +2202,10 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   if (n_rows) TOS_TRY(copy_out(e, out_cells, ws->d_out.p + nb, n_rows * nb * sizeof(tos_xibin)));
   TOS_CUDA_TRY(cudaEventRecord(e->ev[4], st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  if (hc[13]) return fail(TOS_ERR_TIMEOUT, "a wait of the grid sweep ran out");
+  if (hc[13])
+    return fail(TOS_ERR_TIMEOUT, std::string("a wait of the ") +
+                                     (hc[13] & kWaitDiag ? "Polar" : hc[13] & kWaitGaps ? "gap" : "band") +
+                                     " sweep ran out");
   ws->last_valid = (plan == nullptr);  // slot rows are not per-cell sums
   ws->last_nb = nb;
   for (int k = 0; k < 7; ++k) ws->last_inv_scale[k] = 1.0 / A.scale[k];

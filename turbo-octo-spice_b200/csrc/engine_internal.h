@@ -188,6 +188,8 @@ struct tos_engine {
   // (kernel variant, warps per CTA)
   std::mutex tune_mu;
   std::map<int, std::pair<int, int>> brute_tuned;
+  // the longest a kernel waits on a barrier (tos_engine_set_wait_limit; under mu)
+  uint32_t wait_ms = 10000;
   tos::BruteScratch brute;
   tos::HostStage stage;
   // CTAs per SM of the dominant pair-count kernel picked by TOS_XI_TUNE, by

@@ -637,8 +637,13 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
   if (warp == 0) n_taken += prepare_diag<SMEM>(&s_item[0], &s_next[0], diag_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u;
-    ok = bar_wait(&s_full[b], (k >> 1) & 1u);
-    if (!ok) break;
+    ok = bar_wait(&s_full[b], (k >> 1) & 1u, A.wait_ms);
+    if (!ok) {
+      // the copies that this warp started must land before it ends
+      if (k == 0 ? warp == 0 : ((warp - (int)(k - 1)) & (kDiagWarps - 1)) == 0)
+        bar_wait(&s_full[b], (k >> 1) & 1u, kWaitMs);
+      break;
+    }
     DItem it = s_item[b];
     if (it.groups == 0) break;
     if (SMEM) {  // the same pointers, known to be in shared memory
@@ -647,7 +652,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
     }
     if (((warp - (int)k) & (kDiagWarps - 1)) == 0) {  // the warps take turns
       const uint32_t nb = b ^ 1u;
-      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);  // item k - 1 is done by every warp
+      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u, A.wait_ms);  // item k - 1 is done by every warp
       if (!ok) break;
       n_taken += prepare_diag<SMEM>(&s_item[nb], &s_next[nb], diag_smem + (SMEM ? (size_t)nb * buf_len : 0),
                                     &s_full[nb], lane);
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
     __syncwarp();
     if (lane == 0) bar_arrive(&s_empty[b]);
   }
-  if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
+  if (!ok && lane == 0) atomicOr(&A.counters[13], kWaitDiag);  // a wait ran out: the host reports it
   __syncwarp();
   add_counters_diag(A, lane, n_eval, lane == 0 ? Q.rech : 0ull, n_taken);
 }

@@ -618,8 +618,13 @@ __global__ void __launch_bounds__(kGridWarps<L> * 32, L == kGaps ? 2 : 16 / kGri
     n_taken += prepare_item<COORD, SMEM, L>(&s_item[0], &s_next[0], band_smem, &s_full[0], lane);
   for (uint32_t k = 0;; ++k) {
     const uint32_t b = k & 1u, parity = (k >> 1) & 1u;
-    ok = bar_wait(&s_full[b], parity);
-    if (!ok) break;
+    ok = bar_wait(&s_full[b], parity, A.wait_ms);
+    if (!ok) {
+      // the copies that this warp started must land before it ends
+      if (k == 0 ? warp == 0 : ((warp - (int)(k - 1)) & (kGridWarps<L> - 1)) == kGridWarps<L> - 1)
+        bar_wait(&s_full[b], parity, kWaitMs);
+      break;
+    }
     BandItem it = s_item[b];
     if (it.bands == 0) break;
     if (SMEM) {  // the same pointers, known to be in shared memory
@@ -635,7 +640,7 @@ __global__ void __launch_bounds__(kGridWarps<L> * 32, L == kGaps ? 2 : 16 / kGri
     if (q0 == kGridWarps<L> - 1) {
       const uint32_t nb = b ^ 1u;
       // item k - 1 (the other buffer's) is done by every warp
-      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u);
+      if (k > 0) ok = bar_wait(&s_empty[nb], ((k - 1) >> 1) & 1u, A.wait_ms);
       if (!ok) break;
       n_taken += prepare_item<COORD, SMEM, L>(&s_item[nb], &s_next[nb], band_smem + (SMEM ? (size_t)nb * buf_len : 0),
                                                  &s_full[nb], lane);
@@ -651,7 +656,7 @@ __global__ void __launch_bounds__(kGridWarps<L> * 32, L == kGaps ? 2 : 16 / kGri
     __syncwarp();
     if (lane == 0) bar_arrive(&s_empty[b]);
   }
-  if (!ok && lane == 0) atomicExch(&A.counters[13], 1ull);  // a wait ran out: the host reports it
+  if (!ok && lane == 0) atomicOr(&A.counters[13], GAPS ? kWaitGaps : kWaitGrid);  // a wait ran out: the host reports it
   add_counters(A, lane, stats[0], stats[1], n_taken, GAPS ? 8 : 9);
 }
 

@@ -37,6 +37,8 @@ constexpr uint32_t kNoGrid = 0xFFFFFFFFu;  // sightline not on the common grid
 // Pairs of contiguous sightlines of at most this many pixels: the band sweep's
 // layout for short items (xi_grid.cu).
 constexpr uint32_t kShortPixels = 128;
+// Bits of counters[13]: a wait of that sweep ran out.
+constexpr unsigned long long kWaitGrid = 1, kWaitGaps = 2, kWaitDiag = 4;
 constexpr int kPairWarps = 16;  // warps per CTA of the pair kernel
 // u32 words per window slot: the three signed sums (didj, di, dj) as 22+22+rest
 // bit words of a 62-bit fixed-point value, the four positive sums (wgt, wi,
@@ -156,6 +158,7 @@ struct PairArgs {
   float lev_scale, lev_off;
   int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
   int max_np;                // longest sightline
+  uint32_t wait_ms;          // the longest a sweep waits for a copy or another warp
   int short_claim;           // items a claim of the short layout takes
   int grid_split;            // the grid kernel takes the run items whose sightlines are contiguous on the grid
   int gap_split;             // its variant for gaps takes the other run items whose sightlines are on the grid

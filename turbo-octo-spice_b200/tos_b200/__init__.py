@@ -95,6 +95,7 @@ def lib() -> C.CDLL:
         L.tos_last_error.restype = C.c_char_p
         L.tos_abi_version.restype = C.c_int
         L.tos_engine_create.argtypes = [i32, C.POINTER(vp)]
+        L.tos_engine_set_wait_limit.argtypes = [vp, dbl]
         L.tos_engine_destroy.argtypes = [vp]
         L.tos_engine_destroy.restype = None
         L.tos_catalog_create.argtypes = [vp, vp, sz, vp, sz, i32, C.POINTER(vp)]
@@ -229,6 +230,10 @@ class Engine:
     @property
     def handle(self):
         return self._h
+
+    def set_wait_limit(self, seconds: float):
+        """The longest a kernel waits on a barrier (default 10 s)."""
+        _check(lib().tos_engine_set_wait_limit(self._h, seconds))
 
     def close(self):
         if getattr(self, "_h", None):
