@@ -373,6 +373,9 @@ tos_status tos_server_create(int device, int slots, uint64_t memory_budget_bytes
 void tos_server_destroy(tos_server* server);
 /* Count a resident catalogue (created on the server's device with
  * tos_catalog_create) against the budget; TOS_ERR_OOM when it does not fit.
+ * What sightlines with gaps take in addition, laid out on the catalogue's common
+ * grid, is left out when it does not fit (their counts then take longer; until
+ * the catalogue is detached).
  * The catalogue must outlive its requests; detach it before destroying it. */
 tos_status tos_server_attach(tos_server* server, tos_catalog* catalog);
 tos_status tos_server_detach(tos_server* server, tos_catalog* catalog);

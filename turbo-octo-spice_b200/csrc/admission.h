@@ -71,8 +71,9 @@ class Admission {
 
   // Resident catalogue bytes: add (false when they do not fit beside the
   // slots' current workspaces) or remove.
+  bool has_room(uint64_t bytes) const { return in_use() + bytes <= budget_; }
   bool add_resident(uint64_t bytes) {
-    if (in_use() + bytes > budget_) return false;
+    if (!has_room(bytes)) return false;
     resident_ += bytes;
     return true;
   }

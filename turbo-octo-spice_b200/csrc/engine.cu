@@ -903,9 +903,13 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
     TOS_CUDA_TRY(cudaMemcpy(&last, uniq.p + ng - 1, sizeof(float), cudaMemcpyDeviceToHost));
     if (last == kSentinel) --ng;
   }
-  cat->grid_built[w] = true;
+  tmp.release();
+  sorted.release();
   cat->grid_n[w] = 0;
-  if (ng <= 0 || ng > 65535) return TOS_OK;
+  if (ng <= 0 || ng > 65535) {
+    cat->grid_built[w] = true;
+    return TOS_OK;
+  }
   TOS_TRY(cat->d_grid[w].alloc(ng));
   TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_grid[w].p, uniq.p, ng * sizeof(float), cudaMemcpyDeviceToDevice, st));
   TOS_TRY(cat->d_gfirst[w].alloc(cat->n_los));
@@ -920,7 +924,10 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   unsigned long long h[4] = {0, 0, 0, 0};
   TOS_CUDA_TRY(cudaMemcpyAsync(h, nok.p, 32, cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h[0] + h[1] == 0) return TOS_OK;
+  if (h[0] + h[1] == 0) {
+    cat->grid_built[w] = true;
+    return TOS_OK;
+  }
   // for contiguous sightlines the grid sweep takes a pixel's loglam from its
   // grid value: not usable when two pixels of one value differ in it
   TOS_TRY(cat->d_gl[w].alloc(ng));
@@ -939,34 +946,12 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   cat->grid_geo[w] = bad == 0;
   cat->grid_lmid[w] = (double)lmid;
-  if (h[1] || bad) {  // sightlines laid out on the grid
+  if (h[1] || bad) {  // these are laid out on the grid (ensure_layout)
     std::vector<uint32_t> span(cat->n_los);
     TOS_CUDA_TRY(cudaMemcpy(span.data(), cat->d_gspan[w].p, span.size() * 4, cudaMemcpyDeviceToHost));
-    std::vector<uint64_t> go(cat->n_los);
     uint64_t tot = 0;
-    for (size_t s = 0; s < cat->n_los; ++s) {
-      go[s] = tot;
-      tot += (uint64_t)span[s] + 1;
-    }
-    // 64 bytes an entry: beyond 8 GiB of them the pointer sweep keeps the items
-    if (tot <= (8ull << 30) / 64) {
-      TOS_TRY(cat->d_gap_off[w].alloc(go.size()));
-      TOS_TRY(cat->d_gap_pre[w].alloc(tot));
-      TOS_TRY(cat->d_gap_cnt[w].alloc(tot));
-      TOS_TRY(cat->d_gap_row[w].alloc(tot));
-      TOS_TRY(cat->d_gap_one[w].alloc(tot));
-      TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_gap_off[w].p, go.data(), go.size() * 8, cudaMemcpyHostToDevice, st));
-      TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gap_row[w].p, 0, tot * sizeof(double2), st));
-      TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gap_one[w].p, 0, tot * sizeof(double2), st));
-      k_gap_rows<<<gw, 256, 0, st>>>(x, cat->d_loglam_pad.p, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_wd.p,
-                                     cat->d_w.p, cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->grid_lmid[w],
-                                     cat->d_gap_off[w].p, cat->d_gap_row[w].p, cat->d_gap_one[w].p);
-      k_gap_prefix<<<gw, 256, 0, st>>>(cat->n_los, cat->d_off.p, cat->d_pre2.p, cat->d_gspan[w].p,
-                                       cat->d_gap_off[w].p, cat->d_gap_one[w].p, cat->d_gap_pre[w].p,
-                                       cat->d_gap_cnt[w].p);
-      TOS_CUDA_TRY(cudaGetLastError());
-      TOS_CUDA_TRY(cudaStreamSynchronize(st));  // `go` is read until here
-    }
+    for (uint32_t v : span) tot += (uint64_t)v + 1;
+    cat->gaps[w].entries = tot;
   }
   k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, ng, (double)lmid, cat->d_glp[w].p);
   TOS_CUDA_TRY(cudaGetLastError());
@@ -979,7 +964,58 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
   cat->grid_los[w] = h[0];
   cat->grid_short[w] = h[3];
   cat->grid_gaps[w] = h[1];
+  cat->grid_built[w] = true;
   return TOS_OK;
+}
+
+// Bytes that ensure_layout would add (0: none needed, or there already).  Beyond
+// 8 GiB the pointer sweep keeps the sightlines.
+uint64_t layout_bytes(const tos_catalog* cat, int w) {
+  const GapLayout& L = cat->gaps[w];
+  if (L.entries == 0 || L.entries > (8ull << 30) / 64 || L.mem.p) return 0;
+  GapLayout size;
+  size.entries = L.entries;
+  return size.place(cat->n_los, nullptr);
+}
+
+// Lay the on-grid sightlines out on the grid (after ensure_grid) where some need
+// it.  Without the memory for it there is no layout, and that is no error.
+tos_status ensure_layout(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(cat->grid_mu);
+  const uint64_t bytes = cat->no_layout ? 0 : layout_bytes(cat, w);
+  if (bytes == 0) return TOS_OK;
+  GapLayout& L = cat->gaps[w];
+  if (L.mem.alloc(bytes) != TOS_OK) {
+    cudaGetLastError();
+    return TOS_OK;
+  }
+  L.place(cat->n_los, L.mem.p);
+  const int ng = cat->grid_n[w], gw = grid_for(e, cat->n_los * 32, 256);
+  std::vector<uint32_t> span(cat->n_los);
+  std::vector<uint64_t> go(cat->n_los);
+  auto build = [&]() -> tos_status {
+    TOS_CUDA_TRY(cudaMemcpyAsync(span.data(), cat->d_gspan[w].p, span.size() * 4, cudaMemcpyDeviceToHost, st));
+    TOS_CUDA_TRY(cudaStreamSynchronize(st));
+    uint64_t tot = 0;
+    for (size_t s = 0; s < cat->n_los; ++s) {
+      go[s] = tot;
+      tot += (uint64_t)span[s] + 1;
+    }
+    TOS_CUDA_TRY(cudaMemcpyAsync(L.off, go.data(), go.size() * 8, cudaMemcpyHostToDevice, st));
+    TOS_CUDA_TRY(cudaMemsetAsync(L.row, 0, tot * sizeof(double2), st));
+    TOS_CUDA_TRY(cudaMemsetAsync(L.one, 0, tot * sizeof(double2), st));
+    k_gap_rows<<<gw, 256, 0, st>>>((w == 0) ? cat->d_dist_pad.p : cat->d_loglam_pad.p, cat->d_loglam_pad.p,
+                                   cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_wd.p, cat->d_w.p,
+                                   cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->grid_lmid[w], L.off, L.row, L.one);
+    k_gap_prefix<<<gw, 256, 0, st>>>(cat->n_los, cat->d_off.p, cat->d_pre2.p, cat->d_gspan[w].p, L.off, L.one, L.pre,
+                                     L.cnt);
+    TOS_CUDA_TRY(cudaGetLastError());
+    TOS_CUDA_TRY(cudaStreamSynchronize(st));  // `go` is read until here
+    return TOS_OK;
+  };
+  const tos_status s = build();
+  if (s != TOS_OK) L.mem.release();
+  return s;
 }
 
 // Smallest and largest loglam of the pixels as ordered float bits
@@ -1503,8 +1539,7 @@ uint64_t catalog_data_bytes(const tos_catalog* c) {
                c->d_prefix.bytes() + c->d_pre2.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
   for (int w = 0; w < 2; ++w)
     b += c->d_grid[w].bytes() + c->d_gl[w].bytes() + c->d_glp[w].bytes() + c->d_gfirst[w].bytes() +
-         c->d_gspan[w].bytes() + c->d_gap_off[w].bytes() + c->d_gap_pre[w].bytes() + c->d_gap_cnt[w].bytes() +
-         c->d_gap_row[w].bytes() + c->d_gap_one[w].bytes();
+         c->d_gspan[w].bytes() + c->gaps[w].mem.bytes();
   return b;
 }
 
@@ -1513,8 +1548,7 @@ size_t Workspace::bytes() const {
          d_cand.bytes() +
          d_item_off.bytes() + d_item_i.bytes() + d_item_j.bytes() + d_item_sep.bytes() +
          d_item_c.bytes() + d_cell_pairs.bytes() + d_acc.bytes() + d_out.bytes() +
-         d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_ginv.bytes() + d_gtb.bytes() +
-         d_gskew.bytes() + d_gtabs.bytes() + d_glev.bytes() + d_edges.bytes() + d_pthr.bytes() + d_gtz.bytes() + d_cub_tmp.bytes();
+         d_counters.bytes() + d_thr.bytes() + d_gtab.bytes() + d_pthr.bytes() + d_cub_tmp.bytes();
 }
 
 // Counter words of a run: kernel counters [0, 16), the theta-edge flags of
@@ -1947,48 +1981,46 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     TOS_TRY(ensure_grid(e, cat, w, st));
     const int ng = cat->grid_n[w];
     // the boundary tables take 20 bytes per boundary and grid value; beyond
-    // 2 GiB of them the pointer sweep takes the items
-    const bool tables_fit = (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 20.0 < 2147483648.0;
-    if (ng > 0 && tables_fit) {
-      const size_t nbd = 2 * ((size_t)n0 + 1);
-      const int ngp = (ng + 7) / 4 * 4;
-      TOS_TRY(ws->d_gtab.alloc(nbd * ngp));
-      TOS_TRY(ws->d_ginv.alloc(nbd * (ng + 1)));
-      TOS_TRY(ws->d_gtb.alloc(nbd * (ng + 1)));
-      TOS_TRY(ws->d_gtz.alloc(nbd * (ng + 1)));
-      const bool cart = G.type == TOS_CARTESIAN;
-      // levels of d1 d2: finer than a row (at most 2048)
-      const int nlev = cart ? std::min(2048, std::max(64, 2 * ng)) : 0;
+    // 2 GiB of them, or without the memory, the pointer sweep takes the items
+    bool tables_fit = ng > 0 && (double)(2 * ((size_t)n0 + 1)) * (ng + 8.0) * 20.0 < 2147483648.0;
+    const bool cart = G.type == TOS_CARTESIAN;
+    const size_t nbd = 2 * ((size_t)n0 + 1);
+    const int ngp = (ng + 7) / 4 * 4;
+    const int nlev = cart ? std::min(2048, std::max(64, 2 * ng)) : 0;  // levels of d1 d2: finer than a row
+    const int nblk = ngp / 4 + ng / 4 + 2 * kSkewPad;                  // 4-row blocks of a skewed boundary
+    GridTables T;
+    if (tables_fit) {
+      if (cart) edges = code_edges(rg, A.k1, std::ldexp(cat->max_d * cat->max_d, -24) * rg.inv1 * rg.inv1 * 1.01);
+      const size_t bytes = T.place(nbd, ng, ngp, nblk, cart ? nlev + 1 : 0, edges.size(), nullptr);
+      if (ws->d_gtab.alloc(bytes) != TOS_OK) {
+        cudaGetLastError();
+        tables_fit = false;
+      }
+    }
+    if (tables_fit) {
+      T.place(nbd, ng, ngp, nblk, cart ? nlev + 1 : 0, edges.size(), ws->d_gtab.p);
       const double lev0 = (double)cat->grid_lo[w] * cat->grid_lo[w];
       const double dlev = cart ? std::max((double)cat->grid_hi[w] * cat->grid_hi[w] - lev0, 1e-6 * lev0) / nlev : 1.0;
-      if (cart) {
-        edges = code_edges(rg, A.k1, std::ldexp(cat->max_d * cat->max_d, -24) * rg.inv1 * rg.inv1 * 1.01);
-        TOS_TRY(ws->d_edges.alloc(edges.size()));
-        TOS_CUDA_TRY(cudaMemcpyAsync(ws->d_edges.p, edges.data(), edges.size() * sizeof(float4),
-                                     cudaMemcpyHostToDevice, st));
-        TOS_TRY(ws->d_glev.alloc(nbd * (nlev + 1)));
-      }
-      const int nblk = ngp / 4 + ng / 4 + 2 * kSkewPad;  // 4-row blocks of a skewed boundary
-      TOS_TRY(ws->d_gskew.alloc(nbd));
-      TOS_TRY(ws->d_gtabs.alloc((nbd + 31) / 32 * 32 * nblk));
+      if (cart)
+        TOS_CUDA_TRY(cudaMemcpyAsync(T.edges, edges.data(), edges.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
       k_grid_tables<<<(unsigned)nbd, kTableThreads, 0, st>>>(
           cat->d_grid[w].p, cat->d_gl[w].p, cat->d_glp[w].p, cat->grid_lmid[w], ng, ngp, ws->d_thr.p, (int)n0 + 1,
-          G.type == TOS_OBSERVING ? 1 : 0, nblk, ws->d_gtab.p, ws->d_ginv.p, ws->d_gtb.p, ws->d_gtz.p, ws->d_gskew.p,
-          ws->d_gtabs.p, cart ? ws->d_glev.p : nullptr, nlev, lev0, dlev);
+          G.type == TOS_OBSERVING ? 1 : 0, nblk, T.tab, T.inv, T.tb, T.tz, T.skew, T.tabs, cart ? T.lev : nullptr, nlev,
+          lev0, dlev);
       TOS_CUDA_TRY(cudaGetLastError());
-      A.gtab = ws->d_gtab.p;
-      A.ginv = ws->d_ginv.p;
-      A.gtb = ws->d_gtb.p;
-      A.gtz = ws->d_gtz.p;
-      A.gtabs = ws->d_gtabs.p;
-      A.gskew = ws->d_gskew.p;
+      A.gtab = T.tab;
+      A.ginv = T.inv;
+      A.gtb = T.tb;
+      A.gtz = T.tz;
+      A.gtabs = T.tabs;
+      A.gskew = T.skew;
       A.nblk = nblk;
       A.gU = cat->d_grid[w].p;
       A.gl = cat->d_gl[w].p;
       A.glp = cat->d_glp[w].p;
       A.lmid = cat->grid_lmid[w];
-      A.edges = ws->d_edges.p;
-      A.glev = ws->d_glev.p;
+      A.edges = T.edges;
+      A.glev = T.lev;
       A.nlev = nlev;
       A.lev_scale = (float)(1.0 / dlev);
       // a hundredth of a level and 4e-6 of it cover the FP32 rounding of an edge's level
@@ -2004,12 +2036,14 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       A.grid_split = cat->grid_geo[w] && cat->grid_los[w] > 1;
       use_grid = A.grid_split && cat->grid_los[w] > cat->grid_short[w];
       use_short = A.grid_split && cat->grid_short[w] > 1;
-      if (cat->d_gap_off[w].p) {
-        A.gap_off = cat->d_gap_off[w].p;
-        A.gap_pre = cat->d_gap_pre[w].p;
-        A.gap_cnt = cat->d_gap_cnt[w].p;
-        A.gap_row = cat->d_gap_row[w].p;
-        A.gap_one = cat->d_gap_one[w].p;
+      TOS_TRY(ensure_layout(e, cat, w, st));
+      const GapLayout& L = cat->gaps[w];
+      if (L.mem.p) {
+        A.gap_off = L.off;
+        A.gap_pre = L.pre;
+        A.gap_cnt = L.cnt;
+        A.gap_row = L.row;
+        A.gap_one = L.one;
         A.gap_split = 1;
       }
     }

@@ -64,6 +64,19 @@ struct DevBuf {
   size_t bytes() const { return p ? n * sizeof(T) : 0; }
 };
 
+// Cuts one allocation into arrays, each at a 256-byte boundary: with base null
+// it only adds up their size.
+struct Carve {
+  unsigned char* base = nullptr;
+  size_t off = 0;
+  template <class T>
+  T* take(size_t count) {
+    T* p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+    off += (count * sizeof(T) + 255) / 256 * 256;
+    return p;
+  }
+};
+
 // Smallest double x >= 0 with reached(x) (monotone), near the guess g: 0 when
 // reached(0).
 template <class Pred>
@@ -105,6 +118,25 @@ inline double first_double(double g, Pred reached) {
 
 namespace tos {
 
+// A catalogue's sightlines laid out on the common grid (PairArgs::gap_*): an
+// optional form of it that the band sweep for gaps reads; without it the
+// pointer sweep takes those sightlines.
+struct GapLayout {
+  DevBuf<unsigned char> mem;
+  uint64_t* off = nullptr;
+  double2 *pre = nullptr, *cnt = nullptr, *row = nullptr, *one = nullptr;
+  uint64_t entries = 0;  // of each array (0: no sightline needs it)
+  size_t place(size_t n_los, unsigned char* base) {
+    Carve c{base};
+    off = c.take<uint64_t>(n_los);
+    pre = c.take<double2>(entries);
+    cnt = c.take<double2>(entries);
+    row = c.take<double2>(entries);
+    one = c.take<double2>(entries);
+    return c.off;
+  }
+};
+
 // Device scratch of tos_brute_run and tos_brute_tune, kept on the engine
 // between calls (used under its lock) as long as it is small.
 struct BruteScratch {
@@ -126,6 +158,28 @@ struct BruteScratch {
   }
 };
 
+// The band sweep's boundary tables (PairArgs) in one buffer: nbd boundaries,
+// ng grid values, rows of ngp, nblk blocks, nlev levels, n_edges code edges.
+struct GridTables {
+  uint16_t *tab, *inv, *lev;
+  uint32_t *tb, *skew;
+  double* tz;
+  uint2* tabs;
+  float4* edges;
+  size_t place(size_t nbd, size_t ng, size_t ngp, size_t nblk, size_t nlev, size_t n_edges, unsigned char* base) {
+    Carve c{base};
+    tab = c.take<uint16_t>(nbd * ngp);
+    inv = c.take<uint16_t>(nbd * (ng + 1));
+    tb = c.take<uint32_t>(nbd * (ng + 1));
+    tz = c.take<double>(nbd * (ng + 1));
+    skew = c.take<uint32_t>(nbd);
+    tabs = c.take<uint2>((nbd + 31) / 32 * 32 * nblk);
+    lev = c.take<uint16_t>(nbd * nlev);
+    edges = c.take<float4>(n_edges);
+    return c.off;
+  }
+};
+
 // Device scratch of one pair count, kept between runs so that a caller that
 // runs again (a server slot, the catalogue's own runs) allocates only when a
 // run needs more than before.
@@ -142,12 +196,8 @@ struct Workspace {
   DevBuf<tos_xibin> d_out;                        // combined / per row output
   DevBuf<unsigned long long> d_counters;          // misc counters
   DevBuf<float> d_thr;                            // first-axis thresholds of the run sweep
-  DevBuf<uint16_t> d_gtab, d_ginv, d_glev;        // boundary tables of the current call (grid sweep)
-  DevBuf<uint32_t> d_gtb, d_gskew;
-  DevBuf<uint2> d_gtabs;
-  DevBuf<float4> d_edges;
+  DevBuf<unsigned char> d_gtab;                   // boundary tables of the current call (GridTables)
   DevBuf<double> d_pthr;                          // Polar bin thresholds
-  DevBuf<double> d_gtz;
   DevBuf<unsigned char> d_cub_tmp;
   // the last completed per-cell run in d_acc
   bool last_valid = false;
@@ -250,7 +300,7 @@ struct tos_catalog {
   double min_gap = 0;               // smallest positive distance step within a sightline (lower bound)
   uint32_t max_np = 0;
   // common first-axis grids (0: distance, 1: loglam), built on first use
-  mutable std::mutex grid_mu;                                  // guards the grid build
+  mutable std::mutex grid_mu;                          // guards the grids and their layouts
   bool grid_built[2] = {false, false};
   int grid_n[2] = {0, 0};                              // distinct values (0: no usable grid)
   uint64_t grid_los[2] = {0, 0};                       // sightlines contiguous on the grid
@@ -265,10 +315,12 @@ struct tos_catalog {
   uint32_t max_span[2] = {0, 0};
   bool grid_geo[2] = {false, false};                   // loglam is a function of the grid value
   uint64_t grid_gaps[2] = {0, 0};                      // sightlines on the grid with gaps
-  // the sightlines laid out on the grid (PairArgs::gap_*), when some have gaps
-  // or loglam is not a function of the grid value
-  tos::DevBuf<uint64_t> d_gap_off[2];
-  tos::DevBuf<double2> d_gap_pre[2], d_gap_cnt[2], d_gap_row[2], d_gap_one[2];
+  // for sightlines with gaps, or where loglam is not a function of the grid value
+  tos::GapLayout gaps[2];
+  // servers that hold the catalogue; with no_layout one of them had no room for
+  // the layouts, and none is built until all have let go of it (under grid_mu)
+  int servers = 0;
+  bool no_layout = false;
   // the workspace of tos_xi_run on this catalogue; its per-cell sums stay
   // there after the run for the covariance calls
   tos::Workspace run;
@@ -343,3 +395,6 @@ double max_angular_scale(const tos_grid& g, double scale);
 // Build (once) the catalogue's common first-axis grid w (0: distance,
 // 1: loglam) for the grid sweep; thread-safe.
 tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st);
+// The same for its layout for gaps; layout_bytes: what that would add (grid_mu held).
+tos_status ensure_layout(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st);
+uint64_t layout_bytes(const tos_catalog* cat, int w);

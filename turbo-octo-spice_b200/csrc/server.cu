@@ -58,8 +58,6 @@ struct Request {
 
 constexpr double kPi = 3.14159265358979323846;
 
-// Device bytes a run of `cat` on grid g needs in a workspace: the sightline
-// pairs are pairs_estimate's, the rest is exact.
 // Estimated sightline pairs of a run (uniform sky density over the occupied
 // cells, with a 1.5 margin).
 double pairs_estimate(const tos_catalog* cat, const tos_grid& g, double scale) {
@@ -71,6 +69,8 @@ double pairs_estimate(const tos_catalog* cat, const tos_grid& g, double scale) {
   return 1.5 * 0.5 * n * std::min(n, n * disc / area) + n;
 }
 
+// Device bytes a run of `cat` on grid g needs in a workspace: the sightline
+// pairs are pairs_estimate's, the rest is exact.
 uint64_t workspace_estimate(const tos_catalog* cat, const tos_grid& g, double scale, size_t n_rows) {
   const double nb = (double)g.axis[0].nbins * g.axis[1].nbins * g.axis[2].nbins;
   const double nc = (double)cat->cells.size(), n = (double)cat->n_los;
@@ -314,6 +314,21 @@ void tos_server_destroy(tos_server* s) {
   delete s;
 }
 
+// Gives back the layouts that an earlier run built, unless a server or a run
+// may be reading them.
+static bool drop_layouts(tos_catalog* cat, int device) {
+  std::unique_lock<std::mutex> run(cat->run_mu, std::try_to_lock);
+  if (!run.owns_lock()) return false;
+  std::lock_guard<std::mutex> gl(cat->grid_mu);
+  if (cat->servers != 0) return false;
+  int prev = -1;
+  cudaGetDevice(&prev);
+  cudaSetDevice(device);
+  for (GapLayout& L : cat->gaps) L.mem.release();
+  cudaSetDevice(prev);
+  return true;
+}
+
 tos_status tos_server_attach(tos_server* s, tos_catalog* cat) {
   if (!s || !cat) return fail(TOS_ERR_INVALID_ARG, "null argument");
   if (cat->device != s->device) return fail(TOS_ERR_INVALID_ARG, "catalogue is on another device");
@@ -321,7 +336,9 @@ tos_status tos_server_attach(tos_server* s, tos_catalog* cat) {
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->attached.count(cat)) return TOS_OK;
   }
-  // the common-grid tables are built once per catalogue, before any request
+  // the common grids, and the layouts for gaps if the budget has room for them
+  // (without one the pointer sweep takes those sightlines), are built once per
+  // catalogue, before any request
   {
     std::lock_guard<std::mutex> el(s->setup->mu);
     int prev = -1;
@@ -329,14 +346,31 @@ tos_status tos_server_attach(tos_server* s, tos_catalog* cat) {
     cudaSetDevice(s->device);
     tos_status st = TOS_OK;
     for (int w = 0; w < 2 && st == TOS_OK; ++w) st = ensure_grid(s->setup, cat, w, s->setup->stream);
+    uint64_t need = catalog_data_bytes(cat) + cat->run.bytes();
+    {
+      std::lock_guard<std::mutex> gl(cat->grid_mu);
+      need += layout_bytes(cat, 0) + layout_bytes(cat, 1);
+    }
+    bool room;
+    {
+      std::lock_guard<std::mutex> lk(s->mu);
+      room = s->adm.has_room(need);
+    }
+    for (int w = 0; w < 2 && st == TOS_OK && room; ++w) st = ensure_layout(s->setup, cat, w, s->setup->stream);
     cudaSetDevice(prev);
     TOS_TRY(st);
   }
-  const uint64_t bytes = catalog_data_bytes(cat) + cat->run.bytes();
   std::lock_guard<std::mutex> lk(s->mu);
+  uint64_t bytes = catalog_data_bytes(cat) + cat->run.bytes();
+  if (!s->adm.has_room(bytes) && drop_layouts(cat, s->device)) bytes = catalog_data_bytes(cat) + cat->run.bytes();
   if (!s->adm.add_resident(bytes))
     return fail(TOS_ERR_OOM, "catalogue (" + std::to_string(bytes) +
                                  " bytes) does not fit in the server's memory budget");
+  {
+    std::lock_guard<std::mutex> gl(cat->grid_mu);
+    ++cat->servers;
+    if (layout_bytes(cat, 0) + layout_bytes(cat, 1) != 0) cat->no_layout = true;
+  }
   s->attached[cat] = bytes;
   return TOS_OK;
 }
@@ -349,6 +383,10 @@ tos_status tos_server_detach(tos_server* s, tos_catalog* cat) {
   if (s->pending.count(cat)) return fail(TOS_ERR_INVALID_ARG, "catalogue has unfinished requests");
   s->adm.remove_resident(it->second);
   s->attached.erase(it);
+  {
+    std::lock_guard<std::mutex> gl(cat->grid_mu);
+    if (--cat->servers == 0) cat->no_layout = false;
+  }
   s->dispatch();
   return TOS_OK;
 }
