@@ -48,8 +48,8 @@ __global__ void k_fill(float* p, size_t n, float v) {
 // w*delta (exact product of two floats in double), weights; exclusive prefix
 // sums of (w*delta, w, loglam); coordinate ranges; sortedness.
 __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t* npix,
-                       size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pix2, double* wd, float* w,
-                       double4* prefix, double2* pre2, double2* row2, float4* range, unsigned int* flags,
+                       size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pix2,
+                       double2* pre2, double* prel, double2* row2, float4* range, unsigned int* flags,
                        unsigned long long* maxbits) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -58,17 +58,17 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
     const uint64_t o = off[s];
     const uint32_t n = npix[s];
     const uint64_t po = o + (uint64_t)kPad * (s + 1);
-    double4* pre = prefix + o + s;
     double2* p2 = pre2 + o + s;
-    const uint64_t o2 = o + (uint64_t)(3 * kParityPad) * s + kParityPad;  // the first even pixel
+    double* pl = prel + o + s;
+    const uint64_t o2 = o + (uint64_t)(2 * kParityPad) * s + kParityPad;  // the first even pixel
     double c0 = 0, c1 = 0, c2 = 0;
     float dmin = INFINITY, dmax = -INFINITY, lmin = INFINITY, lmax = -INFINITY;
     double mwd = 0, mw = 0, ml = 0, md = 0;
     float gap = INFINITY;  // smallest positive step between consecutive distances
     bool unsorted = false;
     if (lane == 0) {
-      pre[0] = make_double4(0, 0, 0, 0);
       p2[0] = make_double2(0, 0);
+      pl[0] = 0;
     }
     for (uint32_t b = 0; b < n; b += 32) {
       const uint32_t k = b + lane;
@@ -80,8 +80,6 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
         v0 = (double)px.weight * (double)px.value;
         v1 = (double)px.weight;
         v2 = (double)px.loglam;
-        wd[o + k] = v0;
-        w[o + k] = px.weight;
         row2[o + k] = make_double2(v0, v1);
         PixPack q;
         q.d = px.distance;
@@ -117,8 +115,8 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
         }
       }
       if (k < n) {
-        pre[k + 1] = make_double4(c0 + v0, c1 + v1, c2 + v2, 0);
         p2[k + 1] = make_double2(c0 + v0, c1 + v1);
+        pl[k + 1] = c2 + v2;
       }
       c0 += __shfl_sync(kFull, v0, 31);
       c1 += __shfl_sync(kFull, v1, 31);
@@ -674,7 +672,7 @@ __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint3
 // The on-grid sightlines' pixels at their grid entries (the arrays cleared
 // before): (wd, w) and (1, (loglam - lmid) / 2).
 __global__ void k_gap_rows(const float* xpad, const float* lpad, const uint64_t* off, const uint32_t* npix,
-                           size_t n_los, const double* wd, const float* w, const float* U, int ng,
+                           size_t n_los, const double2* row2, const float* U, int ng,
                            const uint32_t* gfirst, double lmid, const uint64_t* gap_off, double2* row, double2* one) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -685,7 +683,7 @@ __global__ void k_gap_rows(const float* xpad, const float* lpad, const uint64_t*
     const uint64_t po = off[s] + (uint64_t)kPad * (s + 1);
     for (uint32_t p = lane; p < npix[s]; p += 32) {
       const uint64_t e = gap_off[s] + (uint32_t)grid_index(U, ng, xpad[po + p]) - f;
-      row[e] = make_double2(wd[off[s] + p], (double)w[off[s] + p]);
+      row[e] = row2[off[s] + p];
       one[e] = make_double2(1.0, 0.5 * ((double)lpad[po + p] - lmid));
     }
   }
@@ -1005,8 +1003,8 @@ tos_status ensure_layout(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st
     TOS_CUDA_TRY(cudaMemsetAsync(L.row, 0, tot * sizeof(double2), st));
     TOS_CUDA_TRY(cudaMemsetAsync(L.one, 0, tot * sizeof(double2), st));
     k_gap_rows<<<gw, 256, 0, st>>>((w == 0) ? cat->d_dist_pad.p : cat->d_loglam_pad.p, cat->d_loglam_pad.p,
-                                   cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_wd.p, cat->d_w.p,
-                                   cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->grid_lmid[w], L.off, L.row, L.one);
+                                   cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_row2.p, cat->d_grid[w].p,
+                                   ng, cat->d_gfirst[w].p, cat->grid_lmid[w], L.off, L.row, L.one);
     k_gap_prefix<<<gw, 256, 0, st>>>(cat->n_los, cat->d_off.p, cat->d_pre2.p, cat->d_gspan[w].p, L.off, L.one, L.pre,
                                      L.cnt);
     TOS_CUDA_TRY(cudaGetLastError());
@@ -1328,11 +1326,10 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   const size_t padded = total + (size_t)kPad * (n_los + 1);
   TOS_TRY(cat->d_dist_pad.alloc(padded));
   TOS_TRY(cat->d_loglam_pad.alloc(padded));
-  TOS_TRY(cat->d_pix2.alloc(total + (size_t)(3 * kParityPad) * n_los));
-  TOS_TRY(cat->d_wd.alloc(total));
-  TOS_TRY(cat->d_w.alloc(total));
-  TOS_TRY(cat->d_prefix.alloc(total + n_los));
+  const size_t parity = total + (size_t)(2 * kParityPad) * n_los + kParityPad;
+  TOS_TRY(cat->d_pix2.alloc(parity));
   TOS_TRY(cat->d_pre2.alloc(total + n_los));
+  TOS_TRY(cat->d_prel.alloc(total + n_los));
   TOS_TRY(cat->d_row2.alloc(total));
   TOS_TRY(cat->d_range.alloc(n_los));
   TOS_TRY(cat->d_flags.alloc(3));
@@ -1384,10 +1381,10 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   if (omega_matter > 0) TOS_TRY(fill_distances_device(e, cat->d_raw.p, total, omega_matter, st));
   k_fill<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_dist_pad.p, padded, kSentinel);
   k_fill<<<grid_for(e, padded, 256), 256, 0, st>>>(cat->d_loglam_pad.p, padded, kSentinel);
-  TOS_CUDA_TRY(cudaMemsetAsync(cat->d_pix2.p, 0, (total + (size_t)(3 * kParityPad) * n_los) * sizeof(PixPack), st));
+  TOS_CUDA_TRY(cudaMemsetAsync(cat->d_pix2.p, 0, parity * sizeof(PixPack), st));
   k_prep<<<grid_for(e, n_los * 32, 256), 256, 0, st>>>(
       cat->d_raw.p, cat->d_off.p, cat->d_npix.p, n_los, cat->d_dist_pad.p, cat->d_loglam_pad.p, cat->d_pix2.p,
-      cat->d_wd.p, cat->d_w.p, cat->d_prefix.p, cat->d_pre2.p, cat->d_row2.p, cat->d_range.p, cat->d_flags.p,
+      cat->d_pre2.p, cat->d_prel.p, cat->d_row2.p, cat->d_range.p, cat->d_flags.p,
       (unsigned long long*)cat->d_maxes.p);
   TOS_CUDA_TRY(cudaGetLastError());
   unsigned int fl[3] = {0u, 0u, 0u};
@@ -1534,9 +1531,9 @@ uint64_t catalog_data_bytes(const tos_catalog* c) {
                c->d_plate_trig.bytes() + c->d_cell_grange.bytes() +
                c->d_group_cell_start.bytes() + c->d_cell_idx.bytes() + c->d_cell_start.bytes() +
                c->d_members.bytes() + c->d_npix.bytes() + c->d_off.bytes() + c->d_raw.bytes() +
-               c->d_dist_pad.bytes() + c->d_loglam_pad.bytes() + c->d_pix2.bytes() + c->d_wd.bytes() +
-               c->d_w.bytes() +
-               c->d_prefix.bytes() + c->d_pre2.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() + c->d_maxes.bytes();
+               c->d_dist_pad.bytes() + c->d_loglam_pad.bytes() + c->d_pix2.bytes() +
+               c->d_pre2.bytes() + c->d_prel.bytes() + c->d_row2.bytes() + c->d_range.bytes() + c->d_flags.bytes() +
+               c->d_maxes.bytes();
   for (int w = 0; w < 2; ++w)
     b += c->d_grid[w].bytes() + c->d_gl[w].bytes() + c->d_glp[w].bytes() + c->d_gfirst[w].bytes() +
          c->d_gspan[w].bytes() + c->gaps[w].mem.bytes();
@@ -1823,9 +1820,9 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   A.loglam_pad = cat->d_loglam_pad.p;
   A.pix2 = cat->d_pix2.p;
   A.max_np = (int)cat->max_np;
-  A.wd = cat->d_wd.p;
-  A.w = cat->d_w.p;
-  A.prefix = cat->d_prefix.p;
+  A.row2 = cat->d_row2.p;
+  A.pre2 = cat->d_pre2.p;
+  A.prel = cat->d_prel.p;
   A.range = cat->d_range.p;
   A.cell_idx = cat->d_cell_idx.p;
   if (plan) {
@@ -2025,8 +2022,6 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       A.lev_scale = (float)(1.0 / dlev);
       // a hundredth of a level and 4e-6 of it cover the FP32 rounding of an edge's level
       A.lev_off = (float)(-lev0 / dlev - 0.01 - 4e-6 * (lev0 / dlev + nlev));
-      A.pre2 = cat->d_pre2.p;
-      A.row2 = cat->d_row2.p;
       A.gfirst = cat->d_gfirst[w].p;
       A.ng = ng;
       A.ngp = ngp;

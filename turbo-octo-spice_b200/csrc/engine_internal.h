@@ -283,11 +283,9 @@ struct tos_catalog {
   tos::DevBuf<tos_pixel> d_raw;     // uploaded pixels, compact order
   tos::DevBuf<float> d_dist_pad, d_loglam_pad;
   tos::DevBuf<tos::PixPack> d_pix2;  // per sightline even pixels, odd pixels, padded (kParityPad)
-  tos::DevBuf<double> d_wd;         // w*delta per pixel, exact in double
-  tos::DevBuf<float> d_w;           // weight per pixel
-  tos::DevBuf<double4> d_prefix;    // per sightline N+1 exclusive prefix sums of (w*delta, w, loglam)
-  tos::DevBuf<double2> d_pre2;      // its (w*delta, w) alone
-  tos::DevBuf<double2> d_row2;      // (w*delta, w) per pixel
+  tos::DevBuf<double2> d_row2;      // (w*delta, w) per pixel, the product exact in double
+  tos::DevBuf<double2> d_pre2;      // per sightline N+1 exclusive prefix sums of (w*delta, w)
+  tos::DevBuf<double> d_prel;       // and of loglam
   tos::DevBuf<float4> d_range;      // per sightline (dmin, dmax, lmin, lmax)
   tos::DevBuf<unsigned int> d_flags;// [0]: bit 0 some sightline is not sorted by distance and
                                     // loglam, bit 1 a non-finite value; [1] order key of the

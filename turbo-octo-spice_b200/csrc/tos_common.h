@@ -33,11 +33,11 @@ constexpr int kPad = 32;
 // finite so that differences of sentinels never produce NaN.
 constexpr float kSentinel = 1.0e30f;
 
-// A pixel's distance, weight and w*delta in one 16-byte load.
 // Padding of the even-first pixel array of the Polar sweep: entries of zero
 // weight before, between and after a sightline's even and odd pixels (a group
 // of 64 diagonals and a block of 16 rows reach 40 entries past either half).
 constexpr int kParityPad = 40;
+// A pixel's distance, weight and w*delta in one 16-byte load.
 struct alignas(16) PixPack {
   float d, w;
   double wd;

@@ -106,6 +106,11 @@ __device__ __forceinline__ bool exact_obs(float l1, float l2, const RefGrid& g, 
   return true;
 }
 
+// Prefix sums of sightline i.
+__device__ __forceinline__ Prefix prefix_of(const PairArgs& A, uint32_t i) {
+  return Prefix{A.pre2 + A.off[i] + i, A.prel + A.off[i] + i};
+}
+
 // Items of the run-sweep kernel when A.run_split is set: z index constant
 // over the item and (Cartesian) 2(1 - cos theta) large enough for the
 // reference's r_perp expression to grow with the column distance along every

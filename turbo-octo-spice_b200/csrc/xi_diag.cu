@@ -75,8 +75,7 @@ struct DItem {
   int dlo, groups;       // first diagonal and number of 64-diagonal groups (0: the end)
   float ap;              // 2(1 - c)
   double c;
-  const double4* prei;   // prefix sums of the two sightlines
-  const double4* prej;
+  uint64_t prei, prej;   // the two sightlines' first prefix sums
   const PixPack* rows;   // padded pixels of sightline i, even ones first
   const PixPack* cols;   // padded pixels of sightline j, even ones first
 };
@@ -212,8 +211,10 @@ __device__ __noinline__ void drain(int buf, WarpQ& Q, int first, int n, int lane
     // the rows of the run inside the matrix
     const int s0 = max(Q.s0[e], -delta), s1 = min(min(Q.s1[e], it.ni), it.nj - delta);
     if (s1 > s0) {
-      const double4 ia = it.prei[s0], ib = it.prei[s1];
-      const double4 ja = it.prej[s0 + delta], jb = it.prej[s1 + delta];
+      const double2 *pi = A.pre2 + it.prei, *pj = A.pre2 + it.prej + delta;
+      const double *li = A.prel + it.prei, *lj = A.prel + it.prej + delta;
+      const double2 ia = pi[s0], ib = pi[s1], ja = pj[s0], jb = pj[s1];
+      const double lz = (li[s1] - li[s0]) + (lj[s1] - lj[s0]);
       const uint32_t b0 = key >> 16, b1 = key & 0xFFFFu;
       const uint32_t idx = it.zb + (b1 + b0 * A.g.n1) * A.g.n2;  // as XiEstimator.cc:196-201
       if (idx < A.g.ntotal)
@@ -226,7 +227,7 @@ __device__ __noinline__ void drain(int buf, WarpQ& Q, int first, int n, int lane
       Q.val[3][lane] = Q.wgt[e];
       Q.val[4][lane] = ib.y - ia.y;
       Q.val[5][lane] = jb.y - ja.y;
-      Q.val[6][lane] = 0.5 * ((ib.z - ia.z) + (jb.z - ja.z));
+      Q.val[6][lane] = 0.5 * lz;
       Q.val[7][lane] = __longlong_as_double((long long)(s1 - s0));
     }
   }
@@ -532,8 +533,8 @@ __device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsi
     const float4 ri = A.range[i], rj = A.range[j];
     it.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
     it.cell = dest_row(A, i, j);
-    it.prei = A.prefix + A.off[i] + i;
-    it.prej = A.prefix + A.off[j] + j;
+    it.prei = A.off[i] + i;
+    it.prej = A.off[j] + j;
     // Column window |d1 - d2| < lim of every row (the pixel-pair kernel's
     // Polar bound: r^2 >= (d2 - d1)^2 + 2(1 - c) dmin_i dmin_j - err), and
     // from it the diagonals that reach it.
@@ -578,8 +579,8 @@ __device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsi
     }
     it.dlo = dlo;
     it.groups = (dhi - dlo) / kDiagSpan + 1;
-    const PixPack *gi = A.pix2 + A.off[i] + (uint64_t)(3 * kParityPad) * i,
-                  *gj = A.pix2 + A.off[j] + (uint64_t)(3 * kParityPad) * j;
+    const PixPack *gi = A.pix2 + A.off[i] + (uint64_t)(2 * kParityPad) * i,
+                  *gj = A.pix2 + A.off[j] + (uint64_t)(2 * kParityPad) * j;
     const int len = A.max_np + 3 * kParityPad;
     it.rows = SMEM ? buf : gi;
     it.cols = SMEM ? buf + len : gj;

@@ -105,7 +105,7 @@ struct BandItem {
   double c;
   const double2* P;    // prefix sums (w*delta, w) of sightline j, by column
   const double2* R;    // (w*delta, w) of sightline i, by row
-  const double4* Ri;   // prefix sums of sightline i
+  const double2* Ri;   // prefix sums of sightline i
   // sightlines with gaps (PairArgs::gap_*): column prefix sums of (pixels,
   // l'/2), row values (1 where there is a pixel, l'/2), and the prefix sums of
   // sightline i
@@ -420,7 +420,7 @@ __device__ __forceinline__ void band_group(const PairArgs& A, const BandItem& it
           }
         } else if (y > y1) {
           const double2 p = it.P[nj];
-          const double4 ra = it.Ri[y1 - fi], rb = it.Ri[y - fi];
+          const double2 ra = it.Ri[y1 - fi], rb = it.Ri[y - fi];
           const double dn = (double)nj, dr = (double)(y - y1);
           x.s[0] = (rb.x - ra.x) * p.x;
           x.s[1] = (rb.x - ra.x) * dn;
@@ -542,7 +542,7 @@ __device__ __noinline__ int prepare_item(BandItem* h, int* next, double2* buf, u
       it.Pi = A.gap_pre + oi;
       it.Ci = A.gap_cnt + oi;
     } else {
-      it.Ri = A.prefix + A.off[i] + i;
+      it.Ri = A.pre2 + A.off[i] + i;
       gP = A.pre2 + A.off[j] + j;
       gR = A.row2 + A.off[i];
     }

@@ -27,7 +27,7 @@ struct Item {
   const float* colx; // padded column coordinate (distance or loglam) of sightline j
   const float* coll; // padded column loglam
   const float* cold; // padded column distance
-  const double4* pre;// prefix sums of sightline j
+  Prefix pre;        // prefix sums of sightline j
 };
 
 // Window slot of a packed key (b0 << 16 | b1), or -1 when outside the window.
@@ -333,7 +333,7 @@ __device__ void sweep_chunk(const PairArgs& A, const Item& it, const Row& R, boo
       bool emit = false;
       if (changed) {
         const int pc = min(max(p2, 0), (int)it.nj);
-        const double4 pn = it.pre[pc];
+        const double3 pn = it.pre[pc];
         if (cur != kInvalidKey) {
           emit = true;
           make_contrib(R, (uint32_t)(p2 - run_start), pn.x - ps0, pn.y - ps1, pn.z - ps2, ct);
@@ -358,7 +358,7 @@ __device__ void sweep_chunk(const PairArgs& A, const Item& it, const Row& R, boo
   const bool emit = cur != kInvalidKey;
   if (emit) {
     const int p_end = t_end + lane;
-    const double4 pn = it.pre[min(max(p_end, 0), (int)it.nj)];
+    const double3 pn = it.pre[min(max(p_end, 0), (int)it.nj)];
     make_contrib(R, (uint32_t)(p_end - run_start), pn.x - ps0, pn.y - ps1, pn.z - ps2, ct);
   }
   if (MODE == 0) {
@@ -390,8 +390,7 @@ __device__ void process_item(const PairArgs& A, Item& it, uint32_t* win, int lan
   const uint64_t oi = A.off[it.i];
   const float* rowd = A.dist_pad + oi + (uint64_t)kPad * (it.i + 1);
   const float* rowl = A.loglam_pad + oi + (uint64_t)kPad * (it.i + 1);
-  const double* rowwd = A.wd + oi;
-  const float* roww = A.w + oi;
+  const double2* row2 = A.row2 + oi;
   const float4 rj = A.range[it.j];
   // Column window |x1 - x2| < lim.  For Polar binning a pair is accepted only
   // if r^2 = (d2 - d1)^2 + 2(1 - c) d1 d2 - err < R^2 (err: float rounding of
@@ -414,8 +413,9 @@ __device__ void process_item(const PairArgs& A, Item& it, uint32_t* win, int lan
     if (active) {
       R.d1 = rowd[row];
       R.l1 = rowl[row];
-      R.wd1 = rowwd[row];
-      R.w1 = (double)roww[row];
+      const double2 q = row2[row];
+      R.wd1 = q.x;
+      R.w1 = q.y;
       R.hl1 = 0.5 * (double)R.l1;
       R.x1 = (COORD == kObs) ? R.l1 : R.d1;
       const float p = __fmul_rn(R.d1, R.d1);
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) pair_kernel(PairArgs A) {
       it.cold = A.dist_pad + oj;
       it.coll = A.loglam_pad + oj;
       it.colx = (COORD == kObs) ? it.coll : it.cold;
-      it.pre = A.prefix + A.off[it.j] + it.j;
+      it.pre = prefix_of(A, it.j);
       const double a = 2.0 * dsub(1.0, it.c);
       it.ap = (COORD == kCart) ? (float)(a * A.g.inv1 * A.g.inv1) : (float)a;
       // z index: constant over the item when both ends of the loglam-sum range agree

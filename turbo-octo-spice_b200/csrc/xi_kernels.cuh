@@ -66,6 +66,18 @@ constexpr int kMaxAddsPerItemBin = 8;
 constexpr double kMagic52 = 6755399441055744.0;  // 1.5 * 2^52
 constexpr long long kMagic52Bits = 0x4338000000000000LL;
 
+// Exclusive prefix sums of one sightline: (wd, w, loglam) of its first k pixels.
+struct Prefix {
+  const double2* w;
+  const double* l;
+#ifdef __CUDACC__
+  __device__ __forceinline__ double3 operator[](int k) const {
+    const double2 a = w[k];
+    return make_double3(a.x, a.y, l[k]);
+  }
+#endif
+};
+
 struct PairArgs {
   // catalogue
   const uint64_t* off;       // compact pixel offset of each sightline
@@ -73,10 +85,10 @@ struct PairArgs {
   const float* dist_pad;     // padded distances
   const float* loglam_pad;   // padded log10 wavelengths
   const PixPack* pix2;       // (distance, weight, w*delta) per pixel: per sightline kParityPad zeros, its even
-                             // pixels, kParityPad zeros, its odd pixels, kParityPad zeros
-  const double* wd;          // w * delta (exact double) per pixel
-  const float* w;            // weight per pixel
-  const double4* prefix;     // per sightline, N+1 exclusive prefix sums of (wd, w, loglam)
+                             // pixels, kParityPad zeros, its odd pixels, and kParityPad zeros, the next one's first
+  const double2* row2;       // (w * delta, w) per pixel
+  const double2* pre2;       // per sightline, N+1 exclusive prefix sums of (wd, w)
+  const double* prel;        // and of loglam
   const float4* range;       // per sightline (dmin, dmax, lmin, lmax)
   const uint32_t* cell_idx;  // cell index of each sightline
   // accumulation row of a pair: the primary sightline's cell, or, when
@@ -143,8 +155,6 @@ struct PairArgs {
   // entries) of (wd, w) and of (1, l'/2), and the values themselves
   const uint64_t* gap_off;
   const double2 *gap_pre, *gap_cnt, *gap_row, *gap_one;
-  const double2* pre2;       // prefix sums (wd, w) alone, laid out as `prefix`
-  const double2* row2;       // (w*delta, w) per pixel
   double lmid;               // loglam near the middle of the grid
   // bounds (x, y) of code edge m = 0 .. n1 on u = 2 (1 - c) d1 d2 inv1^2 as
   // computed in FP32 without the row's rounding term: a column with u < x has

@@ -60,9 +60,9 @@ __device__ __noinline__ void run_group(const PairArgs& A, const SweepItem& it, i
   const Dest d = it.d;
   const double c = it.c;
   const float ap = it.ap, inv1sqf = A.inv1sqf;
-  const float *rowd = it.rowd, *rowl = it.rowl, *roww = it.roww, *rowx = it.rowx, *colx = it.colx;
-  const double* rowwd = it.rowwd;
-  const double4* pre = it.pre;
+  const float *rowd = it.rowd, *rowl = it.rowl, *rowx = it.rowx, *colx = it.colx;
+  const double2* row2 = it.row2;
+  const Prefix pre = it.pre;
   const float ta = A.thr[k], tb = A.thr[k + 1];
   const float x1f = rowx[min(r_lo + phase, r_hi - 1)];
   ColPtr pa, pb;
@@ -83,7 +83,7 @@ __device__ __noinline__ void run_group(const PairArgs& A, const SweepItem& it, i
     const int s = side ? pb.p : pa.p, e = side ? pa.p : pb.p;
     if (e > s) {
       n_eval += (unsigned long long)(e - s);
-      const RowV R = row_values<COORD>(rowd, rowwd, roww, rowl, ap, inv1sqf, r);
+      const RowV R = row_values<COORD>(rowd, row2, rowl, ap, inv1sqf, r);
       do_run<COORD, MINPOS>(A, d, colx, pre, c, R, k, s, e, acc, rech);
     }
   }

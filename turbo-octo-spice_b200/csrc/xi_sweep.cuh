@@ -196,10 +196,10 @@ __device__ __forceinline__ void add_sums(const PairArgs& A, Dest d, const RowV& 
 
 // Add the sub-run [s, e) with r_perp code cc of first-axis bin k.
 template <int COORD, class Acc>
-__device__ __forceinline__ void add_subrun(const PairArgs& A, Dest d, const double4* pre,
+__device__ __forceinline__ void add_subrun(const PairArgs& A, Dest d, const Prefix& pre,
                                            const RowV& R, int k, int cc, int s, int e,
                                            Acc& acc) {
-  const double4 ps = pre[s], pe = pre[e];
+  const double3 ps = pre[s], pe = pre[e];
   add_sums<COORD>(A, d, R, k, cc, e - s, pe.x - ps.x, pe.y - ps.y, pe.z - ps.z, acc);
 }
 
@@ -208,7 +208,7 @@ __device__ __forceinline__ void add_subrun(const PairArgs& A, Dest d, const doub
 // between the ends when they differ) and add.
 template <int COORD, bool MINPOS, class Acc>
 __device__ __forceinline__ void do_run_from(const PairArgs& A, Dest d, const float* colx,
-                                            const double4* pre, double c, const RowV& R, int k, int s,
+                                            const Prefix& pre, double c, const RowV& R, int k, int s,
                                             int e, int code, Acc& acc, unsigned& rech) {
   const int ce = (e - 1 == s) ? code : perp_code<MINPOS>(A, R, colx[e - 1], c, rech);
   const int n1 = (int)A.g.n1;
@@ -244,7 +244,7 @@ __device__ __forceinline__ void do_run_from(const PairArgs& A, Dest d, const flo
 // the run's ends; bisection between them when they differ) and add.
 template <int COORD, bool MINPOS>
 __device__ __forceinline__ void do_run(const PairArgs& A, Dest d, const float* colx,
-                                       const double4* pre, double c, const RowV& R, int k, int s,
+                                       const Prefix& pre, double c, const RowV& R, int k, int s,
                                        int e, RunAcc& acc, unsigned& rech) {
   if (COORD == kObs) {
     add_subrun<COORD>(A, d, pre, R, k, 0, s, e, acc);
@@ -282,9 +282,9 @@ struct SweepItem {
   Dest d;
   double c;
   float ap;  // Cartesian: 2 (1 - c) inv1^2
-  const float *rowd, *rowl, *rowx, *roww, *colx;
-  const double* rowwd;
-  const double4* pre;
+  const float *rowd, *rowl, *rowx, *colx;
+  const double2* row2;
+  Prefix pre;
 };
 
 // Load work item idx; false when the item belongs to another kernel (z index
@@ -313,10 +313,9 @@ __device__ __forceinline__ bool load_item(const PairArgs& A, unsigned long long 
   it.rowd = A.dist_pad + oi;
   it.rowl = A.loglam_pad + oi;
   it.rowx = (COORD == kObs) ? it.rowl : it.rowd;
-  it.rowwd = A.wd + A.off[it.i];
-  it.roww = A.w + A.off[it.i];
+  it.row2 = A.row2 + A.off[it.i];
   it.colx = (COORD == kObs) ? A.loglam_pad + oj : A.dist_pad + oj;
-  it.pre = A.prefix + A.off[it.j] + it.j;
+  it.pre = prefix_of(A, it.j);
   const float cmin = (COORD == kObs) ? rj.z : rj.x, cmax = (COORD == kObs) ? rj.w : rj.y;
   const double a = 2.0 * dsub(1.0, it.c);
   it.ap = (float)(a * A.g.inv1 * A.g.inv1);
@@ -325,30 +324,16 @@ __device__ __forceinline__ bool load_item(const PairArgs& A, unsigned long long 
   return true;
 }
 
-// The loaded values of row r of an item (loaded a row ahead by the grid
-// sweep) and the row values derived from them.
-struct RowRaw {
-  float d1, w1, l1;
-  double wd1;
-};
-
-__device__ __forceinline__ RowRaw row_raw(const float* rowd, const double* rowwd, const float* roww,
-                                          const float* rowl, int r) {
-  RowRaw q;
-  q.d1 = rowd[r];
-  q.wd1 = rowwd[r];
-  q.w1 = roww[r];
-  q.l1 = rowl[r];
-  return q;
-}
-
+// Row values of row r of an item.
 template <int COORD>
-__device__ __forceinline__ RowV row_derive(const RowRaw& q, float ap, float inv1sqf) {
+__device__ __forceinline__ RowV row_values(const float* rowd, const double2* row2, const float* rowl, float ap,
+                                           float inv1sqf, int r) {
   RowV R;
-  R.d1 = q.d1;
-  R.wd1 = q.wd1;
-  R.w1 = (double)q.w1;
-  R.hl1 = 0.5 * (double)q.l1;
+  const double2 q = row2[r];
+  R.d1 = rowd[r];
+  R.wd1 = q.x;
+  R.w1 = q.y;
+  R.hl1 = 0.5 * (double)rowl[r];
   if (COORD == kCart) {
     const float p = __fmul_rn(R.d1, R.d1);
     const float err = __fmaf_rn(R.d1, R.d1, -p);  // d1*d1 = p + err exactly
@@ -358,13 +343,6 @@ __device__ __forceinline__ RowV row_derive(const RowRaw& q, float ap, float inv1
     R.A1 = R.dl1 = 0.f;
   }
   return R;
-}
-
-// Row r of an item.
-template <int COORD>
-__device__ __forceinline__ RowV row_values(const float* rowd, const double* rowwd, const float* roww,
-                                           const float* rowl, float ap, float inv1sqf, int r) {
-  return row_derive<COORD>(row_raw(rowd, rowwd, roww, rowl, r), ap, inv1sqf);
 }
 
 // Warp-sum the kernel's counters into A.counters[0] (evaluated pairs), [1]
