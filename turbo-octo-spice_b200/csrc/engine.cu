@@ -636,11 +636,18 @@ __device__ __forceinline__ int grid_index(const float* U, int ng, float x) {
 // pointers: 540 of 600 values 11.6 / 17.2 | 104 / 70, 204 of 600 10.8 / 16.9 |
 // 102 / 28, 150 of 600 25 / 22 | 60 / 21; 320k / 719k items of 64 of 128
 // values 10.9 / 20.0 | 19.0 / 21.3, 43 of 128 10.5 / 19.9 | 13.0 / 15.2, 16 of
-// 64 7.3 / 12.4 | 4.6 / 6.0).  count[0]: contiguous sightlines, count[1]:
-// those with gaps, count[2]: largest span, count[3]: contiguous ones of at most
-// kShortPixels pixels.
+// 64 7.3 / 12.4 | 4.6 / 6.0).
+//
+// What ensure_grid reads of a grid: values, contiguous sightlines and those with
+// gaps, the largest span, contiguous ones of at most kShortPixels pixels, the sum
+// of the spans, sightlines with a pixel whose loglam is not its grid value's, and
+// (float bits) loglam of the middle value, the first and the last value.
+enum GridInfo {
+  kGridValues = 0, kGridContiguous, kGridGaps, kGridMaxSpan, kGridShort, kGridSpans, kGridBad, kGridMid, kGridLo,
+  kGridHi, kGridInfo
+};
 __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint32_t* npix, size_t n_los,
-                             const float* U, int ng, uint32_t* gfirst, uint32_t* gspan, unsigned long long* count) {
+                             const float* U, int ng, uint32_t* gfirst, uint32_t* gspan, unsigned long long* info) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -661,9 +668,10 @@ __global__ void k_grid_first(const float* xpad, const uint64_t* off, const uint3
       gfirst[s] = f;
       gspan[s] = f == kNoGrid ? 0u : span;
       if (f != kNoGrid) {
-        atomicAdd(&count[span == n ? 0 : 1], 1ull);
-        atomicMax(&count[2], (unsigned long long)span);
-        if (span == n && n <= kShortPixels) atomicAdd(&count[3], 1ull);
+        atomicAdd(&info[span == n ? kGridContiguous : kGridGaps], 1ull);
+        atomicMax(&info[kGridMaxSpan], (unsigned long long)span);
+        atomicAdd(&info[kGridSpans], (unsigned long long)span);
+        if (span == n && n <= kShortPixels) atomicAdd(&info[kGridShort], 1ull);
       }
     }
   }
@@ -754,8 +762,22 @@ __global__ void k_grid_loglam(int pass, const float* xpad, const float* lpad, co
 constexpr int kTableThreads = 256;
 constexpr int kSkewPad = 3;  // blocks before a skewed boundary's first and after its last
 
-// glp[g] = sum over g' < g of gl[g'] - lmid, g = 0 .. ng (one block).
-__global__ void __launch_bounds__(kTableThreads) k_grid_lprefix(const float* gl, int ng, double lmid, double* glp) {
+// The number of grid values: the padding sentinel, the largest value, is none.
+__global__ void k_grid_count(const float* uniq, const int* nsel, unsigned long long* info) {
+  const int ng = *nsel;
+  info[kGridValues] = ng > 0 && uniq[ng - 1] == kSentinel ? ng - 1 : ng;
+}
+
+// glp[g] = sum over g' < g of gl[g'] - lmid, g = 0 .. ng (one block), lmid the
+// loglam of the middle value.
+__global__ void __launch_bounds__(kTableThreads)
+    k_grid_lprefix(const float* gl, const float* U, int ng, double* glp, unsigned long long* info) {
+  const double lmid = (double)gl[ng / 2];
+  if (threadIdx.x == 0) {
+    info[kGridMid] = __float_as_uint(gl[ng / 2]);
+    info[kGridLo] = __float_as_uint(U[0]);
+    info[kGridHi] = __float_as_uint(U[ng - 1]);
+  }
   using Scan = cub::BlockScan<double, kTableThreads>;
   __shared__ typename Scan::TempStorage tmp;
   double base = 0.0;
@@ -880,88 +902,80 @@ tos_status ensure_grid(tos_engine* e, tos_catalog* cat, int w, cudaStream_t st) 
     cat->grid_n[w] = 0;
     return TOS_OK;
   }
-  DevBuf<float> sorted, uniq;
-  DevBuf<int> nsel;
-  TOS_TRY(sorted.alloc(n));
-  TOS_TRY(uniq.alloc(n));
-  TOS_TRY(nsel.alloc(1));
+  // one scratch buffer, two reads by the host: the number of values, then the rest
+  float *sorted = nullptr, *uniq = nullptr;
+  int* nsel = nullptr;
+  unsigned long long* info = nullptr;
+  unsigned char* tmp = nullptr;
   size_t tb1 = 0, tb2 = 0;
-  cub::DeviceRadixSort::SortKeys(nullptr, tb1, x, sorted.p, (int)n, 0, 32, st);
-  cub::DeviceSelect::Unique(nullptr, tb2, sorted.p, uniq.p, nsel.p, (int)n, st);
-  DevBuf<unsigned char> tmp;
-  TOS_TRY(tmp.alloc(std::max(tb1, tb2) + 16));
-  TOS_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, tb1, x, sorted.p, (int)n, 0, 32, st));
-  TOS_CUDA_TRY(cub::DeviceSelect::Unique(tmp.p, tb2, sorted.p, uniq.p, nsel.p, (int)n, st));
-  int ng = 0;
-  TOS_CUDA_TRY(cudaMemcpyAsync(&ng, nsel.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  // the padding sentinel is the largest value: not part of the grid
-  if (ng > 0) {
-    float last = 0;
-    TOS_CUDA_TRY(cudaMemcpy(&last, uniq.p + ng - 1, sizeof(float), cudaMemcpyDeviceToHost));
-    if (last == kSentinel) --ng;
+  cub::DeviceRadixSort::SortKeys(nullptr, tb1, x, sorted, (int)n, 0, 32, st);
+  cub::DeviceSelect::Unique(nullptr, tb2, sorted, uniq, nsel, (int)n, st);
+  DevBuf<unsigned char> scratch;
+  Carve c;
+  for (int pass = 0; pass < 2; ++pass) {
+    c = Carve{scratch.p};
+    sorted = c.take<float>(n);
+    uniq = c.take<float>(n);
+    nsel = c.take<int>(1);
+    info = c.take<unsigned long long>(kGridInfo);
+    tmp = c.take<unsigned char>(std::max(tb1, tb2));
+    if (pass == 0) TOS_TRY(scratch.alloc(c.off));
   }
-  tmp.release();
-  sorted.release();
+  TOS_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp, tb1, x, sorted, (int)n, 0, 32, st));
+  TOS_CUDA_TRY(cub::DeviceSelect::Unique(tmp, tb2, sorted, uniq, nsel, (int)n, st));
+  TOS_CUDA_TRY(cudaMemsetAsync(info, 0, kGridInfo * 8, st));
+  k_grid_count<<<1, 1, 0, st>>>(uniq, nsel, info);
+  TOS_CUDA_TRY(cudaGetLastError());
+  unsigned long long h[kGridInfo] = {};
+  TOS_CUDA_TRY(cudaMemcpyAsync(h, info, 8, cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  const int ng = (int)h[0];
   cat->grid_n[w] = 0;
   if (ng <= 0 || ng > 65535) {
     cat->grid_built[w] = true;
     return TOS_OK;
   }
   TOS_TRY(cat->d_grid[w].alloc(ng));
-  TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_grid[w].p, uniq.p, ng * sizeof(float), cudaMemcpyDeviceToDevice, st));
   TOS_TRY(cat->d_gfirst[w].alloc(cat->n_los));
   TOS_TRY(cat->d_gspan[w].alloc(cat->n_los));
-  DevBuf<unsigned long long> nok;
-  TOS_TRY(nok.alloc(4));
-  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 32, st));
-  const int gw = grid_for(e, cat->n_los * 32, 256);
-  k_grid_first<<<gw, 256, 0, st>>>(x, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_grid[w].p, ng,
-                                   cat->d_gfirst[w].p, cat->d_gspan[w].p, nok.p);
-  TOS_CUDA_TRY(cudaGetLastError());
-  unsigned long long h[4] = {0, 0, 0, 0};
-  TOS_CUDA_TRY(cudaMemcpyAsync(h, nok.p, 32, cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h[0] + h[1] == 0) {
-    cat->grid_built[w] = true;
-    return TOS_OK;
-  }
-  // for contiguous sightlines the grid sweep takes a pixel's loglam from its
-  // grid value: not usable when two pixels of one value differ in it
   TOS_TRY(cat->d_gl[w].alloc(ng));
   TOS_TRY(cat->d_glp[w].alloc(ng + 1));
+  TOS_CUDA_TRY(cudaMemcpyAsync(cat->d_grid[w].p, uniq, ng * sizeof(float), cudaMemcpyDeviceToDevice, st));
+  const int gw = grid_for(e, cat->n_los * 32, 256);
+  k_grid_first<<<gw, 256, 0, st>>>(x, cat->d_off.p, cat->d_npix.p, cat->n_los, cat->d_grid[w].p, ng,
+                                   cat->d_gfirst[w].p, cat->d_gspan[w].p, info);
+  // for contiguous sightlines the grid sweep takes a pixel's loglam from its
+  // grid value: not usable when two pixels of one value differ in it
   TOS_CUDA_TRY(cudaMemsetAsync(cat->d_gl[w].p, 0, ng * sizeof(float), st));
-  TOS_CUDA_TRY(cudaMemsetAsync(nok.p, 0, 8, st));
   for (int pass = 0; pass < 2; ++pass)
     k_grid_loglam<<<gw, 256, 0, st>>>(pass, x, cat->d_loglam_pad.p, cat->d_off.p, cat->d_npix.p, cat->n_los,
                                       cat->d_grid[w].p, ng, cat->d_gfirst[w].p, cat->d_gspan[w].p, cat->d_gl[w].p,
-                                      nok.p);
+                                      info + kGridBad);
+  k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, cat->d_grid[w].p, ng, cat->d_glp[w].p, info);
   TOS_CUDA_TRY(cudaGetLastError());
-  unsigned long long bad = 0;
-  float lmid = 0.f;
-  TOS_CUDA_TRY(cudaMemcpyAsync(&bad, nok.p, 8, cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaMemcpyAsync(&lmid, cat->d_gl[w].p + ng / 2, sizeof(float), cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaMemcpyAsync(h, info, sizeof(h), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  cat->grid_geo[w] = bad == 0;
-  cat->grid_lmid[w] = (double)lmid;
-  if (h[1] || bad) {  // these are laid out on the grid (ensure_layout)
-    std::vector<uint32_t> span(cat->n_los);
-    TOS_CUDA_TRY(cudaMemcpy(span.data(), cat->d_gspan[w].p, span.size() * 4, cudaMemcpyDeviceToHost));
-    uint64_t tot = 0;
-    for (uint32_t v : span) tot += (uint64_t)v + 1;
-    cat->gaps[w].entries = tot;
+  auto as_float = [](unsigned long long v) {
+    const uint32_t u = (uint32_t)v;
+    float f;
+    std::memcpy(&f, &u, 4);
+    return f;
+  };
+  if (h[kGridContiguous] + h[kGridGaps] == 0) {
+    cat->grid_built[w] = true;
+    return TOS_OK;
   }
-  k_grid_lprefix<<<1, kTableThreads, 0, st>>>(cat->d_gl[w].p, ng, (double)lmid, cat->d_glp[w].p);
-  TOS_CUDA_TRY(cudaGetLastError());
-  TOS_CUDA_TRY(cudaStreamSynchronize(st));
-  TOS_CUDA_TRY(cudaMemcpyAsync(&cat->grid_lo[w], cat->d_grid[w].p, sizeof(float), cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaMemcpyAsync(&cat->grid_hi[w], cat->d_grid[w].p + ng - 1, sizeof(float), cudaMemcpyDeviceToHost, st));
-  TOS_CUDA_TRY(cudaStreamSynchronize(st));
+  cat->grid_geo[w] = h[kGridBad] == 0;
+  cat->grid_lmid[w] = (double)as_float(h[kGridMid]);
+  cat->grid_lo[w] = as_float(h[kGridLo]);
+  cat->grid_hi[w] = as_float(h[kGridHi]);
+  // these are laid out on the grid (ensure_layout)
+  if (h[kGridGaps] || h[kGridBad]) cat->gaps[w].entries = h[kGridSpans] + cat->n_los;
   cat->grid_n[w] = ng;
-  cat->max_span[w] = (uint32_t)h[2];
-  cat->grid_los[w] = h[0];
-  cat->grid_short[w] = h[3];
-  cat->grid_gaps[w] = h[1];
+  cat->max_span[w] = (uint32_t)h[kGridMaxSpan];
+  cat->grid_los[w] = h[kGridContiguous];
+  cat->grid_short[w] = h[kGridShort];
+  cat->grid_gaps[w] = h[kGridGaps];
   cat->grid_built[w] = true;
   return TOS_OK;
 }
