@@ -428,10 +428,19 @@ tos_status tos_brute_run(tos_engine* engine, const float* points, size_t n_point
  * warps per CTA on the first min(n_points, 131072) points and keeps the
  * fastest on the engine.  Later tos_brute_run and tos_brute_run_noalloc calls
  * with that bin count use it; results do not depend on the shape (exact
- * integer sums).  The pick is written to *diagonals_per_lane and
+ * integer sums).  Points in lines of equal steps (a regular grid) have a kernel
+ * of their own: only the warps are tuned then (*diagonals_per_lane is 1), on
+ * whole lines, and the pick is used for such points only, as one from other
+ * points is for those.  The pick is written to *diagonals_per_lane and
  * *warps_per_cta (either may be null). */
 tos_status tos_brute_tune(tos_engine* engine, const float* points, size_t n_points, double min,
                           double max, int nbins, int* diagonals_per_lane, int* warps_per_cta);
+
+/* What the engine's last brute-force count ran: points per line of equal steps
+ * (0: the points were not taken as lines), diagonals per lane and warps per CTA
+ * (any may be null; 0 before the first count). */
+tos_status tos_brute_last_shape(tos_engine* engine, int* points_per_line, int* diagonals_per_lane,
+                                int* warps_per_cta);
 
 /* tos_brute_run without any device allocation.  No counterpart in the
  * reference: it is for callers that cannot allocate GPU memory while they

@@ -723,6 +723,7 @@ tos_status brute_launch_shape(tos_engine* e, BruteArgs A, cudaStream_t st, int v
   TOS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
   TOS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem));
+  e->brute_last[0] = A.P, e->brute_last[1] = A.P ? 1 : kVariants[vi].k, e->brute_last[2] = warps;
   TOS_CUDA_TRY(cudaEventRecord(e->ev[4], st));
   fn<<<e->num_sms * std::max(1, per_sm), warps * 32, smem, st>>>(A);
   TOS_CUDA_TRY(cudaGetLastError());
@@ -730,14 +731,15 @@ tos_status brute_launch_shape(tos_engine* e, BruteArgs A, cudaStream_t st, int v
   return TOS_OK;
 }
 
-// The default shape, or the one tos_brute_tune picked for this bin count.
+// The default shape, or the one tos_brute_tune picked for this bin count and
+// kernel (points in lines or not).
 constexpr int kBruteDefaultVariant = 0, kBruteDefaultWarps = 8;
 
 tos_status brute_launch(tos_engine* e, const BruteArgs& A, cudaStream_t st) {
   int vi = kBruteDefaultVariant, warps_max = kBruteDefaultWarps;
   {
     std::lock_guard<std::mutex> lk(e->tune_mu);
-    auto it = e->brute_tuned.find(A.nbins);
+    auto it = e->brute_tuned.find({A.nbins, A.P != 0});
     if (it != e->brute_tuned.end()) {
       vi = it->second.first;
       warps_max = it->second.second;
@@ -776,8 +778,10 @@ tos_status brute_check(const void* points, size_t n_points, double min, double m
 }
 
 // Upload the points and thresholds, check and prepare them, and set up the
-// kernel arguments on the engine's scratch (its lock held).
-tos_status brute_setup(tos_engine* e, const float* points, int n, double min, double max, int nbins, BruteArgs* A) {
+// kernel arguments on the engine's scratch (its lock held), for the first
+// `limit` points or whole lines of them.
+tos_status brute_setup(tos_engine* e, const float* points, int n, double min, double max, int nbins, BruteArgs* A,
+                       int limit = 1 << 30) {
   BruteScratch& W = e->brute;
   cudaStream_t st = e->stream;
   const int nb2 = nbins + 2;
@@ -795,6 +799,7 @@ tos_status brute_setup(tos_engine* e, const float* points, int n, double min, do
   TOS_CUDA_TRY(cudaMemsetAsync(W.misc.p, 0, 9 * 8, st));
   BruteBounds B;
   TOS_TRY(brute_look(W.pts.p, n, W.misc.p + 2, st, &B));
+  if (n > limit) n = B.P ? limit / B.P * B.P : limit;
   brute_args(*A, n, nbins, min, max, B);
   TOS_TRY(brute_prepare(A, W.pts.p, W.pos.p, W.wd.p, st));
   A->th = W.th.p;
@@ -850,8 +855,9 @@ extern "C" tos_status tos_brute_run(tos_engine* e, const float* points, size_t n
 }
 
 // Autotuner of the brute-force kernel's launch shape: every variant (1, 2 or
-// 4 diagonals per lane) with 4, 8 and 16 warps per CTA, timed on the first
-// min(n, 131072) points, best of two timed launches after a warm-up.
+// 4 diagonals per lane; one for points in lines, whose kernel has no such
+// choice) with 4, 8 and 16 warps per CTA, timed on the first 131,072 points (or
+// as many whole lines), best of two timed launches after a warm-up.
 extern "C" tos_status tos_brute_tune(tos_engine* e, const float* points, size_t n_points, double min,
                                      double max, int nbins, int* diagonals_per_lane, int* warps_per_cta) {
   if (!e) return fail(TOS_ERR_INVALID_ARG, "null argument");
@@ -859,14 +865,14 @@ extern "C" tos_status tos_brute_tune(tos_engine* e, const float* points, size_t 
   std::lock_guard<std::mutex> lock(e->mu);
   DevScope dev(e->device);
   BruteKeep keep{e};
-  const int n = (int)std::min<size_t>(n_points, 131072);
   cudaStream_t st = e->stream;
   BruteArgs A{};
-  TOS_TRY(brute_setup(e, points, n, min, max, nbins, &A));
+  TOS_TRY(brute_setup(e, points, (int)n_points, min, max, nbins, &A, 131072));
   const int warp_opts[3] = {4, 8, 16};
   float best = 0.f;
   int best_v = kBruteDefaultVariant, best_w = kBruteDefaultWarps;
-  for (int vi = 0; vi < (int)(sizeof(kVariants) / sizeof(kVariants[0])); ++vi) {
+  const int variants = A.P ? 1 : (int)(sizeof(kVariants) / sizeof(kVariants[0]));
+  for (int vi = 0; vi < variants; ++vi) {
     for (int wo : warp_opts) {
       float t_min = 0.f;
       for (int rep = 0; rep < 3; ++rep) {
@@ -887,10 +893,20 @@ extern "C" tos_status tos_brute_tune(tos_engine* e, const float* points, size_t 
   }
   {
     std::lock_guard<std::mutex> lk(e->tune_mu);
-    e->brute_tuned[nbins] = std::make_pair(best_v, best_w);
+    e->brute_tuned[{nbins, A.P != 0}] = std::make_pair(best_v, best_w);
   }
   if (diagonals_per_lane) *diagonals_per_lane = kVariants[best_v].k;
   if (warps_per_cta) *warps_per_cta = best_w;
+  return TOS_OK;
+}
+
+extern "C" tos_status tos_brute_last_shape(tos_engine* e, int* points_per_line, int* diagonals_per_lane,
+                                           int* warps_per_cta) {
+  if (!e) return fail(TOS_ERR_INVALID_ARG, "null argument");
+  std::lock_guard<std::mutex> lock(e->mu);
+  if (points_per_line) *points_per_line = e->brute_last[0];
+  if (diagonals_per_lane) *diagonals_per_lane = e->brute_last[1];
+  if (warps_per_cta) *warps_per_cta = e->brute_last[2];
   return TOS_OK;
 }
 

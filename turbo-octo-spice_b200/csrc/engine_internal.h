@@ -234,10 +234,12 @@ struct tos_engine {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[8] = {};
   std::mutex mu;
-  // launch shapes picked by the autotuner (tos_brute_tune), by bin count:
+  // launch shapes picked by the autotuner (tos_brute_tune), by bin count and whether points in lines:
   // (kernel variant, warps per CTA)
   std::mutex tune_mu;
-  std::map<int, std::pair<int, int>> brute_tuned;
+  std::map<std::pair<int, bool>, std::pair<int, int>> brute_tuned;
+  // the last brute-force launch: points per line (0: not in lines), diagonals per lane, warps per CTA (under mu)
+  int brute_last[3] = {0, 0, 0};
   // the longest a kernel waits on a barrier (tos_engine_set_wait_limit; under mu)
   uint32_t wait_ms = 10000;
   tos::BruteScratch brute;

@@ -115,6 +115,7 @@ def lib() -> C.CDLL:
         L.tos_brute_run.argtypes = [vp, vp, sz, dbl, dbl, i32, vp, vp, vp, C.POINTER(dbl)]
         L.tos_brute_run_noalloc.argtypes = [vp, vp, sz, dbl, dbl, i32, vp, vp, vp, C.POINTER(dbl)]
         L.tos_brute_tune.argtypes = [vp, vp, sz, dbl, dbl, i32, C.POINTER(i32), C.POINTER(i32)]
+        L.tos_brute_last_shape.argtypes = [vp, C.POINTER(i32), C.POINTER(i32), C.POINTER(i32)]
         L.tos_xi_cell_covariance.argtypes = [vp, vp, vp, vp, vp]
         L.tos_xi_jackknife.argtypes = [vp, vp, i32, sz, C.POINTER(sz), vp, vp, vp]
         L.tos_xi_subsample_covariance.argtypes = [vp, vp, sz, sz, vp, vp, vp]
@@ -508,6 +509,14 @@ def brute_tune(engine: Engine, points: np.ndarray, rmin: float, rmax: float, nbi
     k, w = C.c_int(), C.c_int()
     _check(lib().tos_brute_tune(engine.handle, _ptr(pts), len(pts), rmin, rmax, nbins, C.byref(k), C.byref(w)))
     return k.value, w.value
+
+
+def brute_last_shape(engine: Engine):
+    """(points per line of equal steps or 0, diagonals per lane, warps per CTA)
+    of the engine's last brute-force count."""
+    v = [C.c_int() for _ in range(3)]
+    _check(lib().tos_brute_last_shape(engine.handle, *[C.byref(x) for x in v]))
+    return tuple(x.value for x in v)
 
 
 def brute_run_noalloc(engine: Engine, points_ptr: int, n_points: int, rmin: float, rmax: float,
