@@ -1569,7 +1569,7 @@ constexpr int kChunkCounters = 4128;
 constexpr int kMaxChunks = 64;
 constexpr uint64_t kChunkItemsMin = 131072;  // tens of ms per chunk: the launch tail stays small
 // sweeps that a request runs in chunks
-enum SweepKind { kSweepDiag = 0, kSweepGrid, kSweepShort, kSweepKinds };
+enum SweepKind { kSweepDiag = 0, kSweepGrid, kSweepShort, kSweepGaps, kSweepKinds };
 constexpr size_t kCounterWords = kChunkCounters + kSweepKinds * kMaxChunks;
 
 // Host callback after a shared-GPU sweep chunk: hands the SMs back.
@@ -2134,15 +2134,18 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // of chunk launches, each with its own item counter (ctr[kChunkCounters ..],
   // after the theta-edge flags of observing grids at ctr[16 ..]) and its CTA
   // count asked just before launch.
-  static const char* const sweep_name[kSweepKinds] = {"diagonal", "grid", "short"};
+  static const char* const sweep_name[kSweepKinds] = {"diagonal", "grid", "short", "gap"};
   auto sweep = [&](SweepKind kind, unsigned long long* counter) -> tos_status {
     auto launch = [&](PairArgs& R, int per_sm) -> cudaError_t {
       switch (kind) {
         case kSweepDiag: return launch_diag_kernel(R, minpos, e->num_sms, per_sm, st);
         case kSweepGrid: return launch_grid_kernel(R, G.type, minpos, e->num_sms, per_sm, st);
-        default:
+        case kSweepShort:
           R.max_span = std::min(R.max_span, (int)kShortPixels);
           return launch_short_kernel(R, G.type, minpos, e->num_sms, st);
+        default:
+          R.max_span = (int)cat->max_span[G.type == TOS_OBSERVING ? 1 : 0];
+          return launch_gap_kernel(R, G.type, minpos, e->num_sms, st);
       }
     };
     if (!share) {
@@ -2189,13 +2192,7 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
     if (use_grid) TOS_TRY(sweep(kSweepGrid, ctr + 10));
     if (use_short) TOS_TRY(sweep(kSweepShort, ctr + 15));
     TOS_CUDA_TRY(cudaEventRecord(e->ev[6], st));
-    if (A.gap_split) {
-      PairArgs R = A;
-      R.next_item = ctr + 14;
-      R.max_span = (int)cat->max_span[G.type == TOS_OBSERVING ? 1 : 0];
-      const cudaError_t ge2 = launch_gap_kernel(R, G.type, minpos, e->num_sms, st);
-      if (ge2 != cudaSuccess) return fail(TOS_ERR_CUDA, std::string("gap kernel: ") + cudaGetErrorString(ge2));
-    }
+    if (A.gap_split) TOS_TRY(sweep(kSweepGaps, ctr + 14));
     if (use_runs) {
       PairArgs R = A;
       R.next_item = ctr + 7;
