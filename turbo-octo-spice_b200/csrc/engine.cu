@@ -549,6 +549,16 @@ float polar_r2_small(const RefGrid& g, double max_d, int k0, int k1) {
   return (float)std::max({1e-4, r0 * r0, 2.0 * std::ldexp(t1 * e, k1)});
 }
 
+// Error of the FP32 r_perp code t = sqrt(u) - min1 inv1 near an edge, from the
+// same cancellation (polar_r2_small): u, the square of r_perp inv1, is off by
+// 2^-47 D^2 inv1^2 whatever its size, and sqrt(u) at the smallest edge above 0
+// by that over twice the edge.
+double cart_code_error(const RefGrid& g, double max_d) {
+  const double e = std::ldexp(max_d * max_d, -47) * g.inv1 * g.inv1;
+  const double off = g.min1 * g.inv1, frac = off - std::floor(off);
+  return std::min(e / (2.0 * (frac > 1e-9 ? frac : 1.0)), std::sqrt(e));
+}
+
 // Thresholds of the Polar codes (PairArgs::thr_r2, thr_mu2): code >= k means
 // ref_u32((x - min) * inv) >= k with t > -1 (k = 0: t > -1).
 std::vector<double> polar_thresholds(const RefGrid& g) {
@@ -1893,6 +1903,11 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   A.n1p1f = (float)n1 + 1.0f;
   A.k0 = std::max(0, std::min(13, 21 - bitlen(n0 + 2)));
   A.k1 = std::max(0, std::min(13, 21 - bitlen(n1 + 2)));
+  if (G.type == TOS_CARTESIAN) {
+    const double dt = cart_code_error(rg, cat->max_d);
+    if (dt > 0.125) A.force_exact = 1;  // bins finer than the distances' rounding
+    A.k1 = std::max(0, std::min(A.k1, (int)std::floor(-std::log2(std::max(2.0 * dt, 1e-9)))));
+  }
   A.mag0 = std::ldexp(1.5f, 23 - A.k0);
   A.mag1 = std::ldexp(1.5f, 23 - A.k1);
   std::memcpy(&A.bits0, &A.mag0, 4);
