@@ -97,8 +97,10 @@ tos_status copy_out(tos_engine* e, void* dst, const void* src, size_t bytes) {
   }
   work(0);
   for (std::thread& t : others) t.join();
-  if (err.load() != (int)cudaSuccess)
+  if (err.load() != (int)cudaSuccess) {
+    cudaStreamSynchronize(st);  // a chunk still on its way lands before its slot is used again
     return fail(TOS_ERR_CUDA, std::string("copy to the host: ") + cudaGetErrorString((cudaError_t)err.load()));
+  }
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   return TOS_OK;
 }
