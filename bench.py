@@ -45,6 +45,8 @@ METRIC = "pixel-pairs/s on 1 B200, plain vs batched, ≤1e-6 rel err vs FP64; p5
 UNIT = "pixel-pairs/s"
 NSM = 148
 FP32_LANES_PER_SM = 128
+# What limits each sweep (profiles/): none of them bins every pair any more.
+LIMITED_BY = {"grid_kernel": "lsu", "diag_kernel": "lsu", "line_kernel": "lsu"}
 # FP32-pipe operations per pixel pair counted for the pair-rate roofline
 # (FMA = 1 op; MUFU and shared atomics excluded): Cartesian 6, Polar 7, brute 9.
 OPS_PER_PAIR = {"cartesian": 6, "polar": 7, "brute": 9}
@@ -497,7 +499,9 @@ def engine_arm(args, D):
     sm_mhz = clocks["sm_mhz"] if clocks and clocks.get("sm_mhz") == clocks.get("sm_mhz") else 1965.0
     peak = NSM * FP32_LANES_PER_SM * sm_mhz * 1e6 / 1e12  # tera lane-ops/s
     achieved = pairs * ops / (kernel_ms / 1e3) / 1e12
-    roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+    roof = {"bound": LIMITED_BY.get(kernel_name, "fp32"),
+            "model": "FP32 pair rate: a kernel that bins every pair; no ceiling for a sweep that does not",
+            "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": load_traffic(W["name"]),
             "kernel": kernel_name, "kernel_ms": kernel_ms, "ops_per_pair": ops,
             "pairs_per_launch": pairs, "pairs_in_runs_per_launch": evaluated,

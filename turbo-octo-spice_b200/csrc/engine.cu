@@ -646,7 +646,9 @@ __device__ __forceinline__ int grid_index(const float* U, int ng, float x) {
 // pointers: 540 of 600 values 11.6 / 17.2 | 104 / 70, 204 of 600 10.8 / 16.9 |
 // 102 / 28, 150 of 600 25 / 22 | 60 / 21; 320k / 719k items of 64 of 128
 // values 10.9 / 20.0 | 19.0 / 21.3, 43 of 128 10.5 / 19.9 | 13.0 / 15.2, 16 of
-// 64 7.3 / 12.4 | 4.6 / 6.0).
+// 64 7.3 / 12.4 | 4.6 / 6.0).  One rule serves both coordinates: it lies where
+// the observing sweep breaks even (150 of 600); Cartesian forests that sparse,
+// which would still gain from the grid, go to the pointer sweep too.
 //
 // What ensure_grid reads of a grid: values, contiguous sightlines and those with
 // gaps, the largest span, contiguous ones of at most kShortPixels pixels, the sum

@@ -133,8 +133,9 @@ __device__ __forceinline__ bool diag_item(const PairArgs& A, double zlo, double 
 }
 
 // The kernel that takes item idx, from the predicates above as each kernel
-// applies them (load_item for the sweeps, the pixel-pair kernel's own test): one lane per item, so that a kernel can claim a batch
-// of items and skip the others' without loading each one warp-wide.
+// applies them (load_item for the pointer sweep, the pixel-pair kernel's own
+// test): one lane per item, so that a kernel can claim a batch of items and skip
+// the others' without loading each one warp-wide.
 enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerShort, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerPair };
 __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long idx) {
   const uint32_t i = A.item_i[idx], j = A.item_j[idx];

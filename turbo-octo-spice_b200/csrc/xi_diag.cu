@@ -47,7 +47,7 @@
 namespace tos {
 namespace {
 
-constexpr int kDiagWarps = 8;  // warps per CTA; a CTA takes one item at a time
+constexpr int kDiagWarps = 8;  // warps per CTA; a CTA has two items in flight
 constexpr int kDiagThreads = kDiagWarps * 32;
 constexpr int kDiagRows = 16;  // rows of a block
 constexpr int kDiagSpan = 64;  // diagonals of a warp's group
@@ -610,8 +610,8 @@ __device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsi
 
 // The arguments stay in the kernel's parameter space (__grid_constant__):
 // the inlined sweep reads them as constant-bank operands.  Two item buffers
-// per CTA, as in the band sweep (xi_grid.cu): warp 0 prepares the next item
-// before its share of this one, and each warp takes the item's groups from a
+// per CTA, as in the band sweep (xi_grid.cu): the warps take turns to prepare the
+// next item before their share of this one, and each warp takes the item's groups from a
 // counter and goes on to the next item by itself.
 template <bool MINPOS, bool SMEM>
 __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_constant__ PairArgs A) {

@@ -125,10 +125,11 @@ struct Sums6 {
 };
 
 // ---- the item pipeline ----------------------------------------------------
-// Two item buffers per CTA.  Warp 0 prepares item k + 1 (claims it, finds its
-// bands, starts the bulk copies of its prefix sums and row values) before its
-// share of item k; each warp goes from item to item on its own, so a warp
-// with fewer rows does not wait for the others unless it gets two items ahead.
+// Two item buffers per CTA.  The warps take turns to prepare item k + 1 (claim
+// it, find its bands, start the bulk copies of its prefix sums and row values)
+// before their share of item k; each warp goes from item to item on its own, so
+// a warp with fewer rows does not wait for the others unless it gets two items
+// ahead.
 
 // Row constants of the r_perp code of a row of distance d1.
 __device__ __forceinline__ RowV code_row(const PairArgs& A, float ap, float d1) {

@@ -1,8 +1,8 @@
-// xi_sweep.cuh — the run sweep shared by the grid-sweep kernel (xi_grid.cu,
-// bin boundaries read from a table of the catalogue's common coordinate grid)
-// and the pointer-sweep kernel (xi_runs.cu, boundaries found by walking
-// column pointers): Cartesian (r_par, r_perp) and observing (dloglam, theta)
-// coordinates, items whose z index is constant.
+// xi_sweep.cuh — the run sweep of the pointer-sweep kernel (xi_runs.cu, bin
+// boundaries found by walking column pointers), and what the band sweep
+// (xi_grid.cu) shares with it (the r_perp code of a pair, the adds to a bin):
+// Cartesian (r_par, r_perp) and observing (dloglam, theta) coordinates, items
+// whose z index is constant.
 //
 // For one sightline pair (i, j) with both sightlines sorted, fix a row p1 of
 // i.  Along the columns p2 of j the reference's first-axis value is the float
@@ -177,7 +177,7 @@ __device__ __forceinline__ void RunAcc::add(const PairArgs& A, Dest d, int k, in
 
 // Add a sub-run of m columns with r_perp code cc of first-axis bin k, given
 // the differences of sightline j's prefix sums over it (w*delta, w, loglam),
-// to the lane's code accumulators (RunAcc, or the grid sweep's GridAcc).
+// to the lane's code accumulators.
 template <int COORD, class Acc>
 __device__ __forceinline__ void add_sums(const PairArgs& A, Dest d, const RowV& R, int k, int cc, int m,
                                          double dwd, double dw, double dl, Acc& acc) {
