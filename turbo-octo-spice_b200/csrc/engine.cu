@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <limits>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -49,7 +50,8 @@ __global__ void k_fill(float* p, size_t n, float v) {
 // sums of (w*delta, w, loglam); coordinate ranges; sortedness.
 __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t* npix,
                        size_t n_los, float* dist_pad, float* loglam_pad, PixPack* pix2,
-                       double2* pre2, double* prel, double2* row2, float4* range, unsigned int* flags,
+                       double2* pre2, double* prel, double2* row2, float4* range, float4* rough,
+                       unsigned int* flags,
                        unsigned long long* maxbits) {
   const int lane = threadIdx.x & 31;
   const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
@@ -66,6 +68,8 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
     double mwd = 0, mw = 0, ml = 0, md = 0;
     float gap = INFINITY;  // smallest positive step between consecutive distances
     bool unsorted = false;
+    const float step = n > 1 ? (raw[o + n - 1].distance - raw[o].distance) / (float)(n - 1) : 0.f;
+    int uneven = 0;
     if (lane == 0) {
       p2[0] = make_double2(0, 0);
       pl[0] = 0;
@@ -100,6 +104,7 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
         if (k + 1 < n) {
           const tos_pixel nx = raw[o + k + 1];
           if (!(nx.distance >= px.distance) || !(nx.loglam >= px.loglam)) unsorted = true;
+          uneven += fabsf(nx.distance - px.distance - step) > 0.3f * fabsf(step);
           if (nx.distance > px.distance) gap = fminf(gap, __fsub_rd(nx.distance, px.distance));
         }
       }
@@ -135,7 +140,9 @@ __global__ void k_prep(const tos_pixel* raw, const uint64_t* off, const uint32_t
       gap = fminf(gap, __shfl_xor_sync(kFull, gap, d));
     }
     unsorted = __any_sync(kFull, unsorted);
+    uneven = __reduce_add_sync(kFull, uneven);
     if (lane == 0) {
+      rough[s] = make_float4(step, (float)uneven, n > 1 ? 0.5f * (dmin + dmax) : 0.f, (float)n);
       range[s] = make_float4(dmin, dmax, lmin, lmax);
       if (unsorted) atomicOr(flags, 1u);
       if (n > 0) {
@@ -533,6 +540,24 @@ std::vector<float4> code_edges(const RefGrid& g, int k1, double jit) {
     e[m] = make_float4((float)(s * s - w - jit), (float)(s * s + w + jit), (float)(s * s - w), (float)(s * s + w));
   }
   return e;
+}
+
+// tos_catalog::uneven and step_spread from k_prep's values per sightline: the
+// spread of the mean steps is what a straight line over the distance leaves.
+void set_roughness(tos_catalog* cat, const std::vector<float4>& rough) {
+  double n = 0, steps = 0, uneven = 0, sx = 0, sy = 0, sxx = 0, sxy = 0, syy = 0;
+  for (const float4& q : rough) {
+    if (!(q.w > 1.f)) continue;
+    const double x = q.z, y = q.x;
+    n += 1;
+    steps += q.w - 1;
+    uneven += q.y;
+    sx += x, sy += y, sxx += x * x, sxy += x * y, syy += y * y;
+  }
+  if (n == 0) return;
+  cat->uneven = uneven / steps;
+  const double vx = sxx / n - sx / n * (sx / n), vy = syy / n - sy / n * (sy / n), c = sxy / n - sx / n * (sy / n);
+  cat->step_spread = std::sqrt(std::max(0.0, vy - (vx > 0 ? c * c / vx : 0.0)));
 }
 
 // Smallest FP32 r^2 at which the FP32 codes of a Polar pair are within half of
@@ -1244,6 +1269,10 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
     if (l.pixel_offset != total) contiguous = false;
     total += l.num_pixels;
     cat->max_np = std::max(cat->max_np, l.num_pixels);
+    if (l.num_pixels < cat->short_np[1]) {
+      cat->short_np[1] = std::max(cat->short_np[0], l.num_pixels);
+      cat->short_np[0] = std::min(cat->short_np[0], l.num_pixels);
+    }
   }
   cat->n_pix = total;
   std::vector<double4> trig(n_los);
@@ -1358,6 +1387,8 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   TOS_TRY(cat->d_prel.alloc(total + n_los));
   TOS_TRY(cat->d_row2.alloc(total));
   TOS_TRY(cat->d_range.alloc(n_los));
+  DevBuf<float4> d_rough;  // per sightline mean step, uneven steps, middle distance, pixels
+  TOS_TRY(d_rough.alloc(n_los));
   TOS_TRY(cat->d_flags.alloc(3));
   TOS_TRY(cat->d_maxes.alloc(4));
   cudaStream_t st = e->stream;
@@ -1410,13 +1441,15 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
   TOS_CUDA_TRY(cudaMemsetAsync(cat->d_pix2.p, 0, parity * sizeof(PixPack), st));
   k_prep<<<grid_for(e, n_los * 32, 256), 256, 0, st>>>(
       cat->d_raw.p, cat->d_off.p, cat->d_npix.p, n_los, cat->d_dist_pad.p, cat->d_loglam_pad.p, cat->d_pix2.p,
-      cat->d_pre2.p, cat->d_prel.p, cat->d_row2.p, cat->d_range.p, cat->d_flags.p,
+      cat->d_pre2.p, cat->d_prel.p, cat->d_row2.p, cat->d_range.p, d_rough.p, cat->d_flags.p,
       (unsigned long long*)cat->d_maxes.p);
   TOS_CUDA_TRY(cudaGetLastError());
   unsigned int fl[3] = {0u, 0u, 0u};
   double maxes[4];
   TOS_CUDA_TRY(cudaMemcpyAsync(fl, cat->d_flags.p, sizeof(fl), cudaMemcpyDeviceToHost, st));
+  std::vector<float4> rough(n_los);
   TOS_CUDA_TRY(cudaMemcpyAsync(maxes, cat->d_maxes.p, 32, cudaMemcpyDeviceToHost, st));
+  TOS_CUDA_TRY(cudaMemcpyAsync(rough.data(), d_rough.p, n_los * sizeof(float4), cudaMemcpyDeviceToHost, st));
   TOS_CUDA_TRY(cudaStreamSynchronize(st));
   const unsigned int flags = fl[0];
   cat->sorted = (flags & 1u) == 0;
@@ -1438,6 +1471,7 @@ tos_status tos::catalog_create_impl(tos_engine* e, const tos_sightline* los, siz
     return fail(TOS_ERR_INVALID_ARG,
                 "pixels must have finite value, weight, loglam and distance (filter them as "
                 "HDF5Delta::loadForests does)");
+  set_roughness(cat.get(), rough);
   // the raw copy is no longer needed
   cat->d_raw.release();
   *out = cat.release();
@@ -1581,7 +1615,7 @@ constexpr int kChunkCounters = 4128;
 constexpr int kMaxChunks = 64;
 constexpr uint64_t kChunkItemsMin = 131072;  // tens of ms per chunk: the launch tail stays small
 // sweeps that a request runs in chunks
-enum SweepKind { kSweepDiag = 0, kSweepGrid, kSweepShort, kSweepGaps, kSweepKinds };
+enum SweepKind { kSweepDiag = 0, kSweepDiagPairs, kSweepGrid, kSweepShort, kSweepGaps, kSweepKinds };
 constexpr size_t kCounterWords = kChunkCounters + kSweepKinds * kMaxChunks;
 
 // Host callback after a shared-GPU sweep chunk: hands the SMs back.
@@ -1734,7 +1768,8 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // [0..3] kernel counters, [4] pair-kernel item counter, [5] candidates,
   // [6] window flushes, [7] run-kernel item counter, [8] run items, [9] grid
   // items, [10] grid-kernel item counter, [11] diagonal-kernel item counter,
-  // [12] diagonal items, [13] a wait of a sweep ran out, [14] gap-kernel item counter, [15] short-item kernel's,
+  // [12] diagonal items, [13] a wait of a sweep ran out, [14] gap-kernel item
+  // counter, [15] that of the kernel for short items or (Polar) pair by pair,
   // [16] theta indices on an edge, [17..] their item numbers (4096 at most)
   unsigned long long* ctr = ws->d_counters.p;
   const double theta_min = G.axis[1].min, theta_inv = 1.0 / axis_width(G.axis[1]);
@@ -2087,6 +2122,21 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       set_wide_scales(A, cat, spare_items);
       A.diag_split = 1;
       A.jit2 = (float)(std::ldexp(cat->max_d * cat->max_d, -24) * 1.01 + 1e-6);
+      // Which sweep is the faster one (figures at diag_pairs_kernel): blocks pay
+      // from 128 pixels on, with r bins below 2 from more, and only where a block
+      // of 16 rows meets few changes of |d2 - d1| (uneven steps of either
+      // sightline, different steps of the two, in bins): 3.2 a block with bins of
+      // 4, 0.6 with bins of 2, and 0.45 on a few bins, where the runs that they
+      // cut meet.  One rule for a catalogue's long sightlines: with some of their
+      // items in each sweep both end with idle warps.
+      {
+        const double w = std::min(1.0, 0.25 / rg.inv0);
+        double limit = 3.2 * std::pow(w, 2.42);
+        if (n0 * n1 < 400) limit = std::min(limit, 0.45);
+        A.diag_len = 32 * cat->uneven + 18 * cat->step_spread * rg.inv0 <= limit
+                         ? (int)std::min(1e4, 128 * std::pow(std::max(1.0, 0.5 / w), 1.6))
+                         : std::numeric_limits<int>::max();
+      }
       A.eps0 = 5e-4f + 1e-6f * (float)n0;
       A.eps1 = 5e-4f + 1e-6f * (float)n1;
       pthr = polar_thresholds(rg);
@@ -2151,11 +2201,12 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   // of chunk launches, each with its own item counter (ctr[kChunkCounters ..],
   // after the theta-edge flags of observing grids at ctr[16 ..]) and its CTA
   // count asked just before launch.
-  static const char* const sweep_name[kSweepKinds] = {"diagonal", "grid", "short", "gap"};
+  static const char* const sweep_name[kSweepKinds] = {"diagonal", "pair-by-pair diagonal", "grid", "short", "gap"};
   auto sweep = [&](SweepKind kind, unsigned long long* counter) -> tos_status {
     auto launch = [&](PairArgs& R, int per_sm) -> cudaError_t {
       switch (kind) {
         case kSweepDiag: return launch_diag_kernel(R, minpos, e->num_sms, per_sm, st);
+        case kSweepDiagPairs: return launch_diag_pairs_kernel(R, minpos, e->num_sms, st);
         case kSweepGrid: return launch_grid_kernel(R, G.type, minpos, e->num_sms, per_sm, st);
         case kSweepShort:
           R.max_span = std::min(R.max_span, (int)kShortPixels);
@@ -2204,7 +2255,8 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
   };
   if (n_items > 0) {
     TOS_CUDA_TRY(cudaEventRecord(e->ev[2], st));
-    if (use_diag) TOS_TRY(sweep(kSweepDiag, ctr + 11));
+    if (use_diag && A.max_np > A.diag_len) TOS_TRY(sweep(kSweepDiag, ctr + 11));
+    if (use_diag && cat->short_np[1] <= (uint32_t)A.diag_len) TOS_TRY(sweep(kSweepDiagPairs, ctr + 15));
     TOS_CUDA_TRY(cudaEventRecord(e->ev[7], st));
     if (use_grid) TOS_TRY(sweep(kSweepGrid, ctr + 10));
     if (use_short) TOS_TRY(sweep(kSweepShort, ctr + 15));

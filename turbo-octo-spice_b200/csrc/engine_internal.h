@@ -299,6 +299,10 @@ struct tos_catalog {
   double min_d = 0;                 // smallest distance
   double min_gap = 0;               // smallest positive distance step within a sightline (lower bound)
   uint32_t max_np = 0;
+  uint32_t short_np[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};  // pixels of the two shortest sightlines
+  // mean share of a sightline's steps that differ from their mean by more than
+  // 0.3 of it, and the spread of the mean steps of sightlines at one distance
+  double uneven = 0, step_spread = 0;
   // common first-axis grids (0: distance, 1: loglam), built on first use
   mutable std::mutex grid_mu;                          // guards the grids and their layouts
   bool grid_built[2] = {false, false};

@@ -136,7 +136,7 @@ __device__ __forceinline__ bool diag_item(const PairArgs& A, double zlo, double 
 // applies them (load_item for the pointer sweep, the pixel-pair kernel's own
 // test): one lane per item, so that a kernel can claim a batch of items and skip
 // the others' without loading each one warp-wide.
-enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerShort, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerPair };
+enum ItemOwner { kOwnerNone = 0, kOwnerGrid, kOwnerShort, kOwnerGaps, kOwnerRun, kOwnerDiag, kOwnerDiagPairs, kOwnerPair };
 __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long idx) {
   const uint32_t i = A.item_i[idx], j = A.item_j[idx];
   if (A.npix[i] == 0 || A.npix[j] == 0) return kOwnerNone;
@@ -154,7 +154,8 @@ __device__ __forceinline__ int item_owner(const PairArgs& A, unsigned long long 
     }
     return kOwnerRun;
   }
-  if (diag_item(A, zlo, zhi, zb_lo, zb_hi)) return kOwnerDiag;
+  if (diag_item(A, zlo, zhi, zb_lo, zb_hi))
+    return max(A.npix[i], A.npix[j]) > (uint32_t)A.diag_len ? kOwnerDiag : kOwnerDiagPairs;
   return kOwnerPair;
 }
 
@@ -173,10 +174,10 @@ struct Claim {
 // The next item of kernel `owner` (one warp; false: none left).  A claim takes
 // one item, so that long items spread over the CTAs (`size` items, up to
 // kClaimItems, where they are short); after those of another kernel it takes
-// twice as many, up to kClaimItems, until it holds one of its own: a
-// sweep that owns few of the items goes through the others 32 at a time.  (8.0e6
-// items of 4,000 contiguous sightlines, one of them masked: the gap sweep scanned
-// them in 52 ms one by one, now in 2.)
+// twice as many, up to A.claim_max, until it holds one of its own: a sweep that
+// owns few of the items goes through the others up to 32 at a time.  (8.0e6 items
+// of 4,000 contiguous sightlines, one of them masked: the gap sweep scanned them
+// in 52 ms one by one, now in 2.)
 __device__ __forceinline__ bool claim_item(const PairArgs& A, int owner, Claim& C, int lane, unsigned long long& idx,
                                            int size = 1) {
   unsigned todo = C.todo;
@@ -189,7 +190,7 @@ __device__ __forceinline__ bool claim_item(const PairArgs& A, int owner, Claim& 
       if (item_owner(A, idx) == owner) return true;
       size = 2;
     }
-    for (; todo == 0u; size = min(2 * size, kClaimItems)) {
+    for (; todo == 0u; size = min(2 * size, max(size, A.claim_max))) {
       if (lane == 0) idx = atomicAdd(A.next_item, (unsigned long long)size);
       idx = __shfl_sync(kFull, idx, 0);
       if (idx >= A.n_items) return false;

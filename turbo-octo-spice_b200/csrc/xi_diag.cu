@@ -1,6 +1,7 @@
-// xi_diag.cu — diagonal-sweep kernel of the XiEstimator pair count for Polar
+// xi_diag.cu — diagonal-sweep kernels of the XiEstimator pair count for Polar
 // (r, mu) coordinates (XiEstimator.cc:168-225), items whose z index is
-// constant.
+// constant: in blocks (below), or pair by pair where blocks do not pay
+// (diag_pairs_kernel).
 //
 // Along a row of the pixel-pair matrix the Polar key (r bin, mu bin) changes
 // every few columns, so runs along rows are short.  Along a diagonal
@@ -28,19 +29,21 @@
 // one row later), and a sightline's pixels lie even ones first, then odd ones,
 // so that the lanes of a warp, two diagonals apart, read neighbouring entries.
 //
-// What bounds it: issue (52 % of cycles) and the shared-memory pipe (68 %);
+// What bounds it: issue (53 % of cycles) and the shared-memory pipe (64 %);
 // about a third of the instructions are the block sums, a fifth each the block
 // keys and the pair-by-pair blocks (6.6 % of the pairs).
 //
 // Measured on a B200 against the version that binned every pair (one warp per
-// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 264 ms; five mocks
-// of 5,000 sightlines in all: 292 -> 156 ms; jackknife of 2,500 sightlines (its
+// item): 7,000 sightlines at 16/deg^2, 50 x 20 bins: 486 -> 261 ms; five mocks
+// of 5,000 sightlines in all: 292 -> 153 ms; jackknife of 2,500 sightlines (its
 // few rows once went to the pixel-pair kernel: low words of 32 bits could have
-// wrapped after 2^32 adds): 363 -> 95 ms.  Block bounds from the extremes of
+// wrapped after 2^32 adds): 363 -> 97 ms with its covariance.  Block bounds from the extremes of
 // d1 d2 instead of r^2 sent twice the blocks pair by pair; functions that are
 // not inlined and read the arguments through the kernel's parameters cost 6 %;
 // one lane per run with its own 15 adds touched 32 lines an add and took 30 of
 // 46 shared-memory and L1 cycles a step.
+#include <algorithm>
+
 #include "bulk_pipeline.cuh"
 #include "xi_device.cuh"
 
@@ -80,10 +83,10 @@ struct DItem {
   const PixPack* cols;   // padded pixels of sightline j, even ones first
 };
 
-// The CTA's two items and the launch's arguments for the functions that are
+// The CTA's two items (pair by pair: one a warp) and the launch's arguments for the functions that are
 // not inlined: through a reference to the kernel's parameters they would read
 // them by generic loads.
-__shared__ DItem s_item[2];
+__shared__ DItem s_item[kDiagWarps];
 __shared__ PairArgs s_args;
 __shared__ Claim s_claim;  // of the warp that prepares an item
 
@@ -512,6 +515,66 @@ __device__ __forceinline__ void diag_group(const PairArgs& A, const DItem& it, i
   n_eval_sum += n_eval;
 }
 
+// The constants of item idx (sightlines i, j) and its diagonals [dlo, dhi];
+// false when none reaches the grid (all lanes of one warp).
+__device__ __forceinline__ bool diag_window(const PairArgs& A, unsigned long long idx, uint32_t i, uint32_t j, int lane,
+                                            DItem& it, int& dlo, int& dhi) {
+  it.ni = (int)A.npix[i];
+  it.nj = (int)A.npix[j];
+  it.c = A.item_c[idx];
+  const double a = 2.0 * dsub(1.0, it.c);
+  it.ap = (float)a;
+  const float4 ri = A.range[i], rj = A.range[j];
+  it.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
+  it.cell = dest_row(A, i, j);
+  it.prei = A.off[i] + i;
+  it.prej = A.off[j] + j;
+  // Column window |d1 - d2| < lim of every row (the pixel-pair kernel's
+  // Polar bound: r^2 >= (d2 - d1)^2 + 2(1 - c) dmin_i dmin_j - err), and
+  // from it the diagonals that reach it.
+  dlo = -(it.ni - 1);
+  dhi = it.nj - 1;
+  if (A.prune) {
+    float lim = A.win_lim;
+    if (ri.x > 0.f && rj.x > 0.f) {
+      const double q = A.polar_r2 - fmax(a, 0.0) * (double)ri.x * (double)rj.x * (1.0 - 1e-6) + A.polar_e2;
+      lim = fminf(lim, (float)(sqrt(fmax(q, 0.0)) * (1.0 + 1e-6) + 1e-3));
+    }
+    const float* rowd = A.dist_pad + A.off[i] + (uint64_t)kPad * (i + 1);
+    const float* cold = A.dist_pad + A.off[j] + (uint64_t)kPad * (j + 1);
+    // over stretches of rows: the window's ends grow with the row, so the
+    // first row's lower end and the last row's upper end bound a stretch
+    const int step = (it.ni + 63) >> 6;
+    dlo = 0x7FFFFFFF;
+    dhi = -0x7FFFFFFF;
+    for (int r = lane * step; r < it.ni; r += 32 * step) {
+      const int re = min(r + step, it.ni) - 1;
+      const float xa = rowd[r], xb = rowd[re];
+      int lo = 0, hi = it.nj;  // first column with fl(xa - x2) < lim
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__fsub_rn(xa, cold[mid]) < lim) hi = mid; else lo = mid + 1;
+      }
+      int lo2 = lo, hi2 = it.nj;  // first column with x2 >= xb and fl(x2 - xb) >= lim
+      while (lo2 < hi2) {
+        const int mid = (lo2 + hi2) >> 1;
+        const float x2 = cold[mid];
+        if (x2 >= xb && __fsub_rn(x2, xb) >= lim) hi2 = mid; else lo2 = mid + 1;
+      }
+      if (lo2 > lo) {
+        dlo = min(dlo, lo - re);
+        dhi = max(dhi, lo2 - 1 - r);
+      }
+    }
+    dlo = __reduce_min_sync(kFull, dlo);
+    dhi = __reduce_max_sync(kFull, dhi);
+    if (dhi < dlo) return false;
+    dlo = max(dlo, -(it.ni - 1));
+    dhi = min(dhi, it.nj - 1);
+  }
+  return true;
+}
+
 // Prepare the next owned item into `h` (all lanes of one warp; SMEM: its
 // pixels into buf), arriving on `full`.  Returns the items taken.
 template <bool SMEM>
@@ -525,58 +588,8 @@ __device__ __noinline__ int prepare_diag(DItem* h, int* next, PixPack* buf, unsi
     if (!claim_item(A, kOwnerDiag, s_claim, lane, idx)) break;
     ++taken;
     const uint32_t i = A.item_i[idx], j = A.item_j[idx];
-    it.ni = (int)A.npix[i];
-    it.nj = (int)A.npix[j];
-    it.c = A.item_c[idx];
-    const double a = 2.0 * dsub(1.0, it.c);
-    it.ap = (float)a;
-    const float4 ri = A.range[i], rj = A.range[j];
-    it.zb = zbin_of_sum(__fadd_rn(ri.z, rj.z), A.g);
-    it.cell = dest_row(A, i, j);
-    it.prei = A.off[i] + i;
-    it.prej = A.off[j] + j;
-    // Column window |d1 - d2| < lim of every row (the pixel-pair kernel's
-    // Polar bound: r^2 >= (d2 - d1)^2 + 2(1 - c) dmin_i dmin_j - err), and
-    // from it the diagonals that reach it.
-    int dlo = -(it.ni - 1), dhi = it.nj - 1;
-    if (A.prune) {
-      float lim = A.win_lim;
-      if (ri.x > 0.f && rj.x > 0.f) {
-        const double q = A.polar_r2 - fmax(a, 0.0) * (double)ri.x * (double)rj.x * (1.0 - 1e-6) + A.polar_e2;
-        lim = fminf(lim, (float)(sqrt(fmax(q, 0.0)) * (1.0 + 1e-6) + 1e-3));
-      }
-      const float* rowd = A.dist_pad + A.off[i] + (uint64_t)kPad * (i + 1);
-      const float* cold = A.dist_pad + A.off[j] + (uint64_t)kPad * (j + 1);
-      // over stretches of rows: the window's ends grow with the row, so the
-      // first row's lower end and the last row's upper end bound a stretch
-      const int step = (it.ni + 63) >> 6;
-      dlo = 0x7FFFFFFF;
-      dhi = -0x7FFFFFFF;
-      for (int r = lane * step; r < it.ni; r += 32 * step) {
-        const int re = min(r + step, it.ni) - 1;
-        const float xa = rowd[r], xb = rowd[re];
-        int lo = 0, hi = it.nj;  // first column with fl(xa - x2) < lim
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (__fsub_rn(xa, cold[mid]) < lim) hi = mid; else lo = mid + 1;
-        }
-        int lo2 = lo, hi2 = it.nj;  // first column with x2 >= xb and fl(x2 - xb) >= lim
-        while (lo2 < hi2) {
-          const int mid = (lo2 + hi2) >> 1;
-          const float x2 = cold[mid];
-          if (x2 >= xb && __fsub_rn(x2, xb) >= lim) hi2 = mid; else lo2 = mid + 1;
-        }
-        if (lo2 > lo) {
-          dlo = min(dlo, lo - re);
-          dhi = max(dhi, lo2 - 1 - r);
-        }
-      }
-      dlo = __reduce_min_sync(kFull, dlo);
-      dhi = __reduce_max_sync(kFull, dhi);
-      if (dhi < dlo) continue;
-      dlo = max(dlo, -(it.ni - 1));
-      dhi = min(dhi, it.nj - 1);
-    }
+    int dlo, dhi;
+    if (!diag_window(A, idx, i, j, lane, it, dlo, dhi)) continue;
     it.dlo = dlo;
     it.groups = (dhi - dlo) / kDiagSpan + 1;
     const PixPack *gi = A.pix2 + A.off[i] + (uint64_t)(2 * kParityPad) * i,
@@ -673,6 +686,119 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const __grid_cons
   add_counters_diag(A, lane, n_eval, lane == 0 ? Q.rech : 0ull, n_taken);
 }
 
+// ---- pair by pair -----------------------------------------------------------
+// Items for which blocks do not pay: in short sightlines most of a block's 16
+// rows and a group's 64 diagonals lie outside the matrix, and a CTA an item is
+// bound by the chain of reads that prepares it; missing pixels or unlike steps
+// change |d2 - d1| inside the blocks, and fine bins leave few of one key.  Each
+// such item has a warp, whose lanes walk a diagonal each, row by row, and bin
+// every pair.  Bound by issue (80 % of cycles, 125 instructions a step).
+//
+// Measured on a B200 (ms): all items in blocks | pair by pair | the sweep before
+// the blocks, which binned every pair.  50 x 20 bins to 200:
+//   328,000 items of 16 pixels                       3.81 | 0.76 | 0.78
+//   of 64                                            7.48 | 4.52 | 4.15
+//   of 128                                           13.1 | 13.0 | 12.4
+//   of 256                                           26.6 | 41.0 | 40.2
+//   73,000 of 560, none masked                       13.1 | 26.6 | 26.5
+//   8 % masked (windows and single pixels)           20.5 | 26.0 | 25.8
+//   222,000 of 128 in 150, scattered                 19.6 | 10.9 | 13.4
+//   54,000 of 560, every sightline its own step      31.1 | 32.6 | 32.7
+// 200 x 100 bins, 73,000 of 560: none masked 27.3 | 30.1 | 29.3, 8 % masked
+// 37.7 | 30.5 | 31.6; 100 x 50: 18.1 | 27.8 | 27.6, 27.9 | 27.7 | 27.7; 25 x 4
+// to 150 (the blocks' runs meet on its 100 bins): 6.7 | 13.9 | 13.7, 16.7 | 13.4
+// | 15.6.
+
+// One item's arrays: distances (padded by sentinels) and (w*delta, w).
+struct PairsItem {
+  const float *rowd, *cold;
+  const double2 *row2, *col2;
+};
+
+// Diagonals d0 .. d0 + 31 (lane = diagonal - d0, up to dhi) of the warp's item.
+template <bool MINPOS>
+__device__ __forceinline__ void pairs_group(const PairArgs& A, const PairsItem& p, int ni, int nj, float ap, int buf,
+                                            int d0, int dhi, int lane, WarpQ& Q, unsigned& n_eval, unsigned& rech) {
+  const int delta = d0 + lane;
+  const int s_lo = max(0, -(d0 + 31)), s_hi = min(ni, nj - d0);
+  const int lo = max(0, -delta);
+  const int rows = delta <= dhi ? max(min(ni, nj - delta) - lo, 0) : 0;  // of the lane, from lo
+  n_eval += rows;
+  // column s + delta: -31 .. nj + 31, within the padding of the distances
+  const float *rd = p.rowd + s_lo, *cd = p.cold + (s_lo + delta);
+  const double2 *rw = p.row2 + s_lo, *cw = p.col2 + (s_lo + delta);
+  uint32_t cur = kInvalidKey;
+  int s0 = 0, qn = 0;
+  double didj = 0.0, wgt = 0.0;
+#pragma unroll 1
+  for (int s = s_lo; s < s_hi; ++s, ++rd, ++cd, ++rw, ++cw) {
+    const bool in = (unsigned)(s - lo) < (unsigned)rows;
+    const float x2 = *cd;
+    const double2 r = *rw;
+    double2 q = make_double2(0.0, 0.0);
+    if (in) q = *cw;
+    DRow R;
+    R.x1 = R.d1 = *rd;
+    const float d2 = __fmul_rn(R.d1, R.d1);
+    R.dl1 = -__fmaf_rn(R.d1, R.d1, -d2);  // -(d1*d1 - fl(d1*d1)), exact
+    R.A1 = __fmul_rn(R.d1, ap);
+    bool recheck;
+    int b0, b1;
+    uint32_t key = polar_key<MINPOS>(A, R, x2, recheck, b0, b1);
+    recheck = recheck && in;
+    if (__any_sync(kFull, recheck)) {
+      if (recheck) {
+        key = polar_key_exact(s_args, R.d1, x2, s_item[buf].c, b0, b1);
+        ++rech;
+      }
+    }
+    if (!in) key = kInvalidKey;
+    const bool change = key != cur;
+    push_run(buf, Q, qn, change && cur != kInvalidKey, cur, s0, s, delta, didj, wgt, lane);
+    if (change) {
+      cur = key;
+      s0 = s;
+      didj = 0.0;
+      wgt = 0.0;
+    }
+    didj = __fma_rn(r.x, q.x, didj);  // (no bin: the run's sums are dropped)
+    wgt = __fma_rn(r.y, q.y, wgt);
+  }
+  push_run(buf, Q, qn, cur != kInvalidKey, cur, s0, s_hi, delta, didj, wgt, lane);
+  drain(buf, Q, 0, qn, lane);
+}
+
+template <bool MINPOS>
+__global__ void __launch_bounds__(kDiagThreads, 3) diag_pairs_kernel(const __grid_constant__ PairArgs A) {
+  extern __shared__ PixPack diag_smem[];  // the warps' queues
+  __shared__ Claim s_claims[kDiagWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  WarpQ& Q = reinterpret_cast<WarpQ*>(diag_smem)[warp];
+  if (tid == 0) s_args = A;
+  if (lane == 0) s_claims[warp].todo = 0u;
+  __syncthreads();
+  unsigned long long n_eval = 0, n_rech = 0, n_taken = 0, idx = 0;
+  while (claim_item(A, kOwnerDiagPairs, s_claims[warp], lane, idx, A.short_claim)) {
+    ++n_taken;
+    const uint32_t i = A.item_i[idx], j = A.item_j[idx];
+    DItem it;
+    int dlo, dhi;
+    if (!diag_window(A, idx, i, j, lane, it, dlo, dhi)) continue;
+    __syncwarp();  // the last item's sums are added
+    if (lane == 0) s_item[warp] = it;
+    __syncwarp();
+    const PairsItem p = {A.dist_pad + A.off[i] + (uint64_t)kPad * (i + 1), A.dist_pad + A.off[j] + (uint64_t)kPad * (j + 1),
+                         A.row2 + A.off[i], A.row2 + A.off[j]};
+    const int ni = it.ni, nj = it.nj;
+    const float ap = it.ap;
+    unsigned ev = 0, re = 0;
+    for (int d0 = dlo; d0 <= dhi; d0 += 32) pairs_group<MINPOS>(A, p, ni, nj, ap, warp, d0, dhi, lane, Q, ev, re);
+    n_eval += ev;
+    n_rech += re;
+  }
+  add_counters_diag(A, lane, n_eval, n_rech, n_taken);
+}
+
 // Two items of two padded sightlines.
 size_t diag_smem_bytes(const PairArgs& a) { return (size_t)4 * (a.max_np + 3 * kParityPad) * sizeof(PixPack); }
 
@@ -693,7 +819,9 @@ cudaError_t launch_diag(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
     return cudaSuccess;
   }
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-  kern<<<num_sms * per_sm, kDiagThreads, smem, stream>>>(a);
+  PairArgs b = a;
+  b.claim_max = claim_limit(a.n_items, num_sms * per_sm);
+  kern<<<num_sms * per_sm, kDiagThreads, smem, stream>>>(b);
   return cudaGetLastError();
 }
 
@@ -707,7 +835,31 @@ cudaError_t launch_diag2(const PairArgs& a, int num_sms, int ctas_per_sm, cudaSt
              : launch_diag<MINPOS, false>(a, num_sms, ctas_per_sm, stream, max_out);
 }
 
+template <bool MINPOS>
+cudaError_t launch_pairs(const PairArgs& a, int num_sms, cudaStream_t stream) {
+  constexpr size_t smem = kDiagWarps * sizeof(WarpQ);
+  auto kern = diag_pairs_kernel<MINPOS>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kDiagThreads, smem);
+  if (e != cudaSuccess) return e;
+  const int ctas = num_sms * (per_sm > 0 ? per_sm : 1);
+  PairArgs b = a;
+  b.claim_max = claim_limit(a.n_items, ctas * kDiagWarps);
+  // short items several at a time (16 of 32 pixels), as many as leave each warp several claims
+  b.short_claim = (int)std::min<unsigned long long>(
+      std::max(1, std::min(16, 512 / std::max(a.max_np, 1))),
+      std::max<unsigned long long>(1, a.n_items / (4ull * ctas * kDiagWarps)));
+  kern<<<ctas, kDiagThreads, smem, stream>>>(b);
+  return cudaGetLastError();
+}
+
 }  // namespace
+
+cudaError_t launch_diag_pairs_kernel(const PairArgs& a, bool minpos, int num_sms, cudaStream_t stream) {
+  return minpos ? launch_pairs<true>(a, num_sms, stream) : launch_pairs<false>(a, num_sms, stream);
+}
 
 cudaError_t launch_diag_kernel(const PairArgs& a, bool minpos, int num_sms, int ctas_per_sm, cudaStream_t stream,
                                int* max_out) {

@@ -687,6 +687,7 @@ cudaError_t launch_grid(const PairArgs& a, int num_sms, int ctas_per_sm, cudaStr
   }
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
   PairArgs b = a;
+  b.claim_max = claim_limit(a.n_items, num_sms * per_sm);
   // (as many as leave each CTA several claims)
   b.short_claim = (int)std::min<unsigned long long>(
       kShortClaim, std::max<unsigned long long>(1, a.n_items / (4ull * num_sms * per_sm)));

@@ -78,6 +78,14 @@ struct Prefix {
 #endif
 };
 
+// The most items a claim may grow to with `workers` claiming at once: one of
+// them may hold as many of its kernel's items as it claims, so that a claim stays
+// below 1/256 of a worker's share of the list.
+inline int claim_limit(unsigned long long n_items, int workers) {
+  const unsigned long long m = n_items / (256ull * (unsigned)workers);
+  return m < 1 ? 1 : m > 32 ? 32 : (int)m;
+}
+
 struct PairArgs {
   // catalogue
   const uint64_t* off;       // compact pixel offset of each sightline
@@ -169,7 +177,9 @@ struct PairArgs {
   int ng, ngp;               // grid values; row length of gtab (a multiple of 4, above ng + 3)
   int max_np;                // longest sightline
   uint32_t wait_ms;          // the longest a sweep waits for a copy or another warp
-  int short_claim;           // items a claim of the short layout takes
+  int diag_len;              // Polar: the block sweep takes items whose longer sightline has more pixels
+  int short_claim;           // items a claim of short items takes
+  int claim_max;             // and one after items of another kernel at most (claim_limit)
   int grid_split;            // the grid kernel takes the run items whose sightlines are contiguous on the grid
   int gap_split;             // its variant for gaps takes the other run items whose sightlines are on the grid
   int diag_split;            // Polar: the diagonal-sweep kernel takes the items whose z index is
@@ -216,8 +226,12 @@ cudaError_t launch_short_kernel(const PairArgs& a, int coord, bool minpos, int n
 // The same for the items with gapped sightlines (item_owner: kOwnerGaps).
 cudaError_t launch_gap_kernel(const PairArgs& a, int coord, bool minpos, int num_sms, cudaStream_t stream);
 
+// Launch the Polar sweep that bins pair by pair (xi_diag.cu) over the items that
+// diag_item() accepts whose sightlines have at most diag_len pixels.
+cudaError_t launch_diag_pairs_kernel(const PairArgs& a, bool minpos, int num_sms, cudaStream_t stream);
+
 // Launch the persistent diagonal-sweep kernel (xi_diag.cu) over the Polar
-// items that diag_item() accepts (every field on the wide scale).
+// items that diag_item() accepts with a sightline of more than diag_len pixels (every field on the wide scale).
 cudaError_t launch_diag_kernel(const PairArgs& a, bool minpos, int num_sms, int ctas_per_sm, cudaStream_t stream,
                                int* max_out = nullptr);
 
