@@ -250,7 +250,9 @@ tos_status tos_catalog_groups(const tos_catalog* catalog, uint32_t* group_ids, s
                                   * sweep) with 1 .. max CTAs per SM on the first 65,536
                                   * sightline pairs, keep the fastest on the engine for this
                                   * coordinate type and bin count (later calls use it); the
-                                  * results do not depend on the pick */
+                                  * results do not depend on the pick.  The sweeps for gaps,
+                                  * for short sightlines and pair by pair are not tuned: where
+                                  * they take most of those pairs nothing is picked */
 
 /* Maximum angular scale of a grid for a transverse comoving scale:
  * CartesianGrid::maxAngularScale (CartesianGrid.h:45-46),

@@ -2183,13 +2183,19 @@ tos_status xi_run_impl(tos_engine* e, tos_catalog* cat, Workspace* ws, const tos
       TOS_CUDA_TRY(cudaEventSynchronize(e->ev[5]));
       float ms = 0.f;
       TOS_CUDA_TRY(cudaEventElapsedTime(&ms, e->ev[4], e->ev[5]));
+      if (p == 0) {  // a kernel that takes few of the items is not what is timed
+        unsigned long long taken = 0;
+        TOS_CUDA_TRY(cudaMemcpyAsync(&taken, ctr + (use_diag ? 12 : 9), 8, cudaMemcpyDeviceToHost, st));
+        TOS_CUDA_TRY(cudaStreamSynchronize(st));
+        if (2 * taken < std::min<uint64_t>(n_items, kTuneItems)) break;
+      }
       if (p > 0 && (best == 0.f || ms < best)) {
         best = ms;
         pick = p;
       }
     }
-    ctas_per_sm = pick;
-    {
+    if (best > 0.f) {
+      ctas_per_sm = pick;
       std::lock_guard<std::mutex> lk(e->tune_mu);
       e->xi_tuned[tune_key] = pick;
     }
